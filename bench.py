@@ -1168,9 +1168,12 @@ def main():
                        "substeps_per_step": substeps, "dt": loop.stableTime,
                        "l2": "flushed between steps (256 MiB write)", "replicas": world,
                        "path": {1: "gather", 2: "resident"}.get(loop.path, loop.path), "patches": loop.patches,
-                       "front_warps": loop._native.get_option(_native.FW_OPT_FRONT_WARPS) if loop.path == 2 else None},
+                       "front_warps": loop._native.get_option(_native.FW_OPT_FRONT_WARPS)
+                       if loop.path == 2 and not loop._native.get_option(_native.FW_OPT_CLUSTER) else None},
             "roofline": {"bound": "hbm",
-                         "kernel": "k_resident (all substeps of a step)" if loop.path == 2 else
+                         "kernel": ("k_cluster, grid form (all substeps of a step)"
+                                    if loop._native.get_option(_native.FW_OPT_CLUSTER) else
+                                    "k_resident (all substeps of a step)") if loop.path == 2 else
                                    "substep = k_elements + k_nodes",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_kind": which, "algorithmic_bytes_per_substep": bstep,

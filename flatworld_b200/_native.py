@@ -35,6 +35,8 @@ FW_OPT_STREAM_PATCH = 8
 FW_OPT_STREAM_MINB = 9
 FW_OPT_STREAM_BULK = 10
 FW_OPT_RES_THREADS = 11
+FW_OPT_CLUSTER = 12
+FW_MAX_RUNS = 4  # runs per scene of fw_step_runs
 FW_PACK_PINNED = 1
 
 _lock = threading.Lock()
@@ -100,6 +102,7 @@ _SIGNATURES = {
     "fw_finalize": (C.c_int, [_vp]),
     "fw_step": (C.c_int, [_vp, C.c_int32, C.c_float]),
     "fw_step_scenes": (C.c_int, [_vp, C.c_int32, _f32p]),
+    "fw_step_runs": (C.c_int, [_vp, C.c_int32, _i32p, _f32p]),
     "fw_step_served": (C.c_int, [_vp, _f32p]),
     "fw_step_served_n": (C.c_int, [_vp, _f32p, C.c_int32]),
     "fw_set_active": (C.c_int, [_vp, _i32p]),
@@ -442,6 +445,12 @@ class NativeWorld:
     def step_scenes(self, n: int, dt_per_scene):
         d = _f(dt_per_scene)
         self._check(self._L.fw_step_scenes(self._h, int(n), d[1]), "fw_step_scenes")
+
+    def step_runs(self, counts, dts):
+        """Every active scene through its own runs: counts[s, k] substeps of
+        dts[s, k], k ascending (fw_step_runs)."""
+        n, t = _i(counts), _f(dts)
+        self._check(self._L.fw_step_runs(self._h, int(np.shape(counts)[1]), n[1], t[1]), "fw_step_runs")
 
     def step_served(self, dt_per_scene):
         """One substep; scenes with dt <= 0 stay frozen.  dt must be float32,

@@ -63,6 +63,7 @@ class BatchedLoop:
         self.dt = np.array([lay.dt for lay in self.layouts], dtype=np.float64)
         self.counters = np.zeros(S, dtype=np.int64)
         self._active = np.ones(S, dtype=np.int32)
+        self._runs = None  # the last advanceWithTime's runs, as arrays (_advance_runs)
 
     # ---- sizes
     @property
@@ -138,6 +139,9 @@ class BatchedLoop:
         fewer substeps are frozen while the others finish."""
         runs = [substep_schedule(frame_dt, lay.stableTime, lay.default_dt, lay.useAdapative)
                 for lay in self.layouts]
+        if (self.path == "stream" and max(len(r) for r in runs) <= _native.FW_MAX_RUNS
+                and self._native.get_option(_native.FW_OPT_CLUSTER) == 1):
+            return self._advance_runs(runs)
         pos = [0] * self.S      # index into each scene's run list
         left = [r[0][0] if r else 0 for r in runs]
         base_active = self._active.copy()
@@ -165,6 +169,24 @@ class BatchedLoop:
                     if pos[s] < len(runs[s]):
                         left[s] = runs[s][pos[s]][0]
         self._set_active(base_active)
+
+    def _advance_runs(self, runs):
+        """advanceWithTime where every scene is stepped on chip: the scenes' runs
+        (count, dt) in one native call."""
+        if self._runs is None or self._runs[0] != runs:
+            width = max(1, max(len(r) for r in runs))
+            counts = np.zeros((self.S, width), np.int32)
+            dts = np.zeros((self.S, width), np.float32)
+            last = np.full(self.S, np.nan)
+            for s, scene_runs in enumerate(runs):
+                for k, (n, dt) in enumerate(scene_runs):
+                    counts[s, k], dts[s, k], last[s] = n, np.float32(dt), dt
+            self._runs = (runs, counts, dts, last)
+        _, counts, dts, last = self._runs
+        self._native.step_runs(counts, dts)
+        active = self._active != 0
+        self.counters += np.where(active, counts.sum(axis=1), 0)
+        self.dt = np.where(active & ~np.isnan(last), last, self.dt)
 
     def synchronize(self):
         self._native.synchronize()

@@ -70,7 +70,7 @@ __global__ void k_na_elements(int N, int E, const float2* __restrict__ x, const 
       sy = j2_param[e].x;
       H = j2_param[e].y;
     }
-    fw::element_forces(a, b, c, jinv[e], m, sy, H, j2, f1, f2, f3);
+    fw::element_forces(fw::Scalar2{}, a, b, c, jinv[e], m, sy, H, j2, f1, f2, f3);
     if (mises) j2_state[e] = j2;
   }
   corners[3 * e] = f1;

@@ -201,7 +201,7 @@ __device__ __forceinline__ float res_element(const ResSmem& s, int q, const floa
     H = s.j2p[q].y;
   }
   float2 f1, f2, f3;
-  fw::element_forces(a, b, cc, s.jinv[q], m, sy, H, j2, f1, f2, f3);
+  fw::element_forces(fw::Scalar2{}, a, b, cc, s.jinv[q], m, sy, H, j2, f1, f2, f3);
   if (mises) s.j2[q] = j2;
   s.f[3 * q] = f1;
   s.f[3 * q + 1] = f2;

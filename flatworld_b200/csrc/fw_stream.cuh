@@ -159,7 +159,7 @@ __device__ __forceinline__ void stream_element(const Dev& d, const float2* sx, f
     H = jp.y;
   }
   float2 f1, f2, f3;
-  fw::element_forces(sx[c.x & 0xFFFFu], sx[c.x >> 16], sx[c.y & 0xFFFFu], ji, m, sy, H, j2, f1, f2, f3);
+  fw::element_forces(fw::Packed2{d.one}, sx[c.x & 0xFFFFu], sx[c.x >> 16], sx[c.y & 0xFFFFu], ji, m, sy, H, j2, f1, f2, f3);
   if (mises && (c.y >> 16)) j2_out[e] = j2;
   sf[3 * q] = f1;
   sf[3 * q + 1] = f2;

@@ -21,11 +21,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdarg>
 #include <map>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/fwb200.h"
@@ -42,6 +44,7 @@ namespace {
 constexpr int kBlock = 256;     // default block size of the gather kernels
 constexpr int kMaxBlock = 512;  // launch bound (block sizes are a runtime option)
 constexpr int kGraphSteps = 32;
+constexpr int kCluMinSteps = 3;  // substeps of a call from which a stream world's scenes are stepped on chip
 
 struct Dev {
   float2* x;
@@ -125,6 +128,7 @@ struct Dev {
   // 0.4 / sqrt(E / rho) per body (0 for spring domains: not monitored).
   int32_t* cfl_ord;
   float* body_cfl;
+  float one = 1.0f;  // fw::Packed2::one
 };
 
 }  // namespace
@@ -292,7 +296,7 @@ __device__ __forceinline__ float element_step(const Dev& d, int e) {
       H = q.y;
     }
     float2 f1, f2, f3;
-    fw::element_forces(a, b, c, ji, m, sy, H, j2, f1, f2, f3);
+    fw::element_forces(fw::Scalar2{}, a, b, c, ji, m, sy, H, j2, f1, f2, f3);
     if (mises) d.j2state[e] = j2;
     d.corner[q0] = f1;
     d.corner[q1] = f2;
@@ -1093,8 +1097,16 @@ __global__ void k_energy_groups(const int* first, int n_groups, const double4* p
 
 #include "fw_resident.cuh"
 #include "fw_stream.cuh"
+#include "fw_cluster.cuh"
 
 // ------------------------------------------------------------------ context
+
+// A node's corners (CSR, ascending 3 * triangle + corner) and the rest shape,
+// kept where a step may be laid out after fw_finalize.
+struct HostLists {
+  std::vector<int32_t> off, slot;
+  std::vector<float2> x0;
+};
 
 struct fw_ctx {
   int device = 0;
@@ -1211,6 +1223,30 @@ struct fw_ctx {
   int st_minb = 32;             // FW_OPT_STREAM_MINB: CTAs per SM the kernel's registers are budgeted for
   int st_bulk = 0;              // FW_OPT_STREAM_BULK: stage triangle records with one bulk copy
   size_t st_smem_bulk = 0;
+  // cluster-resident scenes (fw_cluster.cuh): the launches that step them, by cluster size and patch size; the
+  // other scenes' patches and ids (stream worlds)
+  struct CluGroup {
+    CluLaunch r{};
+    int scenes = 0, threads = 0;
+    size_t smem = 0;
+  };
+  int clu_opt = 1;          // FW_OPT_CLUSTER
+  bool shape_asked = false;  // a launch shape of the resident or stream step was set explicitly: that step runs
+  std::vector<CluGroup> clu;
+  std::vector<CluScene> clu_scenes;
+  int* d_flags = nullptr;  // the steps' error flags, one word each, read in one copy: enum Flag
+  enum Flag { kFlagFlex, kFlagRigid, kFlagStream, kFlagCluster, kFlagResident, kFlags };
+  uint32_t clu_epoch = 0;  // grid form: tags used so far
+  std::vector<int32_t> rest_scenes;  // stream worlds: scenes too large for a cluster
+  int32_t* d_rest_scenes = nullptr;
+  int4* d_rest_rng = nullptr;
+  int rest_patches = 0;
+  CluRun* d_runs = nullptr;  // fw_step_runs: every scene's runs
+  int clu_patches = 0;
+  uint64_t clu_last_key = 0;
+  HostLists lists;
+  std::vector<cudaStream_t> side_streams;  // the groups after the first run beside it
+  std::vector<cudaEvent_t> side_events;
   bool res_adj = false;            // the reverse pass runs resident (k_res_adj)
   size_t res_adj_smem = 0;
   unsigned long long* fll = nullptr;  // [2][N][4] flag-in-data force adjoints of the reverse pass
@@ -1257,7 +1293,6 @@ struct fw_ctx {
   std::vector<double> flex_clock;  // per FEM-FEM scene: the float64 substep dt (host copy)
   double flex_clock_all = 0.0;     // fw_set_flex_clock before fw_finalize
   double* d_flex_clock = nullptr;
-  int* d_flex_err = nullptr;
   int32_t* cfl_ord_buf = nullptr;  // CFL monitor (fw_set_cfl_monitor)
   float* cfl_coef_buf = nullptr;
   // spring-mass domains: per body its node mass (0: an FEM body)
@@ -1303,6 +1338,15 @@ int dalloc(fw_ctx* c, T** p, size_t count) {
   if (e != cudaSuccess)
     return fail(c, FW_ERR_OOM, "cudaMalloc(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
   c->allocs.push_back((void*)*p);
+  return FW_OK;
+}
+
+int alloc_flags(fw_ctx* c) {
+  if (c->d_flags) return FW_OK;
+  cudaError_t e = cudaMalloc((void**)&c->d_flags, sizeof(int) * fw_ctx::kFlags);
+  if (e != cudaSuccess) return fail(c, FW_ERR_OOM, "cudaMalloc of the error flags failed: %s", cudaGetErrorString(e));
+  c->allocs.push_back(c->d_flags);
+  FW_CUDA(c, cudaMemsetAsync(c->d_flags, 0, sizeof(int) * fw_ctx::kFlags, c->stream));
   return FW_OK;
 }
 
@@ -1439,6 +1483,12 @@ int stream_steps(fw_ctx* c, int n);
 
 int arena_stream_steps(fw_ctx* c, int n);
 
+int launch_cluster(fw_ctx* c, int n, const float2* x_in, float2* x_out, const float4* j2_in, float4* j2_out,
+                   const CluRun* runs = nullptr, bool direct = false);
+
+int build_resident(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<int32_t>& slot,
+                   const std::vector<float2>& x0, bool has_j2);
+
 int run_steps(fw_ctx* c, int n) {
   int rc = FW_OK;
   if (c->arena && c->a_stream) return arena_stream_steps(c, n);
@@ -1490,29 +1540,46 @@ StreamKernel stream_kernel(int nodes, int minb, int bulk) {
 // (starting buffer, dt mode, dt, count).
 int stream_steps(fw_ctx* c, int n) {
   c->host_counter += n;
+  // a patch is loaded once per call: one or two substeps cost a batch less on
+  // the stream kernels (256 ragged bodies, one substep: 88 / 190 us)
+  const bool clu = !c->clu.empty() && n >= kCluMinSteps;
+  StreamDev sd = c->sd;
+  if (!clu) sd.list = nullptr;
+  if (clu) {
+    // the scenes that fit on clusters in one go; the rest below, in buffers that end where this leaves the state
+    const bool moved = !c->rest_scenes.empty() && (n & 1);
+    const int rc = launch_cluster(c, n, c->d.x, moved ? c->d.x_alt : c->d.x, c->d.j2state,
+                                  moved ? c->d.j2_alt : c->d.j2state);
+    if (rc || c->rest_scenes.empty()) return rc;
+  }
   while (n > 0) {
     const int m = std::min(n, kGraphSteps);
     const uint64_t parity = c->d.x == c->x_buf0 ? 0 : 1;
     const uint64_t key = (1ull << 62) | (parity << 61) | ((uint64_t)(c->d.uniform_dt ? 1 : 0) << 60) |
-                         ((uint64_t)m << 32) | (c->d.uniform_dt ? float_bits(c->d.dt_uniform) : 0u);
+                         ((uint64_t)(clu ? 1 : 0) << 59) | ((uint64_t)m << 32) |
+                         (c->d.uniform_dt ? float_bits(c->d.dt_uniform) : 0u);
     cudaGraphExec_t g = nullptr;
     int rc = cached_graph(c, c->graphs, key, [&] {
       float2 *xa = c->d.x, *xb = c->d.x_alt;
       float4 *ja = c->d.j2state, *jb = c->d.j2_alt;
       for (int k = 0; k < m; ++k) {
-        k_control<<<1, kMaxBlock, 0, c->stream>>>(c->d);
+        const int nr = (int)c->rest_scenes.size();
+        if (clu)
+          k_control_scenes<<<(nr + 127) / 128, 128, 0, c->stream>>>(c->d, c->d_rest_scenes, nr, c->d_rest_rng);
+        else
+          k_control<<<1, kMaxBlock, 0, c->stream>>>(c->d);
         // the patch step as a programmatic dependent of the control (see k_stream)
         cudaLaunchAttribute pdl[1];
         pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         pdl[0].val.programmaticStreamSerializationAllowed = 1;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(c->st_P);
+        cfg.gridDim = dim3(clu ? c->rest_patches : c->st_P);
         cfg.blockDim = dim3(c->st_nodes);
         cfg.dynamicSmemBytes = c->st_bulk ? c->st_smem_bulk : c->st_smem;
         cfg.stream = c->stream;
         cfg.attrs = pdl;
         cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, stream_kernel(c->st_nodes, c->st_minb, c->st_bulk), c->d, c->sd,
+        cudaLaunchKernelEx(&cfg, stream_kernel(c->st_nodes, c->st_minb, c->st_bulk), c->d, sd,
                            (const float2*)xa, xb, (const float4*)ja, jb);
         std::swap(xa, xb);
         std::swap(ja, jb);
@@ -1707,10 +1774,8 @@ int build_stream(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<i
     FW_CUDA(c, cudaMemcpyAsync(c->d.j2_alt, c->d.j2state, sizeof(float4) * E, cudaMemcpyDeviceToDevice, c->stream));
   StreamElem* dse = nullptr;
   StreamNode* dsn = nullptr;
-  int* derr = nullptr;
-  if ((r = dalloc(c, &dse, re.size())) || (r = dalloc(c, &dsn, rn.size())) || (r = dalloc(c, &derr, 1))) return r;
-  FW_CUDA(c, cudaMemsetAsync(derr, 0, sizeof(int), c->stream));
-  c->sd = StreamDev{dp, dn, dh, de, dc, dcp, dcs, no_max, nh_max, ne_max, dse, dsn, derr};
+  if ((r = dalloc(c, &dse, re.size())) || (r = dalloc(c, &dsn, rn.size()))) return r;
+  c->sd = StreamDev{dp, dn, dh, de, dc, dcp, dcs, no_max, nh_max, ne_max, dse, dsn, c->d_flags + fw_ctx::kFlagStream};
   c->st_ne = (int)re.size();
   c->st_no = (int)rn.size();
   if ((r = stream_records(c))) return r;
@@ -1752,6 +1817,566 @@ void rcb(const std::vector<float2>& x, std::vector<int>& idx, int lo, int hi, in
   rcb(x, idx, mid, hi, p0 + k1, np - k1, part);
 }
 
+
+// ------------------------------------------------------------------ cluster-resident scenes
+
+// f(k) for k in [0, n) on up to `threads` host threads (this one among them).
+template <class F>
+void parallel_for(int n, int threads, F f) {
+  std::atomic<int> next{0};
+  auto work = [&] {
+    for (int k; (k = next.fetch_add(1)) < n;) f(k);
+  };
+  std::vector<std::thread> pool;
+  for (int k = 1; k < std::min(n, threads); ++k) pool.emplace_back(work);
+  work();
+  for (std::thread& th : pool) th.join();
+}
+
+int host_threads() { return (int)std::min(16u, std::max(1u, std::thread::hardware_concurrency())); }
+
+// One scene's patches for `ctas` CTAs into out / blob (ids relative to the
+// scene; byte offsets relative to blob).  Returns false when the scene does not
+// fit the encodings.
+bool make_cluster_patches(const fw_ctx* c, const CluScene& sc, int nn, const std::vector<int32_t>& off,
+                          const std::vector<int32_t>& slot, const std::vector<float2>& x0,
+                          const std::vector<uint32_t>& word, int ctas, std::vector<int>& part, int threads,
+                          std::vector<CluPatch>& out, std::vector<unsigned char>& blob) {
+  const int32_t* conn = c->h_conn.data();
+  std::vector<int> idx(nn);
+  for (int k = 0; k < nn; ++k) idx[k] = sc.n0 + k;
+  rcb(x0, idx, 0, nn, 0, ctas, part);
+  struct Part {
+    std::vector<int> owned, tri, halo;  // ascending; interior triangles first
+    std::vector<unsigned char> blob;
+    int n_int = 0;
+  };
+  std::vector<Part> parts(ctas);
+  for (int i = sc.n0; i < sc.n0 + nn; ++i) parts[part[i]].owned.push_back(i);
+  parallel_for(ctas, threads, [&](int p) {
+    Part& q = parts[p];
+    for (int n : q.owned)
+      for (int k = off[n]; k < off[n + 1]; ++k) q.tri.push_back(slot[k] / 3);
+    std::sort(q.tri.begin(), q.tri.end());
+    q.tri.erase(std::unique(q.tri.begin(), q.tri.end()), q.tri.end());
+    for (int e : q.tri)
+      for (int k = 0; k < 3; ++k)
+        if (part[conn[3 * e + k]] != p) q.halo.push_back(conn[3 * e + k]);
+    std::sort(q.halo.begin(), q.halo.end());
+    q.halo.erase(std::unique(q.halo.begin(), q.halo.end()), q.halo.end());
+    q.n_int = (int)(std::stable_partition(q.tri.begin(), q.tri.end(), [&](int e) {
+      return part[conn[3 * e]] == p && part[conn[3 * e + 1]] == p && part[conn[3 * e + 2]] == p;
+    }) - q.tri.begin());
+  });
+  // per node the (patch << 24 | halo slot) that read it, as ranges of one list
+  std::vector<int32_t> doff(nn + 1, 0);
+  for (const Part& q : parts)
+    for (int n : q.halo) doff[n - sc.n0 + 1]++;
+  for (int i = 0; i < nn; ++i) doff[i + 1] += doff[i];
+  std::vector<uint32_t> dest(doff[nn]);
+  {
+    std::vector<int32_t> fill(doff.begin(), doff.end() - 1);
+    for (int p = 0; p < ctas; ++p)
+      for (size_t j = 0; j < parts[p].halo.size(); ++j)
+        dest[fill[parts[p].halo[j] - sc.n0]++] = ((uint32_t)p << 24) | (uint32_t)j;
+  }
+  out.assign(ctas, CluPatch{});
+  std::atomic<bool> fits{true};
+  parallel_for(ctas, threads, [&](int p) {
+    Part& pt = parts[p];
+    std::vector<int>& ow = pt.owned;
+    // boundary nodes, then the others that neighbours read, then the rest, each group ascending
+    auto first = std::stable_partition(ow.begin(), ow.end(), [&](int n) { return (word[n] & fw::NODE_BOUNDARY) != 0; });
+    std::stable_partition(first, ow.end(), [&](int n) { return doff[n - sc.n0] < doff[n - sc.n0 + 1]; });
+    const std::vector<int>&tri = pt.tri, &h = pt.halo;
+    CluPatch& q = out[p];
+    q.no = (int)ow.size();
+    q.nh = (int)h.size();
+    q.ne = (int)tri.size();
+    q.n_int = pt.n_int;
+    q.nbnd = (int)(first - ow.begin());
+    if (q.no >= (int)kCluSlotNodes || q.nh >= (int)kCluHalo || q.no + q.nh >= 0x7FFF) {
+      fits = false;
+      return;
+    }
+    std::vector<std::pair<int, int>> order(q.no);  // node -> its place here
+    for (int i = 0; i < q.no; ++i) order[i] = {ow[i], i};
+    std::sort(order.begin(), order.end());
+    auto local = [&](int n) {
+      if (part[n] == p)
+        return (uint32_t)std::lower_bound(order.begin(), order.end(), std::make_pair(n, 0))->second;
+      return kCluHalo | (uint32_t)(std::lower_bound(h.begin(), h.end(), n) - h.begin());
+    };
+    std::vector<int32_t> gid(q.no), hid(q.nh), eid(q.ne);
+    std::vector<uint32_t> info(q.no), push, pos(q.ne);
+    std::vector<uint2> tr(q.ne);
+    for (int i = 0; i < q.no; ++i) {
+      const int n = ow[i], body = (int)(word[n] >> fw::NODE_BODY_SHIFT) - sc.body0;
+      const int d0 = doff[n - sc.n0], dn = doff[n - sc.n0 + 1] - d0;
+      if (dn > 7 || push.size() >= (1u << 15)) {
+        fits = false;
+        return;
+      }
+      gid[i] = n - sc.n0;
+      info[i] = (word[n] & (fw::NODE_BC_MASK | fw::NODE_BOUNDARY)) | ((uint32_t)body << kCluBodyShift) |
+                ((uint32_t)dn << kCluPushCntShift) | ((uint32_t)push.size() << kCluPushOffShift);
+      for (int k = 0; k < dn; ++k) push.push_back(dest[d0 + k]);
+      q.deg = std::max(q.deg, off[n + 1] - off[n]);
+    }
+    if (q.deg > 30 || (int64_t)(q.deg + 4) * q.no >= (int64_t)kCluNoSlot) {
+      fits = false;
+      return;
+    }
+    for (int j = 0; j < q.nh; ++j) hid[j] = h[j] - sc.n0;
+    for (int k = 0; k < q.ne; ++k) {
+      const int e = tri[k];
+      const int* cn = conn + 3 * e;
+      eid[k] = e - sc.e0;
+      q.n_j2 += c->h_type[e] == fw::MAT_MISES ? 1 : 0;
+      uint32_t sl[3], at[3];
+      for (int m = 0; m < 3; ++m) {
+        at[m] = local(cn[m]);
+        sl[m] = kCluNoSlot;
+        if (part[cn[m]] != p) continue;
+        const int32_t *b = slot.data() + off[cn[m]], *en = slot.data() + off[cn[m] + 1];
+        const int32_t* it = std::lower_bound(b, en, 3 * e + m);  // a node's corners ascend
+        sl[m] = (uint32_t)(it - b) * kCluSlotNodes + at[m];
+      }
+      tr[k] = make_uint2((at[0] | (part[cn[0]] == p ? 0x8000u : 0u)) | (at[1] << 16), at[2] | (sl[0] << 16));
+      pos[k] = sl[1] | (sl[2] << 16);
+    }
+    q.npush = (int)push.size();
+    auto put = [&](const void* src, size_t bytes) {
+      const int64_t o = (int64_t)pt.blob.size();
+      pt.blob.resize(((size_t)o + bytes + 15) & ~(size_t)15);
+      if (bytes) memcpy(pt.blob.data() + o, src, bytes);
+      return o;
+    };
+    q.gid = put(gid.data(), 4 * gid.size());
+    q.info = put(info.data(), 4 * info.size());
+    q.hid = put(hid.data(), 4 * hid.size());
+    q.push = put(push.data(), 4 * push.size());
+    q.eid = put(eid.data(), 4 * eid.size());
+    q.tri = put(tr.data(), 8 * tr.size());
+    q.pos = put(pos.data(), 4 * pos.size());
+  });
+  if (!fits) return false;
+  for (int p = 0; p < ctas; ++p) {
+    const int64_t base = (int64_t)blob.size();
+    for (int64_t* o : {&out[p].gid, &out[p].info, &out[p].hid, &out[p].push, &out[p].eid, &out[p].tri, &out[p].pos})
+      *o += base;
+    blob.insert(blob.end(), parts[p].blob.begin(), parts[p].blob.end());
+  }
+  return true;
+}
+
+// The maxima of a patch into a launch's.
+void clu_widen(CluLaunch& r, const CluPatch& q) {
+  r.no = std::max(r.no, q.no);
+  r.nh = std::max(r.nh, q.nh);
+  r.ne = std::max(r.ne, q.ne);
+  r.deg = std::max(r.deg, q.deg);
+  r.npush = std::max(r.npush, q.npush);
+  r.nbnd = std::max(r.nbnd, q.nbnd);
+  r.has_j2 |= q.n_j2 > 0 ? 1 : 0;
+}
+
+size_t clu_smem(CluLaunch r) { return clu_layout(r); }
+
+// Threads of a CTA, control warps included: a control warp for the boxes and
+// one per 64 boundary nodes for their contact forces, at most 4; and a thread
+// per triangle where that fits a CTA (r.one), else an equal share of them.
+// Where the scenes fill the GPU (`shared`), two triangles per thread: 384
+// bodies of 60 to 400 nodes ran 5.06 / 4.08 / 4.53 / 4.83 us per substep at
+// 1 / 2 / 3 / 4, 256 of 100 to 20000 nodes 33.5 / 33.4 / 33.3 / 36.3.
+int clu_threads(CluLaunch& r, bool shared) {
+  r.ctl = r.np ? std::min(4, 1 + (r.nbnd + 63) / 64) : 1;
+  const int most = kCluMaxThreads - 32 * r.ctl, work = std::max(1, std::max(r.ne, r.no));
+  int rounds = (work + most - 1) / most;
+  if (shared && r.ne >= 128) rounds = std::max(rounds, 2);
+  r.one = rounds == 1 ? 1 : 0;
+  return (((work + rounds - 1) / rounds + 31) / 32 + r.ctl) * 32;
+}
+
+// Does a launch of `ctas`-CTA clusters with this much shared memory fit the device?
+bool clu_fits(const CluLaunch& r, int threads, size_t smem) {
+  if (r.ctas == 1) return true;
+  if (r.grid) {
+    int per_sm = 0, sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, clu_kernel(threads, r.one, 1), threads, smem);
+    cudaGetLastError();
+    return e == cudaSuccess && per_sm * sms >= r.ctas;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = r.ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(r.ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, clu_kernel(threads, r.one, 0), &cfg);
+  cudaGetLastError();
+  return e == cudaSuccess && n >= 1;
+}
+
+// Cut the world's scenes for clusters where they fit, group them into
+// launches, and (stream worlds) list what is left.  Leaves c->clu empty when
+// nothing fits.
+int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<int32_t>& slot,
+                  const std::vector<float2>& x0, const std::vector<uint32_t>& word, bool single) {
+  if (!c->clu_opt || c->shape_asked) return FW_OK;
+  int optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+  const size_t cap = (size_t)optin - kCluStatic;
+  for (int grid = 0; grid < 2; ++grid)
+    for (int one = 0; one < 2; ++one)
+      for (int threads : {512, 1024}) {
+        CluKernel k = clu_kernel(threads, one, grid);
+        FW_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+        if (!grid) FW_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      }
+  const int S = c->S;
+  std::vector<CluScene> scenes(S);
+  std::vector<int> nn(S, 0);
+  std::vector<char> ok(S, 0);
+  {  // bodies, nodes, triangles and pairs of a scene, each one contiguous range
+    for (int s = 0; s < S; ++s) scenes[s].body0 = -1;
+    for (int b = 0; b < c->B; ++b) {
+      CluScene& sc = scenes[c->h_scene[b]];
+      if (sc.body0 < 0) {
+        sc = CluScene{c->h_scene[b], 0, c->h_noff[b], c->h_eoff[b], b, 0, 0, 0};
+        ok[sc.scene] = 1;
+      }
+      const int s = sc.scene;
+      const int ne0 = sc.e0;
+      if (b != sc.body0 + sc.nb || c->h_noff[b] != sc.n0 + nn[s]) ok[s] = 0;
+      if (c->h_eoff[b] < ne0) ok[s] = 0;
+      sc.nb += 1;
+      nn[s] += c->h_ncnt[b];
+    }
+    std::vector<int> cnt(c->B, 0);
+    for (const Pair& p : c->h_pairs) cnt[p.body]++;
+    int at = 0;
+    std::vector<int> first(c->B + 1, 0);
+    for (int b = 0; b < c->B; ++b) {
+      first[b] = at;
+      at += cnt[b];
+    }
+    first[c->B] = at;
+    for (int s = 0; s < S; ++s) {
+      if (!ok[s]) continue;
+      CluScene& sc = scenes[s];
+      sc.pair0 = first[sc.body0];
+      sc.np = first[sc.body0 + sc.nb] - sc.pair0;
+      if (sc.nb > kCluMaxBodies || sc.np > kCluMaxPairs || nn[s] <= 0) ok[s] = 0;
+    }
+  }
+  // triangles of a patch share one material when their body's do
+  std::vector<char> scene_tri(S, 0);
+  for (int b = 0; b < c->B; ++b) {
+    const int s = c->h_scene[b];
+    if (scenes[s].nb > 1) scene_tri[s] = 1;
+    const int e0 = c->h_eoff[b];
+    for (int e = e0 + 1; e < e0 + c->h_ecnt[b] && !scene_tri[s]; ++e)
+      if (c->h_E[e] != c->h_E[e0] || c->h_nu[e] != c->h_nu[e0] || c->h_type[e] != c->h_type[e0] ||
+          c->h_sy[e] != c->h_sy[e0] || c->h_H[e] != c->h_H[e0])
+        scene_tri[s] = 1;
+  }
+  std::vector<int> part(c->N, 0), n_tri(S, 0);
+  for (int b = 0; b < c->B; ++b) n_tri[c->h_scene[b]] += c->h_ecnt[b];
+  std::vector<CluPatch> patches;
+  std::vector<unsigned char> blob;
+  struct Made {
+    int s, ctas;
+    size_t smem;
+    int tri, grid;
+  };
+  std::vector<Made> made;
+  // nodes of a patch: one scene, 128 (64 to 128 run within 3% of each other on
+  // meshes of 441 to 8232 nodes, 192 takes a fourth longer); many, an SM's
+  // share of all nodes, as far as they fit
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+  const int want_nodes = single ? 128 : std::min(1300, std::max(128, c->N / sms));
+  const bool shared = !single && (int64_t)c->E > (int64_t)sms * 900;
+  // each scene by itself (disjoint ranges of part), on the host's threads
+  struct Cut {
+    int ctas = 0;
+    size_t smem = 0;
+    int kind = 0;
+    std::vector<CluPatch> patches;
+    std::vector<unsigned char> blob;
+  };
+  std::vector<Cut> cuts(S);
+  bool size_ok[kCluMaxCtas + 1] = {};  // cluster sizes that fit the device with all of an SM's shared memory
+  for (int k = 1; !single && k <= kCluMaxCtas; k *= 2) {
+    CluLaunch r{};
+    r.ctas = k;
+    size_ok[k] = clu_fits(r, kCluMaxThreads, cap);
+  }
+  parallel_for(S, host_threads(), [&](int s) {
+    if (!ok[s]) return;
+    const int most = single ? sms : kCluMaxCtas;
+    int ctas = single ? std::min(sms, (nn[s] + want_nodes - 1) / want_nodes) : 1;
+    while (!single && ctas < most && (nn[s] + ctas - 1) / ctas > want_nodes) ctas *= 2;
+    for (; ctas <= most && ctas <= nn[s]; ctas *= 2) {
+      // more nodes than threads and not enough room for positions, node state,
+      // corner forces and triangle records: not cut at all
+      if (nn[s] > ctas * kCluMaxThreads && (int64_t)nn[s] * 32 + (int64_t)n_tri[s] * 56 > (int64_t)ctas * (int64_t)cap) continue;
+      Cut& k = cuts[s];
+      k.patches.clear();
+      k.blob.clear();
+      if (!make_cluster_patches(c, scenes[s], nn[s], off, slot, x0, word, ctas, part, S == 1 ? host_threads() : 1, k.patches,
+                                k.blob))
+        continue;
+      CluLaunch r{};
+      r.ctas = ctas;
+      r.grid = single ? 1 : 0;
+      for (const CluPatch& q : k.patches) clu_widen(r, q);
+      r.nb = scenes[s].nb;
+      r.np = scenes[s].np;
+      r.per_tri = scene_tri[s];
+      const int threads = clu_threads(r, shared);
+      k.smem = clu_smem(r);
+      if (k.smem > cap || !(single ? clu_fits(r, threads, k.smem) : size_ok[ctas])) continue;
+      k.ctas = ctas;
+      k.kind = scene_tri[s] * 2 + (r.has_j2 ? 1 : 0);
+      break;
+    }
+  });
+  for (int s = 0; s < S; ++s) {
+    Cut& k = cuts[s];
+    if (!k.ctas) continue;
+    const int64_t base = (int64_t)blob.size();
+    scenes[s].patch0 = (int)patches.size();
+    for (CluPatch& q : k.patches) {
+      for (int64_t* o : {&q.gid, &q.info, &q.hid, &q.push, &q.eid, &q.tri, &q.pos}) *o += base;
+      patches.push_back(q);
+    }
+    blob.insert(blob.end(), k.blob.begin(), k.blob.end());
+    made.push_back(Made{s, k.ctas, k.smem, k.kind, single ? 1 : 0});
+  }
+  if (made.empty()) return FW_OK;
+  if (single && made.size() != (size_t)S) return FW_OK;
+  int rc;
+  int n_halo = 0;
+  for (CluPatch& q : patches) {
+    q.halo0 = n_halo;
+    n_halo += q.nh;
+  }
+  CluPatch* dp = nullptr;
+  unsigned char* db = nullptr;
+  if ((rc = upload(c, &dp, patches)) || (rc = upload(c, &db, blob))) return rc;
+  // groups: same cluster size and, for one CTA, the same kind of triangles and
+  // similar shared memory (so that small patches share an SM), largest first; a
+  // scene joins while the common carve-up fits
+  std::stable_sort(made.begin(), made.end(), [](const Made& a, const Made& b) {
+    return a.ctas != b.ctas ? a.ctas > b.ctas : (a.ctas == 1 && a.tri != b.tri ? a.tri > b.tri : a.smem > b.smem);
+  });
+  std::vector<std::vector<CluScene>> lists;
+  int group_tri = -1;
+  size_t group_smem = 0;
+  for (const Made& m : made) {
+    const CluScene& sc = scenes[m.s];
+    auto widened = [&](CluLaunch r) {
+      for (int k = 0; k < m.ctas; ++k) clu_widen(r, patches[sc.patch0 + k]);
+      r.nb = std::max(r.nb, sc.nb);
+      r.np = std::max(r.np, sc.np);
+      r.per_tri |= m.tri >> 1;
+      clu_threads(r, shared);
+      return r;
+    };
+    bool join = !c->clu.empty() && c->clu.back().r.ctas == m.ctas && (m.ctas > 1 || (group_tri == m.tri && 2 * m.smem > group_smem));
+    if (join && clu_smem(widened(c->clu.back().r)) > cap) join = false;
+    if (!join) {
+      fw_ctx::CluGroup g;
+      g.r.ctas = m.ctas;
+      g.r.grid = m.grid;
+      c->clu.push_back(g);
+      lists.emplace_back();
+      group_tri = m.tri;
+      group_smem = m.smem;
+    }
+    c->clu.back().r = widened(c->clu.back().r);
+    lists.back().push_back(sc);
+    ok[m.s] = 2;
+  }
+  for (size_t k = 0; k < c->clu.size(); ++k) {
+    fw_ctx::CluGroup& g = c->clu[k];
+    CluScene* ds = nullptr;
+    if ((rc = upload(c, &ds, lists[k]))) return rc;
+    g.r.scene = ds;
+    g.r.patch = dp;
+    g.r.blob = db;
+    g.r.err = c->d_flags + fw_ctx::kFlagCluster;
+    g.r.withhold_cta = -1;
+    g.r.wait_limit = kCluWaitLimit;
+    if (g.r.grid) {
+      g.r.n_halo = n_halo;
+      const size_t nbox = 4 * (size_t)kCluBoxRing * g.r.ctas * g.r.nb;
+      if ((rc = dalloc(c, &g.r.ghalo, 2 * (size_t)n_halo)) || (rc = dalloc(c, &g.r.gbox, nbox))) return rc;
+      FW_CUDA(c, cudaMemsetAsync(g.r.ghalo, 0, sizeof(ulonglong2) * 2 * (size_t)n_halo, c->stream));
+      FW_CUDA(c, cudaMemsetAsync(g.r.gbox, 0, sizeof(unsigned long long) * nbox, c->stream));
+    }
+    g.scenes = (int)lists[k].size();
+    g.threads = clu_threads(g.r, shared);
+    g.smem = clu_layout(g.r);
+  }
+  FW_CUDA(c, cudaStreamSynchronize(c->stream));
+  for (int s = 0; s < S; ++s)
+    if (ok[s] != 2) c->rest_scenes.push_back(s);
+  if (!c->rest_scenes.empty()) {  // their patches go to the stream kernels
+    std::vector<int32_t> plist;
+    std::vector<int4> rng(S, make_int4(0, 0, 0, 0));
+    for (int s : c->rest_scenes) {  // bodies and pairs as ranges: k_control_scenes needs them contiguous
+      const CluScene& sc = scenes[s];
+      if (sc.body0 < 0 || ok[s] == 0) {
+        c->clu.clear();
+        c->rest_scenes.clear();
+        return FW_OK;
+      }
+      rng[s] = make_int4(sc.body0, sc.nb, sc.pair0, sc.np);
+    }
+    std::vector<StreamPatch> sp(c->st_P);
+    FW_CUDA(c, cudaMemcpy(sp.data(), c->sd.patch, sizeof(StreamPatch) * c->st_P, cudaMemcpyDeviceToHost));
+    for (int p = 0; p < c->st_P; ++p)
+      if (ok[sp[p].scene] != 2) plist.push_back(p);
+    int32_t* dl = nullptr;
+    if ((rc = upload(c, &dl, plist)) || (rc = upload(c, &c->d_rest_scenes, c->rest_scenes)) ||
+        (rc = upload(c, &c->d_rest_rng, rng)))
+      return rc;
+    c->sd.list = dl;
+    c->rest_patches = (int)plist.size();
+    FW_CUDA(c, cudaStreamSynchronize(c->stream));
+  }
+  c->clu_patches = (int)patches.size();
+  const size_t G = c->clu.size();
+  while (c->side_streams.size() + 1 < G) {
+    cudaStream_t st = nullptr;
+    FW_CUDA(c, cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    c->side_streams.push_back(st);
+  }
+  while (G > 1 && c->side_events.size() < G) {
+    cudaEvent_t ev = nullptr;
+    FW_CUDA(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    c->side_events.push_back(ev);
+  }
+  return FW_OK;
+}
+
+// The resident patches, laid out when they are first needed (> 0: they do not fit).
+int own_resident(fw_ctx* c) {
+  if (c->path != FW_PATH_RESIDENT || c->res.err) return FW_OK;
+  const int rc = build_resident(c, c->lists.off, c->lists.slot, c->lists.x0, c->d.has_j2 != 0);
+  if (rc < 0) return rc;
+  FW_CUDA(c, cudaStreamSynchronize(c->stream));
+  return rc;
+}
+
+// Back to the path's own kernels for every scene.
+int cluster_off(fw_ctx* c) {
+  if (c->clu.empty()) return FW_OK;
+  const int rc = own_resident(c);
+  if (rc < 0) return rc;
+  if (rc > 0) c->path = FW_PATH_GATHER;
+  c->clu.clear();
+  c->rest_scenes.clear();
+  c->sd.list = nullptr;
+  drop_graphs(c);
+  return FW_OK;
+}
+
+// From here on the scenes' triangles carry their own Lame constants.
+int cluster_per_tri(fw_ctx* c) {
+  int optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+  for (fw_ctx::CluGroup& g : c->clu) {
+    if (g.r.per_tri) continue;
+    g.r.per_tri = 1;
+    g.smem = clu_layout(g.r);
+    if (g.smem + kCluStatic > (size_t)optin || !clu_fits(g.r, g.threads, g.smem)) return cluster_off(c);
+  }
+  return FW_OK;
+}
+
+// n substeps of every cluster-resident scene: the groups side by side (forked
+// from the context stream and joined to it), reading x_in / j2_in and leaving
+// the state in x_out / j2_out.
+int launch_cluster(fw_ctx* c, int n, const float2* x_in, float2* x_out, const float4* j2_in, float4* j2_out,
+                   const CluRun* runs, bool direct) {
+  const size_t G = c->clu.size();
+  if (G > 1 && !direct && n < (1 << 26)) {  // fork, launches and join as one graph: about 6 us of host work a group less
+    const uint64_t key = (3ull << 62) | ((uint64_t)(runs ? 1 : 0) << 61) | ((uint64_t)(x_in == c->x_buf0 ? 1 : 0) << 60) |
+                         ((uint64_t)(x_in == x_out ? 1 : 0) << 59) | ((uint64_t)(c->d.uniform_dt ? 1 : 0) << 58) |
+                         ((uint64_t)n << 32) | (c->d.uniform_dt ? float_bits(c->d.dt_uniform) : 0u);
+    const bool again = key == c->clu_last_key;
+    c->clu_last_key = key;
+    if (!again) return launch_cluster(c, n, x_in, x_out, j2_in, j2_out, runs, true);  // a graph pays from the second call on
+    cudaGraphExec_t g = nullptr;
+    int rc = FW_OK;
+    const int64_t before = c->launches;
+    const int rg = cached_graph(c, c->graphs, key,
+                                [&] { rc = launch_cluster(c, n, x_in, x_out, j2_in, j2_out, runs, true); }, &g);
+    c->launches = before;
+    if (rg || rc) return rg ? rg : rc;
+    FW_CUDA(c, cudaGraphLaunch(g, c->stream));
+    c->launches += (int64_t)G;
+    return FW_OK;
+  }
+  if (G > 1) FW_CUDA(c, cudaEventRecord(c->side_events[0], c->stream));
+  for (size_t k = 0; k < G; ++k) {
+    fw_ctx::CluGroup& g = c->clu[k];
+    cudaStream_t st = k == 0 ? c->stream : c->side_streams[k - 1];
+    if (k > 0) FW_CUDA(c, cudaStreamWaitEvent(st, c->side_events[0], 0));
+    CluLaunch r = g.r;
+    r.runs = runs;
+    r.wait_limit = c->wait_limit > 0 ? c->wait_limit : kCluWaitLimit;
+    r.withhold_cta = c->withhold_cta;
+    if (c->res.rec_x) {
+      r.rec_x = c->res.rec_x;
+      r.rec_v = c->res.rec_v;
+      r.rec_gates = c->res.rec_gates;
+      r.rec_stride = c->res.rec_stride;
+    }
+    cudaLaunchAttribute at[1];
+    if (r.grid) {  // every patch on an SM at once; this launch's tags follow the last one's
+      at[0].id = cudaLaunchAttributeCooperative;
+      at[0].val.cooperative = 1;
+      if (c->clu_epoch > 0xF0000000u) {  // about to wrap: clear the words, restart
+        FW_CUDA(c, cudaMemsetAsync(r.ghalo, 0, sizeof(ulonglong2) * 2 * (size_t)r.n_halo, st));
+        FW_CUDA(c, cudaMemsetAsync(r.gbox, 0, sizeof(unsigned long long) * 4 * kCluBoxRing * (size_t)r.ctas * r.nb, st));
+        c->clu_epoch = 0;
+      }
+      r.ep0 = c->clu_epoch;
+      c->clu_epoch += (uint32_t)n + 2u;
+    } else {
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = r.ctas;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(g.scenes * r.ctas);
+    cfg.blockDim = dim3(g.threads);
+    cfg.dynamicSmemBytes = g.smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = r.ctas > 1 ? 1 : 0;
+    FW_CUDA(c, cudaLaunchKernelEx(&cfg, clu_kernel(g.threads, r.one, r.grid), (const Dev)c->d, (const CluLaunch)r, x_in, x_out, j2_in, j2_out, n));
+    c->launches += 1;
+    if (k > 0) {
+      FW_CUDA(c, cudaEventRecord(c->side_events[k], st));
+      FW_CUDA(c, cudaStreamWaitEvent(c->stream, c->side_events[k], 0));
+    }
+  }
+  return check_kernel(c, "cluster step");
+}
+
 // Build the patches of the resident path; returns FW_OK, or a positive value
 // (with c->res_reason) when the world does not fit and the gather path is used.
 int build_resident(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<int32_t>& slot,
@@ -1764,6 +2389,10 @@ int build_resident(fw_ctx* c, const std::vector<int32_t>& off, const std::vector
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
   int P = c->patches_req > 0 ? c->patches_req : std::max(1, std::min(sms, (N + 127) / 128));
   if (P > N) P = N;
+  if ((int64_t)N * 40 + (int64_t)E * 64 > (int64_t)P * optin) {  // node state, corner forces and triangle records alone
+    c->res_reason = "patches of " + std::to_string(N / P) + " nodes do not fit in shared memory";
+    return 1;
+  }
   std::vector<int> idx(N), part(N, 0);
   for (int i = 0; i < N; ++i) idx[i] = i;
   rcb(x0, idx, 0, N, 0, P, part);
@@ -1904,8 +2533,7 @@ int build_resident(fw_ctx* c, const std::vector<int32_t>& off, const std::vector
   if ((rc = upload(c, &dpatch, patches)) || (rc = upload(c, &dn, rnodes)) || (rc = upload(c, &dh, rhalo)) ||
       (rc = upload(c, &de, reid)) || (rc = upload(c, &dc, rconn)) || (rc = upload(c, &dcp, rcsrp)) ||
       (rc = upload(c, &dcs, rcsrs)) || (rc = dalloc(c, &r.xpub, 2 * (size_t)N)) ||
-      (rc = dalloc(c, &r.aabb3, 12 * (size_t)c->B)) || (rc = dalloc(c, &r.bar, 1)) ||
-      (rc = dalloc(c, &r.err, 1)))
+      (rc = dalloc(c, &r.aabb3, 12 * (size_t)c->B)) || (rc = dalloc(c, &r.bar, 1)))
     return rc;
   if (ll) {
     const size_t nbll = 4 * (size_t)kBoxRing * c->B * P;
@@ -1922,7 +2550,7 @@ int build_resident(fw_ctx* c, const std::vector<int32_t>& off, const std::vector
   r.conn = dc;
   r.csr_ptr = dcp;
   r.csr_slot = dcs;
-  FW_CUDA(c, cudaMemsetAsync(r.err, 0, sizeof(int), c->stream));
+  r.err = c->d_flags + fw_ctx::kFlagResident;
   c->res_smem = smem;
   return FW_OK;
 }
@@ -1936,6 +2564,10 @@ int launch_resident(fw_ctx* c, int n) {
     n -= kMaxStepsPerLaunch;
   }
   if (n <= 0) return FW_OK;
+  if (!c->clu.empty()) {
+    c->host_counter += n;
+    return launch_cluster(c, n, c->d.x, c->d.x, c->d.j2state, c->d.j2state);
+  }
   const int step0 = (int)c->host_counter;
   const bool ll = c->res_ll;
   if (ll && c->res_epoch > 0xF0000000u) {  // epochs about to wrap: clear the words, restart
@@ -1962,36 +2594,32 @@ int launch_resident(fw_ctx* c, int n) {
   return check_kernel(c, "resident step");
 }
 
+// The error flags of the work queued so far (waits for it); a plain gather
+// world raises none.
 int check_device_error(fw_ctx* c) {
-  if (c->has_flex) {
-    int ferr = 0;
-    FW_CUDA(c, cudaMemcpyAsync(&ferr, c->d_flex_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    FW_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (ferr & 1)
-      return fail(c, FW_ERR_ARG, "FEM-FEM contact: a node received more than %d contact forces in one substep",
-                  kFlexListCap);
-  }
-  if (c->has_rigid) {
-    int rerr = 0;
-    FW_CUDA(c, cudaMemcpyAsync(&rerr, c->rd.err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    FW_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (rerr & 1)
-      return fail(c, FW_ERR_UNSUPPORTED,
-                  "a rigid body came within 0.01 of a ground or of another contact rigid (rigid-rigid and "
-                  "rigid-ground contact, the reference's constraint solve, are outside this library), or its "
-                  "state is no longer finite");
-  }
-  if (c->path == FW_PATH_STREAM && c->sd.err) {
-    int serr = 0;
-    FW_CUDA(c, cudaMemcpyAsync(&serr, c->sd.err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    FW_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (serr) return fail(c, FW_ERR_TIMEOUT, "stream step: a staged copy of triangle records did not complete");
-  }
-  if (c->path != FW_PATH_RESIDENT) return FW_OK;
-  int err = 0;
-  FW_CUDA(c, cudaMemcpyAsync(&err, c->res.err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  if (!c->has_flex && !c->has_rigid && c->clu.empty() && c->path == FW_PATH_GATHER) return FW_OK;
+  int flag[fw_ctx::kFlags];
+  FW_CUDA(c, cudaMemcpyAsync(flag, c->d_flags, sizeof(flag), cudaMemcpyDeviceToHost, c->stream));
   FW_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (err) return fail(c, FW_ERR_TIMEOUT, "resident step: a CTA gave up waiting for the others");
+  if (flag[fw_ctx::kFlagFlex] & 1)
+    return fail(c, FW_ERR_ARG, "FEM-FEM contact: a node received more than %d contact forces in one substep",
+                kFlexListCap);
+  if (flag[fw_ctx::kFlagRigid] & 1)
+    return fail(c, FW_ERR_UNSUPPORTED,
+                "a rigid body came within 0.01 of a ground or of another contact rigid (rigid-rigid and "
+                "rigid-ground contact, the reference's constraint solve, are outside this library), or its "
+                "state is no longer finite");
+  if (c->path == FW_PATH_STREAM && flag[fw_ctx::kFlagStream])
+    return fail(c, FW_ERR_TIMEOUT, "stream step: a staged copy of triangle records did not complete");
+  if (flag[fw_ctx::kFlagCluster]) {
+    FW_CUDA(c, cudaMemsetAsync(c->d_flags + fw_ctx::kFlagCluster, 0, sizeof(int), c->stream));
+    return fail(c, FW_ERR_TIMEOUT, "cluster step: a CTA gave up waiting for the others");
+  }
+  if (c->path == FW_PATH_RESIDENT && flag[fw_ctx::kFlagResident]) {
+    if (!c->clu.empty())  // no k_res_prologue clears it
+      FW_CUDA(c, cudaMemsetAsync(c->d_flags + fw_ctx::kFlagResident, 0, sizeof(int), c->stream));
+    return fail(c, FW_ERR_TIMEOUT, "resident step: a CTA gave up waiting for the others");
+  }
   return FW_OK;
 }
 
@@ -2415,6 +3043,8 @@ void fw_destroy(fw_ctx* c) {
   for (void* p : c->allocs) cudaFree(p);
   for (void* p : {(void*)c->d_echunk, (void*)c->d_epart, (void*)c->d_efirst, (void*)c->d_eout})
     if (p) cudaFree(p);
+  for (cudaStream_t st : c->side_streams) cudaStreamDestroy(st);
+  for (cudaEvent_t ev : c->side_events) cudaEventDestroy(ev);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;
 }
@@ -2972,12 +3602,11 @@ int build_flex(fw_ctx* c) {
       (rc = upload(c, &dslot, slot)) || (rc = dalloc(c, &dcnt, std::max(1, n_slots))) ||
       (rc = dalloc(c, &ditem, std::max(1, n_slots) * kFlexListCap)) ||
       (rc = dalloc(c, &dforce, std::max(1, n_slots) * kFlexListCap)) || (rc = dalloc(c, &c->d_flex_clock, n_fs)) ||
-      (rc = dalloc(c, &c->d_flex_err, 1)) || (rc = upload(c, &ptied, pair_tied)) ||
+      (rc = upload(c, &ptied, pair_tied)) ||
       (rc = upload(c, &telem, minus1)) || (rc = dalloc(c, &tw0, std::max(n_items, 1))) ||
       (rc = dalloc(c, &tw1, std::max(n_items, 1))) || (rc = dalloc(c, &tgap, std::max(n_items, 1))))
     return rc;
   FW_CUDA(c, cudaMemsetAsync(grid, 0, sizeof(FlexGrid) * n_fs, c->stream));
-  FW_CUDA(c, cudaMemsetAsync(c->d_flex_err, 0, sizeof(int), c->stream));
   FW_CUDA(c, cudaMemcpyAsync(c->d_flex_clock, c->flex_clock.data(), sizeof(double) * n_fs, cudaMemcpyHostToDevice,
                              c->stream));
   FW_CUDA(c, cudaMemsetAsync(dcnt, 0, sizeof(int32_t) * std::max(1, n_slots), c->stream));
@@ -2990,7 +3619,7 @@ int build_flex(fw_ctx* c) {
   f.cell_end = cend; f.cursor = cursor; f.sorted = sorted; f.crange = crange; f.ecell = ecell;
   f.srec = srec; f.scell = scell;
   f.seg = dseg; f.seg_off = dsegoff;
-  f.sc = dsc; f.clock_dt = c->d_flex_clock; f.err = c->d_flex_err;
+  f.sc = dsc; f.clock_dt = c->d_flex_clock; f.err = c->d_flags + fw_ctx::kFlagFlex;
   f.pair_tied = ptied; f.tie_elem = telem; f.tie_w0 = tw0; f.tie_w1 = tw1; f.tie_gap = tgap;
   c->flex_pre_smem = sizeof(float4) * (size_t)max_dom_fem;
   int optin = 0;
@@ -3124,6 +3753,7 @@ int fw_finalize(fw_ctx* c) {
     bcv[i] = make_float2(c->h_bcv[2 * i], c->h_bcv[2 * i + 1]);
   }
   // ---- device buffers
+  if (int rf = alloc_flags(c)) return rf;
   Dev& d = c->d;
   d.N = N; d.E = E; d.B = B; d.S = S; d.P = (int)pairs.size(); d.has_j2 = has_j2;
   int rc = 0;
@@ -3238,12 +3868,12 @@ int fw_finalize(fw_ctx* c) {
         (rc = dalloc(c, &r.item, (size_t)n_ritems)) || (rc = upload(c, &r.gbox, c->h_gbox)) ||
         (rc = upload(c, &r.gkind, c->h_gkind)) || (rc = upload(c, &r.rp_off, rp_off)) ||
         (rc = upload(c, &r.rp_rng, rp_rng)) || (rc = upload(c, &r.rs, rs)) ||
-        (rc = upload(c, &c->d_rclock, ck)) || (rc = dalloc(c, &r.count, S)) || (rc = dalloc(c, &r.err, 1)) ||
+        (rc = upload(c, &c->d_rclock, ck)) || (rc = dalloc(c, &r.count, S)) ||
         (rc = dalloc(c, &r.done, rs.size())))
       return rc;
     FW_CUDA(c, cudaMemsetAsync(r.count, 0, sizeof(int) * S, c->stream));
     FW_CUDA(c, cudaMemsetAsync(r.done, 0, sizeof(int) * rs.size(), c->stream));
-    FW_CUDA(c, cudaMemsetAsync(r.err, 0, sizeof(int), c->stream));
+    r.err = c->d_flags + fw_ctx::kFlagRigid;
     r.clock = c->d_rclock;
     d.rig = r.rig;
     d.ritem = r.item;
@@ -3268,18 +3898,25 @@ int fw_finalize(fw_ctx* c) {
   }
   if (c->path_req == FW_PATH_STREAM) {
     if ((rc = build_stream(c, off, slot, x0, has_j2))) return rc;
+    if ((rc = build_cluster(c, off, slot, x0, word, false))) return rc;
     c->path = FW_PATH_STREAM;
     FW_CUDA(c, cudaStreamSynchronize(c->stream));
   } else if (c->path_req != FW_PATH_GATHER) {
-    rc = build_resident(c, off, slot, x0, has_j2);
-    if (rc < 0) return rc;
-    if (rc == 0) {
+    if (S == 1 && c->patches_req == 0 && (rc = build_cluster(c, off, slot, x0, word, true))) return rc;
+    if (!c->clu.empty()) {
       c->path = FW_PATH_RESIDENT;
-    } else if (c->path_req == FW_PATH_RESIDENT) {
-      return fail(c, FW_ERR_ARG, "resident path requested but unavailable: %s", c->res_reason.c_str());
+    } else {
+      rc = build_resident(c, off, slot, x0, has_j2);
+      if (rc < 0) return rc;
+      if (rc == 0) {
+        c->path = FW_PATH_RESIDENT;
+      } else if (c->path_req == FW_PATH_RESIDENT) {
+        return fail(c, FW_ERR_ARG, "resident path requested but unavailable: %s", c->res_reason.c_str());
+      }
     }
     FW_CUDA(c, cudaStreamSynchronize(c->stream));
   }
+  if (!c->clu.empty() && S == 1) c->lists = HostLists{std::move(off), std::move(slot), std::move(x0)};
   c->finalized = true;
   return FW_OK;
 }
@@ -3315,12 +3952,14 @@ int fw_set_option(fw_ctx* c, int32_t option, int32_t value) {
         return fail(c, FW_ERR_ARG, "FW_OPT_FRONT_WARPS must be %s", c->res_threads == 1024 ? "8, 12 or 16 (1024 threads)"
                                                                                           : "2, 4, 6 or 8");
       c->front_warps = value;
+      c->shape_asked = true;
       return FW_OK;
     }
     case FW_OPT_RES_THREADS: {
       if (c->finalized) return fail(c, FW_ERR_STATE, "FW_OPT_RES_THREADS after fw_finalize");
       if (value != 512 && value != 1024) return fail(c, FW_ERR_ARG, "FW_OPT_RES_THREADS must be 512 or 1024");
       c->res_threads = value;
+      c->shape_asked = true;
       c->front_warps = value == 1024 ? 12 : 6;  // the default split for that size
       return FW_OK;
     }
@@ -3343,16 +3982,19 @@ int fw_set_option(fw_ctx* c, int32_t option, int32_t value) {
     case FW_OPT_WAIT_LIMIT:
       if (value < 0) return fail(c, FW_ERR_ARG, "FW_OPT_WAIT_LIMIT must be >= 0");
       c->wait_limit = value;
+      drop_graphs(c);  // they hold the limit
       return FW_OK;
     case FW_OPT_TEST_WITHHOLD:
       if (value < -1) return fail(c, FW_ERR_ARG, "FW_OPT_TEST_WITHHOLD must be >= -1");
       c->withhold_cta = value;
+      drop_graphs(c);
       return FW_OK;
     case FW_OPT_STREAM_PATCH: {
       if (c->finalized) return fail(c, FW_ERR_STATE, "FW_OPT_STREAM_PATCH after fw_finalize");
       if (value != 64 && value != 128) return fail(c, FW_ERR_ARG, "FW_OPT_STREAM_PATCH must be 64 or 128");
       c->st_nodes = value;
       c->st_minb = value == 64 ? 32 : 16;
+      c->shape_asked = true;
       return FW_OK;
     }
     case FW_OPT_STREAM_MINB: {
@@ -3361,6 +4003,9 @@ int fw_set_option(fw_ctx* c, int32_t option, int32_t value) {
                     c->st_nodes == 64 ? "16, 20, 24 or 32" : "8, 10, 12 or 16");
       c->st_minb = value;
       if (c->st_bulk && !stream_kernel(c->st_nodes, value, 1)) c->st_bulk = 0;  // loads-only budget
+      c->shape_asked = true;
+      if (!c->arena)
+        if (int rc = cluster_off(c)) return rc;
       drop_graphs(c);
       return FW_OK;
     }
@@ -3371,6 +4016,9 @@ int fw_set_option(fw_ctx* c, int32_t option, int32_t value) {
       if (value && !stream_kernel(c->st_nodes, c->st_minb, 1))
         return fail(c, FW_ERR_ARG, "FW_OPT_STREAM_BULK: no staged variant at %d CTAs per SM", c->st_minb);
       c->st_bulk = value;
+      c->shape_asked = true;
+      if (!c->arena)
+        if (int rc = cluster_off(c)) return rc;
       drop_graphs(c);
       return FW_OK;
     }
@@ -3378,7 +4026,14 @@ int fw_set_option(fw_ctx* c, int32_t option, int32_t value) {
       if (c->finalized) return fail(c, FW_ERR_STATE, "FW_OPT_RES_SYNC after fw_finalize");
       if (value != 0 && value != 1) return fail(c, FW_ERR_ARG, "FW_OPT_RES_SYNC must be 0 or 1");
       c->res_sync = value;
+      c->shape_asked = true;
       return FW_OK;
+    }
+    case FW_OPT_CLUSTER: {
+      if (value != 0 && value != 1) return fail(c, FW_ERR_ARG, "FW_OPT_CLUSTER must be 0 or 1");
+      if (c->finalized && value) return fail(c, FW_ERR_STATE, "FW_OPT_CLUSTER: clusters are laid out by fw_finalize");
+      c->clu_opt = value;
+      return value ? FW_OK : cluster_off(c);
     }
     default:
       return fail(c, FW_ERR_ARG, "fw_set_option: unknown option %d", option);
@@ -3396,6 +4051,7 @@ int fw_get_option(const fw_ctx* c, int32_t option, int32_t* value) {
     case FW_OPT_STREAM_MINB: *value = c->st_minb; return FW_OK;
     case FW_OPT_STREAM_BULK: *value = c->st_bulk; return FW_OK;
     case FW_OPT_RES_SYNC: *value = c->res_sync; return FW_OK;
+    case FW_OPT_CLUSTER: *value = c->clu.empty() ? 0 : (c->rest_scenes.empty() ? 1 : 2); return FW_OK;
     default: return FW_ERR_ARG;
   }
 }
@@ -3517,6 +4173,7 @@ int fw_arena_init(fw_ctx* c, int64_t max_nodes, int64_t max_elems, int32_t max_b
   c->cur_active.assign(S, 0);
   c->N = (int)N; c->E = (int)E; c->B = B; c->S = S;
   cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
+  if ((rc = alloc_flags(c))) return rc;
   c->arena = true;
   c->finalized = true;
   c->path = FW_PATH_GATHER;
@@ -3532,18 +4189,16 @@ int fw_arena_init(fw_ctx* c, int64_t max_nodes, int64_t max_elems, int32_t max_b
     uint16_t *dcp = nullptr, *dcs = nullptr;
     StreamElem* dse = nullptr;
     StreamNode* dsn = nullptr;
-    int* derr = nullptr;
     if ((rc = dalloc(c, &dp, Pcap)) || (rc = dalloc(c, &dn, N)) || (rc = dalloc(c, &dh, Hcap)) ||
         (rc = dalloc(c, &de, Tcap)) || (rc = dalloc(c, &dc, Tcap)) || (rc = dalloc(c, &dcp, CPcap)) ||
         (rc = dalloc(c, &dcs, 3 * E)) || (rc = dalloc(c, &dse, Tcap)) || (rc = dalloc(c, &dsn, N)) ||
-        (rc = dalloc(c, &derr, 1)) || (rc = dalloc(c, &c->d_plist, Pcap)) || (rc = dalloc(c, &c->d_budget, S)) ||
+        (rc = dalloc(c, &c->d_plist, Pcap)) || (rc = dalloc(c, &c->d_budget, S)) ||
         (rc = dalloc(c, &c->d_budget2, S)) || (rc = dalloc(c, &c->d_dt2, S)) ||
         (rc = dalloc(c, &c->d_slist, S)) || (rc = dalloc(c, &c->d_srng, S)) ||
         (rc = dalloc(c, &d.x_alt, N)) ||
         (rc = dalloc(c, &d.j2_alt, E)))
       return rc;
-    FW_CUDA(c, cudaMemsetAsync(derr, 0, sizeof(int), c->stream));
-    c->sd = StreamDev{dp, dn, dh, de, dc, dcp, dcs, 1, 1, 1, dse, dsn, derr, c->d_plist};
+    c->sd = StreamDev{dp, dn, dh, de, dc, dcp, dcs, 1, 1, 1, dse, dsn, c->d_flags + fw_ctx::kFlagStream, c->d_plist};
     c->fl_patch.init(Pcap);
     c->fl_halo.init(Hcap);
     c->fl_ptri.init(Tcap);
@@ -3833,6 +4488,7 @@ int fw_set_element_young(fw_ctx* c, int32_t first, int32_t count, const float* y
   k_set_young<<<(count + kBlock - 1) / kBlock, kBlock, 0, c->stream>>>(c->d, dst, c->d_poisson, first, first + count);
   c->launches += 1;
   if ((rc = check_kernel(c, "set young"))) return rc;
+  if ((rc = cluster_per_tri(c))) return rc;
   if (c->path != FW_PATH_STREAM) return FW_OK;
   // a body's triangles may now differ: the stream records take their Lame
   // constants per triangle from here on
@@ -3879,6 +4535,9 @@ int fw_adj_begin(fw_ctx* c, int32_t max_segment_steps) {
   // Resident reverse pass when the world runs resident and the adjoint state
   // fits on chip too (J2 worlds reverse on the gather kernels).
   if (c->path == FW_PATH_RESIDENT && !c->res_adj && !c->d.has_j2) {
+    if (!c->clu.empty() && (rc = own_resident(c)) < 0) return rc;
+  }
+  if (c->path == FW_PATH_RESIDENT && !c->res_adj && !c->d.has_j2 && c->res.err) {
     int optin = 0, sms = 148;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
@@ -4077,7 +4736,7 @@ int fw_tan_read(fw_ctx* c, float* dx, float* dv, int32_t on_device) {
 int fw_get_path(const fw_ctx* c, int32_t* path, int32_t* patches) {
   if (!c || !path) return FW_ERR_ARG;
   *path = c->finalized ? c->path : FW_PATH_AUTO;
-  if (patches) *patches = c->path == FW_PATH_RESIDENT ? c->res.P : (c->path == FW_PATH_STREAM ? c->st_P : 0);
+  if (patches) *patches = !c->clu.empty() && c->rest_scenes.empty() ? c->clu_patches : (c->path == FW_PATH_RESIDENT ? c->res.P : (c->path == FW_PATH_STREAM ? c->st_P : 0));
   return FW_OK;
 }
 
@@ -4098,6 +4757,27 @@ int fw_step_scenes(fw_ctx* c, int32_t n_steps, const float* dt) {
   if (rc) return rc;
   c->d.uniform_dt = 0;
   return run_steps(c, n_steps);
+}
+
+int fw_step_runs(fw_ctx* c, int32_t n_runs, const int32_t* counts, const float* dts) {
+  if (!c || !counts || !dts) return FW_ERR_ARG;
+  if (!c->finalized) return fail(c, FW_ERR_STATE, "fw_step_runs before fw_finalize");
+  if (n_runs < 1 || n_runs > kCluRuns) return fail(c, FW_ERR_ARG, "fw_step_runs: n_runs outside [1, %d]", kCluRuns);
+  if (c->path != FW_PATH_STREAM || c->clu.empty() || !c->rest_scenes.empty())
+    return fail(c, FW_ERR_STATE, "fw_step_runs: not every scene of the world is stepped on chip (FW_OPT_CLUSTER)");
+  std::vector<CluRun> runs(c->S, CluRun{});
+  for (int s = 0; s < c->S; ++s)
+    for (int k = 0; k < n_runs; ++k) {
+      const int n = counts[(size_t)s * n_runs + k];
+      if (n < 0) return fail(c, FW_ERR_ARG, "fw_step_runs: scene %d: count < 0", s);
+      runs[s].n[k] = n;
+      runs[s].dt[k] = dts[(size_t)s * n_runs + k];
+    }
+  int rc;
+  if (!c->d_runs && (rc = dalloc(c, &c->d_runs, c->S))) return rc;
+  // pageable source: staged before the call returns; on the stream, after the last launch that read the buffer
+  FW_CUDA(c, cudaMemcpyAsync(c->d_runs, runs.data(), sizeof(CluRun) * c->S, cudaMemcpyHostToDevice, c->stream));
+  return launch_cluster(c, 0, c->d.x, c->d.x, c->d.j2state, c->d.j2state, c->d_runs);
 }
 
 int fw_set_active(fw_ctx* c, const int32_t* active) {

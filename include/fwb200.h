@@ -311,9 +311,21 @@ int fw_set_path(fw_ctx* ctx, int32_t path, int32_t patches);
  * 6 or 8 of 16 warps (default 6), or 8, 12 or 16 of 32 (default 12).  Same
  * bits. */
 #define FW_OPT_RES_THREADS 11
+/* FW_OPT_CLUSTER: 1 (default) steps scenes that fit on chip patch by patch, all
+ * substeps of a call in one launch: a single scene of the resident path on up
+ * to one patch per SM, and every scene of the stream path that fits the shared
+ * memory of a thread-block cluster, each on its own.  0 leaves every scene to
+ * the path's own kernels, also when set after fw_finalize.  Setting a launch
+ * shape of the resident or stream step (FRONT_WARPS, RES_THREADS, RES_SYNC,
+ * STREAM_PATCH / MINB / BULK, or a patch count in fw_set_path) has the same
+ * effect, and so have more than 8 bodies or 32 contact pairs in a scene.  Same
+ * bits.  fw_get_option: 0 none, 1 every scene, 2 some scenes of the world are
+ * stepped this way. */
+#define FW_OPT_CLUSTER 12
 int fw_set_option(fw_ctx* ctx, int32_t option, int32_t value);
 /* The value an option has now.  Readable: FRONT_WARPS, RES_THREADS,
- * BLOCK_ELEMS, BLOCK_NODES, STREAM_PATCH, STREAM_MINB, STREAM_BULK, RES_SYNC;
+ * BLOCK_ELEMS, BLOCK_NODES, STREAM_PATCH, STREAM_MINB, STREAM_BULK, RES_SYNC,
+ * CLUSTER;
  * FW_ERR_ARG for the others.  No reference counterpart (a tuning readout). */
 int fw_get_option(const fw_ctx* ctx, int32_t option, int32_t* value);
 
@@ -338,6 +350,15 @@ int fw_step(fw_ctx* ctx, int32_t n_steps, float dt);
 /* Like fw_step with a per-scene dt[] (float32, n_scenes entries) for the
  * batched and served forms, where each scene has its own step. */
 int fw_step_scenes(fw_ctx* ctx, int32_t n_steps, const float* dt_per_scene);
+
+/* Every active scene s advances through its own runs in one call: counts[s *
+ * n_runs] substeps of dts[s * n_runs], then counts[s * n_runs + 1] of dts[s *
+ * n_runs + 1], ... (1 <= n_runs <= 4, counts >= 0).  For stream worlds whose
+ * scenes are all stepped on chip (fw_get_option(FW_OPT_CLUSTER) = 1); FW_ERR_STATE
+ * otherwise.  Same bits as the fw_step_scenes calls that stop at each scene's
+ * ends.  Replaces the per-loop advanceWithTime calls of independent scenes,
+ * flatworld/explicitloop.py:558-589. */
+int fw_step_runs(fw_ctx* ctx, int32_t n_runs, const int32_t* counts, const float* dts);
 
 /* One substep for a served world: scene s advances by dt[s] if dt[s] > 0 and
  * is frozen otherwise (dt has one entry per scene; for an arena world

@@ -1,0 +1,169 @@
+"""Scenes stepped on chip patch by patch (fw_cluster.cuh) against the gather and
+stream steps: same bits, at the sizes where the patches, halos, corner slots
+and cluster sizes change, and through every gate decision."""
+
+import numpy as np
+import pytest
+
+import flatworld_b200 as fw
+from flatworld_b200 import _native
+from flatworld_b200.batch import BatchedLoop
+from tests import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _rectangle(nx, ny, mat, ground, cell=0.02, **kw):
+    conn, coords = fw.structured_rectangle(nx, ny, nx * cell, ny * cell, origin=(0.0, 0.0), jitter=0.1, seed=nx)
+    fem = fw.FemDomain(fw.Mesh(2, conn, coords), fw.SolidProp(mat), [fw.Gravity([0.0, -9.8])],
+                       initials=[fw.InitialVel("ALL", [0.1, -1.0])], **kw)
+    return [ground, fem] if ground is not None else [fem]
+
+
+def _plane(y=-0.005):
+    return fw.GroundDomain(2, [0.0, y], [0.0, 1.0])
+
+
+def _bump(lo, hi):
+    xs = np.linspace(lo, hi, 64)
+    return fw.HeightFieldDomain(2, (0.01 * np.sin(40 * xs) - 0.015).astype(np.float32), lb=[lo, -1.0], ub=[hi, 1.0])
+
+
+MATS = {"elastic": fw.Elastic(5e4, 0.3, 500.0), "neohookean": fw.HyperElastic(5e4, 0.3, 500.0),
+        "mises": fw.MisesPlastic(5e4, 0.3, 500.0, sigma_y=300.0, H=5e3)}
+
+
+def _disk():
+    """A fan around one node (24 corners on it) inside a ring: more corner slots than a structured mesh needs."""
+    n = 24
+    a = 2 * np.pi * np.arange(n) / n
+    pts = np.concatenate([[[0.0, 0.0]], *[r * np.stack([np.cos(a), np.sin(a)], 1) for r in (0.05, 0.1, 0.15)]])
+    tri = [[0, 1 + i, 1 + (i + 1) % n] for i in range(n)]
+    for ring in range(2):
+        for i in range(n):
+            p, q = 1 + ring * n + i, 1 + ring * n + (i + 1) % n
+            tri += [[p, p + n, q], [q, p + n, q + n]]
+    mesh = fw.Mesh(2, np.asarray(tri, np.int32), (pts + [0.0, 0.151]).astype(np.float32))
+    return [_plane(0.0), fw.FemDomain(mesh, fw.SolidProp(MATS["neohookean"]), [fw.Gravity([0.0, -9.8])])]
+
+
+SINGLE = {
+    "one patch": lambda: _rectangle(3, 2, MATS["elastic"], _plane()),
+    "two patches": lambda: _rectangle(15, 8, MATS["neohookean"], _plane()),
+    "a thread per triangle, J2": lambda: _rectangle(60, 31, MATS["mises"], _plane()),
+    "several triangles per thread": lambda: _rectangle(260, 251, MATS["neohookean"], _plane(), cell=0.004),
+    "nodes of many corners": _disk,
+    "no pairs": lambda: _rectangle(40, 17, MATS["mises"], None),
+    "seven bodies": lambda: scenes.multi_block_scene(fw, 7),
+    "boundary conditions": lambda: scenes.bcs_scene(fw),
+    "forces from outside the gate box": lambda: _rectangle(40, 30, MATS["neohookean"], _bump(0.25, 0.55)),
+    "nodes below the gate box": lambda: _rectangle(20, 20, MATS["elastic"], _plane(0.12)),
+    "voxels": lambda: scenes.voxel_disk_scene(fw),
+}
+
+
+def _same(a, b, energy=True):
+    pa, pb = a._packed, b._packed
+    na, nb = a._native, b._native
+    for field in (_native.FW_FIELD_X, _native.FW_FIELD_V):
+        assert np.array_equal(na.read_nodes(field, 0, pa.N), nb.read_nodes(field, 0, pb.N), equal_nan=True)
+    for u, v in zip(na.read_plastic(pa.E), nb.read_plastic(pb.E)):
+        assert np.array_equal(u, v, equal_nan=True)
+    assert np.array_equal(na.read_aabb(pa.B), nb.read_aabb(pb.B))
+    assert np.array_equal(na.read_counters(pa.S), nb.read_counters(pb.S))
+
+
+@pytest.mark.parametrize("name", SINGLE)
+def test_single_scene_bitwise(name):
+    a = fw.ExplicitLoop(0.0, SINGLE[name](), damping=0.02)
+    b = fw.ExplicitLoop(0.0, SINGLE[name](), damping=0.02, path="gather")
+    assert a._native.get_option(_native.FW_OPT_CLUSTER) == 1 and a.path == 2
+    for lp in (a, b):
+        lp.enable_cfl_monitor()
+        lp.advance()
+        for n in (2, 17, 150):
+            lp.advance_n(n)
+    _same(a, b)
+    assert a.currentStableTime() == b.currentStableTime()
+    for lp in (a, b):  # positions set between calls: the next gates still use the last substep's boxes
+        x = lp._native.read_nodes(_native.FW_FIELD_X, 0, lp._packed.N)
+        lp._native.write_nodes(_native.FW_FIELD_X, 0, x + np.float32([0.0, 0.01]))
+        lp.advance_n(3)
+    _same(a, b)
+
+
+def test_moduli_per_triangle_and_set_later():
+    def build(path="auto"):
+        doms = _rectangle(40, 20, MATS["neohookean"], _plane())
+        doms[1].elementYoung = np.linspace(4e4, 6e4, doms[1].nelements).astype(np.float32)
+        return fw.ExplicitLoop(1e-4, doms, useAdapativeDT=False, path=path)
+
+    a, b = build(), build("gather")
+    u, v = (fw.ExplicitLoop(1e-4, _rectangle(40, 20, MATS["mises"], _plane()), useAdapativeDT=False, path=p)
+            for p in ("auto", "gather"))
+    for lp in (a, b, u, v):
+        lp.advance_n(40)
+        lp._native.set_element_young(np.linspace(6e4, 4e4, lp._packed.E).astype(np.float32))
+        lp.advance_n(40)
+    assert all(lp._native.get_option(_native.FW_OPT_CLUSTER) == 1 for lp in (a, u))
+    _same(a, b)
+    _same(u, v)
+
+
+def _batch(sizes):
+    out = []
+    for k, (nx, ny) in enumerate(sizes):
+        mat = list(MATS.values())[k % 3]
+        out.append(_rectangle(nx, ny, mat, _plane() if k % 2 else _bump(-1.0, 6.0),
+                              cell=0.01))
+    return out
+
+
+@pytest.mark.parametrize("sizes,covered", [
+    ([(4, 3), (9, 9), (30, 20), (60, 40), (100, 60), (130, 90)], 1),  # clusters of 1 to 16
+    ([(9, 9), (200, 160), (30, 20)], 2),  # one scene too large for a cluster: the stream kernels step it
+    ([(8, 5 + k % 7) for k in range(70)], 1),
+], ids=["cluster sizes", "one too large", "many small"])
+def test_batch_bitwise(sizes, covered):
+    a = BatchedLoop(_batch(sizes), dt=5e-5, useAdapativeDT=False)
+    b = BatchedLoop(_batch(sizes), dt=5e-5, useAdapativeDT=False, stream_patch=64)
+    assert a._native.get_option(_native.FW_OPT_CLUSTER) == covered
+    assert b._native.get_option(_native.FW_OPT_CLUSTER) == 0
+    frozen = np.ones(len(sizes), np.int32)
+    frozen[::3] = 0
+    for lp in (a, b):
+        lp._packed = lp.packed
+        lp.advance(1)
+        lp._set_active(frozen)
+        lp.advance(7)
+        lp._set_active(np.ones(len(sizes), np.int32))
+        lp.advance(64)
+        lp.advanceWithTime(3.3e-4)
+    _same(a, b)
+    a._native.set_option(_native.FW_OPT_CLUSTER, 0)  # the path's own kernels go on from the same state
+    for lp in (a, b):
+        lp.advance(9)
+    _same(a, b)
+
+
+def test_wait_runs_out_and_the_context_recovers():
+    lp = fw.ExplicitLoop(0.0, SINGLE["two patches"]())
+    lp.advance_n(20)
+    lp._native.set_option(_native.FW_OPT_WAIT_LIMIT, 4096)
+    lp._native.set_option(_native.FW_OPT_TEST_WITHHOLD, 1)
+    lp.advance_n(10)
+    with pytest.raises(RuntimeError, match="gave up"):
+        lp.synchronize()
+    lp._native.set_option(_native.FW_OPT_TEST_WITHHOLD, -1)
+    lp.advance_n(10)
+    lp.synchronize()
+    b = BatchedLoop(_batch([(60, 40), (9, 9), (61, 41)]), dt=5e-5, useAdapativeDT=False)
+    b.advance(20)
+    b._native.set_option(_native.FW_OPT_WAIT_LIMIT, 4096)
+    b._native.set_option(_native.FW_OPT_TEST_WITHHOLD, 1)
+    b.advance(10)
+    with pytest.raises(RuntimeError, match="gave up"):
+        b.synchronize()
+    b._native.set_option(_native.FW_OPT_TEST_WITHHOLD, -1)
+    b.advance(10)
+    b.synchronize()
