@@ -1056,7 +1056,10 @@ __device__ void node_energy(const Dev& d, int i, double& ke, double& ext, double
 }
 
 constexpr int kEnergyThreads = 256;
-constexpr int kEnergyChunk = 8192;
+// Nodes and triangles of a block.  The FP64 logarithm and divides of a NeoHookean
+// triangle set a block's time, so the blocks have to fill the SMs: chunks of
+// 8192 left 131072 triangles on 16 of them (92 us a report, 43 with 1024).
+constexpr int kEnergyChunk = 1024;
 
 // One block per chunk: fixed-order strided sums, then a fixed tree.
 __global__ void __launch_bounds__(kEnergyThreads) k_energy_chunks(Dev d, const EnergyChunk* ch, double4* part) {
@@ -1079,18 +1082,26 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy_chunks(Dev d, const E
   if (t == 0) part[blockIdx.x] = make_double4(sm[0][0], sm[1][0], sm[2][0], sm[3][0]);
 }
 
-// One thread per group: its chunks' partials in chunk order.
-__global__ void k_energy_groups(const int* first, int n_groups, const double4* part, double4* out) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= n_groups) return;
+// One block per group: strided sums of its chunks' partials, then a fixed tree.
+constexpr int kEnergyGroupThreads = 64;
+__global__ void __launch_bounds__(kEnergyGroupThreads) k_energy_groups(const int* first, const double4* part, double4* out) {
+  __shared__ double4 sm[kEnergyGroupThreads];
+  const int g = blockIdx.x, t = threadIdx.x;
   double4 s = make_double4(0.0, 0.0, 0.0, 0.0);
-  for (int k = first[g]; k < first[g + 1]; ++k) {
-    s.x += part[k].x;
-    s.y += part[k].y;
-    s.z += part[k].z;
-    s.w += part[k].w;
+  for (int k = first[g] + t; k < first[g + 1]; k += kEnergyGroupThreads) {
+    const double4 p = part[k];
+    s = make_double4(s.x + p.x, s.y + p.y, s.z + p.z, s.w + p.w);
   }
-  out[g] = s;
+  sm[t] = s;
+  __syncthreads();
+  for (int h = kEnergyGroupThreads / 2; h > 0; h >>= 1) {
+    if (t < h) {
+      const double4 a = sm[t], b = sm[t + h];
+      sm[t] = make_double4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+    }
+    __syncthreads();
+  }
+  if (t == 0) out[g] = sm[0];
 }
 
 }  // namespace
@@ -1264,6 +1275,8 @@ struct fw_ctx {
   int* d_efirst = nullptr;
   double4* d_eout = nullptr;
   size_t energy_cap = 0, energy_gcap = 0;
+  int energy_chunks = 0, energy_groups = 0;
+  bool energy_dirty = true;  // the chunks on the device are not those of the present scenes
   bool res_ll = false;       // resident path uses flag-in-data words
   uint32_t res_epoch = 1;    // epoch base of the next resident launch
   int path = FW_PATH_GATHER;
@@ -4268,6 +4281,7 @@ int fw_arena_commit_pack(fw_ctx* c, const fw_pack* pk, int32_t* scene_out) {
   const int s = c->free_scene_ids.back();
   c->free_scene_ids.pop_back();
   a.live = true;
+  c->energy_dirty = true;
   // upload (queued on the stream: the steps that follow see the scene, and a
   // pinned pack's copy runs asynchronously): the whole pack in one copy to
   // the device staging buffer, then one kernel puts each part in its range
@@ -4394,6 +4408,7 @@ int fw_arena_remove(fw_ctx* c, int32_t s) {
     c->fl_csrp.give(a.cp0, a.ncp);
   }
   a = fw_ctx::ArenaScene{};
+  c->energy_dirty = true;
   c->cur_active[s] = 0;
   c->free_scene_ids.push_back(s);
   c->chunks_dirty = true;
@@ -4891,54 +4906,63 @@ int fw_read_reference_shape(fw_ctx* c, float* area, float* jinv) {
 int fw_energy(fw_ctx* c, double* out) {
   if (!c || !out) return FW_ERR_ARG;
   if (!c->finalized) return fail(c, FW_ERR_STATE, "fw_energy before fw_finalize");
-  // groups: bodies (summed per scene below) or, in an arena, scene slots
-  struct Range { int n0, nn, e0, ne; };
-  std::vector<Range> groups;
-  if (c->arena) {
-    for (const fw_ctx::ArenaScene& a : c->ascenes)
-      groups.push_back(a.live ? Range{(int)a.n0, (int)a.nn, (int)a.e0, (int)a.ne} : Range{0, 0, 0, 0});
-  } else {
-    for (int b = 0; b < c->B; ++b) groups.push_back(Range{c->h_noff[b], c->h_ncnt[b], c->h_eoff[b], c->h_ecnt[b]});
-  }
-  const int G = (int)groups.size();
-  std::vector<EnergyChunk> chunks;
-  std::vector<int> first(G + 1, 0);
-  for (int g = 0; g < G; ++g) {
-    first[g] = (int)chunks.size();
-    const Range& r = groups[g];
-    const int n = std::max(1, (std::max(r.nn, r.ne) + kEnergyChunk - 1) / kEnergyChunk);
-    for (int k = 0; k < n; ++k) {
-      EnergyChunk ch;
-      ch.group = g;
-      ch.n0 = r.n0 + std::min(r.nn, k * kEnergyChunk);
-      ch.nn = std::max(0, std::min(kEnergyChunk, r.nn - k * kEnergyChunk));
-      ch.e0 = r.e0 + std::min(r.ne, k * kEnergyChunk);
-      ch.ne = std::max(0, std::min(kEnergyChunk, r.ne - k * kEnergyChunk));
-      chunks.push_back(ch);
+  // groups: bodies (summed per scene below) or, in an arena, scene slots; laid
+  // out once, and again after an arena's scenes changed
+  if (c->energy_dirty) {
+    struct Range { int n0, nn, e0, ne; };
+    std::vector<Range> groups;
+    if (c->arena) {
+      for (const fw_ctx::ArenaScene& a : c->ascenes)
+        groups.push_back(a.live ? Range{(int)a.n0, (int)a.nn, (int)a.e0, (int)a.ne} : Range{0, 0, 0, 0});
+    } else {
+      for (int b = 0; b < c->B; ++b) groups.push_back(Range{c->h_noff[b], c->h_ncnt[b], c->h_eoff[b], c->h_ecnt[b]});
     }
+    const int G = (int)groups.size();
+    std::vector<EnergyChunk> chunks;
+    std::vector<int> first(G + 1, 0);
+    for (int g = 0; g < G; ++g) {
+      first[g] = (int)chunks.size();
+      const Range& r = groups[g];
+      const int n = (std::max(r.nn, r.ne) + kEnergyChunk - 1) / kEnergyChunk;
+      for (int k = 0; k < n; ++k) {
+        EnergyChunk ch;
+        ch.group = g;
+        ch.n0 = r.n0 + std::min(r.nn, k * kEnergyChunk);
+        ch.nn = std::max(0, std::min(kEnergyChunk, r.nn - k * kEnergyChunk));
+        ch.e0 = r.e0 + std::min(r.ne, k * kEnergyChunk);
+        ch.ne = std::max(0, std::min(kEnergyChunk, r.ne - k * kEnergyChunk));
+        chunks.push_back(ch);
+      }
+    }
+    first[G] = (int)chunks.size();
+    const size_t nc = chunks.size();
+    if (nc > c->energy_cap || (size_t)G + 1 > c->energy_gcap) {
+      for (void* p : {(void*)c->d_echunk, (void*)c->d_epart, (void*)c->d_efirst, (void*)c->d_eout})
+        if (p) cudaFree(p);
+      c->d_echunk = nullptr;
+      c->d_epart = nullptr;
+      c->d_efirst = nullptr;
+      c->d_eout = nullptr;
+      c->energy_cap = c->energy_gcap = 0;
+      const size_t cap = std::max(nc, (size_t)64), gcap = std::max((size_t)G + 1, (size_t)64);
+      FW_CUDA(c, cudaMalloc((void**)&c->d_echunk, sizeof(EnergyChunk) * cap));
+      FW_CUDA(c, cudaMalloc((void**)&c->d_epart, sizeof(double4) * cap));
+      FW_CUDA(c, cudaMalloc((void**)&c->d_efirst, sizeof(int) * gcap));
+      FW_CUDA(c, cudaMalloc((void**)&c->d_eout, sizeof(double4) * gcap));
+      c->energy_cap = cap;
+      c->energy_gcap = gcap;
+    }
+    if (nc)
+      FW_CUDA(c, cudaMemcpyAsync(c->d_echunk, chunks.data(), sizeof(EnergyChunk) * nc, cudaMemcpyHostToDevice, c->stream));
+    FW_CUDA(c, cudaMemcpyAsync(c->d_efirst, first.data(), sizeof(int) * (G + 1), cudaMemcpyHostToDevice, c->stream));
+    c->energy_chunks = (int)nc;
+    c->energy_groups = G;
+    c->energy_dirty = false;
   }
-  first[G] = (int)chunks.size();
-  const size_t nc = chunks.size();
-  if (nc > c->energy_cap || (size_t)G + 1 > c->energy_gcap) {
-    for (void* p : {(void*)c->d_echunk, (void*)c->d_epart, (void*)c->d_efirst, (void*)c->d_eout})
-      if (p) cudaFree(p);
-    c->d_echunk = nullptr;
-    c->d_epart = nullptr;
-    c->d_efirst = nullptr;
-    c->d_eout = nullptr;
-    c->energy_cap = c->energy_gcap = 0;
-    const size_t cap = std::max(nc, (size_t)64), gcap = std::max((size_t)G + 1, (size_t)64);
-    FW_CUDA(c, cudaMalloc((void**)&c->d_echunk, sizeof(EnergyChunk) * cap));
-    FW_CUDA(c, cudaMalloc((void**)&c->d_epart, sizeof(double4) * cap));
-    FW_CUDA(c, cudaMalloc((void**)&c->d_efirst, sizeof(int) * gcap));
-    FW_CUDA(c, cudaMalloc((void**)&c->d_eout, sizeof(double4) * gcap));
-    c->energy_cap = cap;
-    c->energy_gcap = gcap;
-  }
-  FW_CUDA(c, cudaMemcpyAsync(c->d_echunk, chunks.data(), sizeof(EnergyChunk) * nc, cudaMemcpyHostToDevice, c->stream));
-  FW_CUDA(c, cudaMemcpyAsync(c->d_efirst, first.data(), sizeof(int) * (G + 1), cudaMemcpyHostToDevice, c->stream));
-  k_energy_chunks<<<(unsigned)nc, kEnergyThreads, 0, c->stream>>>(c->d, c->d_echunk, c->d_epart);
-  k_energy_groups<<<(G + 127) / 128, 128, 0, c->stream>>>(c->d_efirst, G, c->d_epart, c->d_eout);
+  const int G = c->energy_groups;
+  if (c->energy_chunks > 0)
+    k_energy_chunks<<<(unsigned)c->energy_chunks, kEnergyThreads, 0, c->stream>>>(c->d, c->d_echunk, c->d_epart);
+  k_energy_groups<<<G, kEnergyGroupThreads, 0, c->stream>>>(c->d_efirst, c->d_epart, c->d_eout);
   c->launches += 2;
   int rc = check_kernel(c, "energy");
   if (rc) return rc;
