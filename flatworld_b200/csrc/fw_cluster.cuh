@@ -680,7 +680,7 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
           for (int p = p_lo; p < p_hi; ++p) {
             const Pair& pr = s.pairs()[p];
             float2 cf;
-            const bool hit = pr.body - sc.body0 == body && fw::contact_force(pr, d.heights, d.occ, x, v, dt, cf);
+            const bool hit = pr.body - sc.body0 == body && fw::contact_force(pr, d.heights, d.occ, d.vox, x, v, dt, cf);
             bool on = k == 0 ? s.gate()[p] != 0
                              : x.x >= pr.glo[0] && x.x <= pr.ghi[0] && x.y >= pr.glo[1] && x.y <= pr.ghi[1];
             if (k > 0 && __any_sync(0xFFFFFFFFu, hit && !on))  // a force from outside the gate box: the gate itself

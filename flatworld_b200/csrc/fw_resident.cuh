@@ -259,7 +259,7 @@ __device__ __forceinline__ float2 res_node(const Dev& d, const ResSmem& s, const
     for (int q = 0; q < pn; ++q) {
       if (!s.gate[p0 + q]) continue;
       float2 cf;
-      if (fw::contact_force(s.pairs[p0 + q], heights, occ, x, v, dt, cf)) {
+      if (fw::contact_force(s.pairs[p0 + q], heights, occ, d.vox, x, v, dt, cf)) {
         f.x += cf.x;
         f.y += cf.y;
       }

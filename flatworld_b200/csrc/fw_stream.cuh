@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(NT, MINB) k_stream(Dev d, StreamDev sd, const 
       for (int k = 0; k < pn; ++k) {
         if (!d.pair_active[p0 + k]) continue;
         float2 cf;
-        if (fw::contact_force(d.pairs[p0 + k], d.heights, d.occ, x, v, dt, cf)) {
+        if (fw::contact_force(d.pairs[p0 + k], d.heights, d.occ, d.vox, x, v, dt, cf)) {
           f.x += cf.x;
           f.y += cf.y;
         }

@@ -24,6 +24,7 @@
 #include <atomic>
 #include <cstdarg>
 #include <map>
+#include <mutex>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -74,6 +75,7 @@ struct Dev {
   int32_t* pair_active;
   float* heights;
   int8_t* occ;
+  ushort4* vox;        // per voxel cell its nearest free cells (k_voxel_table); null: none
   float* scene_dt;
   float* scene_damp;
   int32_t* scene_counter;
@@ -446,7 +448,7 @@ __device__ __forceinline__ void node_step(const Dev& d, int i, bool valid) {
         }
         if (!d.pair_active[p0 + k]) continue;
         float2 cf;
-        if (fw::contact_force(d.pairs[p0 + k], d.heights, d.occ, x, v, dt, cf)) {
+        if (fw::contact_force(d.pairs[p0 + k], d.heights, d.occ, d.vox, x, v, dt, cf)) {
           f.x += cf.x;
           f.y += cf.y;
         }
@@ -630,6 +632,34 @@ __global__ void k_rigid_init(Rigid* rig, int n) {
   if (a >= n) return;
   fw::rigid_rot(rig[a]);
   if (rig[a].type != fw::RIGID_ANALYTICAL) fw::rigid_aabb(rig[a]);  // an analytical entry starts at getBBox()
+}
+
+// Per cell of the voxel pairs [p0, p0 + gridDim.x) the nearest free cells that
+// fw::contact_force looks for (zero for a cell that is not occupied): a block
+// per pair, a thread per row (walked both ways) and per column.
+__global__ void k_voxel_table(Dev d, int p0) {
+  const Pair pr = d.pairs[p0 + blockIdx.x];
+  if (pr.kind != fw::PAIR_VOXEL || pr.pad) return;
+  const int nx = pr.n0, ny = pr.n1;
+  const int8_t* g = d.occ + pr.table;
+  ushort4* w = d.vox + pr.table;
+  for (int line = threadIdx.x; line < nx + ny; line += blockDim.x) {
+    const bool col = line < ny;  // a line along i at j = line, or along j at i = line - ny
+    const int n = col ? nx : ny;
+    const size_t at = col ? (size_t)line : (size_t)(line - ny) * ny, step = col ? (size_t)ny : 1;
+    int free1 = 0;  // nearest free cell passed, + 1
+    for (int k = 0; k < n; ++k) {
+      const int8_t o = g[at + k * step];
+      (col ? w[at + k * step].x : w[at + k * step].z) = o == 1 ? (unsigned short)free1 : 0;
+      if (o == 0) free1 = k + 1;
+    }
+    int ahead = n;
+    for (int k = n - 1; k >= 0; --k) {
+      const int8_t o = g[at + k * step];
+      (col ? w[at + k * step].y : w[at + k * step].w) = o == 1 ? (unsigned short)ahead : 0;
+      if (o == 0) ahead = k;
+    }
+  }
 }
 
 // Reference-shape precompute, _prepare_fem_data_kernel
@@ -1049,7 +1079,7 @@ __device__ void node_energy(const Dev& d, int i, double& ke, double& ext, double
         if (depth < 0.0f) pen += 0.5 * (double)pr.penalty * (double)depth * (double)depth;
         continue;
       }
-      if (fw::contact_force(pr, d.heights, d.occ, x, make_float2(0.f, 0.f), 0.f, f))
+      if (fw::contact_force(pr, d.heights, d.occ, d.vox, x, make_float2(0.f, 0.f), 0.f, f))
         pen += 0.5 * ((double)f.x * f.x + (double)f.y * f.y) / (double)pr.penalty;
     }
   }
@@ -1112,6 +1142,40 @@ __global__ void __launch_bounds__(kEnergyGroupThreads) k_energy_groups(const int
 
 // ------------------------------------------------------------------ context
 
+// Page-locked blocks for reads into pageable memory, one to a context while
+// they last (a context without one reads as before), handed back when it goes.
+// They are parts of one allocation made for the first context: one costs the
+// driver as much as a dozen small reads.
+constexpr size_t kHostRead = 128 << 10;         // larger reads go to the caller's memory directly
+constexpr size_t kHostBlock = 256 + kHostRead;  // the error flags, then the data
+constexpr int kHostBlocks = 16;
+std::mutex host_blocks_lock;
+unsigned char* host_slab = nullptr;
+bool host_tried = false, host_taken[kHostBlocks] = {};
+
+unsigned char* take_host_block() {
+  std::lock_guard<std::mutex> hold(host_blocks_lock);
+  if (!host_tried) {
+    host_tried = true;
+    if (cudaHostAlloc((void**)&host_slab, kHostBlock * kHostBlocks, cudaHostAllocPortable) != cudaSuccess) {
+      host_slab = nullptr;
+      cudaGetLastError();
+    }
+  }
+  for (int k = 0; host_slab && k < kHostBlocks; ++k)
+    if (!host_taken[k]) {
+      host_taken[k] = true;
+      return host_slab + k * kHostBlock;
+    }
+  return nullptr;
+}
+
+void give_host_block(unsigned char* b) {
+  if (!b) return;
+  std::lock_guard<std::mutex> hold(host_blocks_lock);
+  host_taken[(size_t)(b - host_slab) / kHostBlock] = false;
+}
+
 // A node's corners (CSR, ascending 3 * triangle + corner) and the rest shape,
 // kept where a step may be laid out after fw_finalize.
 struct HostLists {
@@ -1120,6 +1184,7 @@ struct HostLists {
 };
 
 struct fw_ctx {
+  unsigned char* host = nullptr;  // a page-locked block (kHostBlock), or null
   int device = 0;
   std::string err;
   cudaStream_t own_stream = nullptr;
@@ -2609,11 +2674,35 @@ int launch_resident(fw_ctx* c, int n) {
 
 // The error flags of the work queued so far (waits for it); a plain gather
 // world raises none.
+bool raises_flags(const fw_ctx* c) {
+  return c->has_flex || c->has_rigid || !c->clu.empty() || c->path != FW_PATH_GATHER;
+}
+
+int report_flags(fw_ctx* c, const int* flag);
+
 int check_device_error(fw_ctx* c) {
-  if (!c->has_flex && !c->has_rigid && c->clu.empty() && c->path == FW_PATH_GATHER) return FW_OK;
-  int flag[fw_ctx::kFlags];
-  FW_CUDA(c, cudaMemcpyAsync(flag, c->d_flags, sizeof(flag), cudaMemcpyDeviceToHost, c->stream));
+  if (!raises_flags(c)) return FW_OK;
+  int local[fw_ctx::kFlags];
+  int* flag = c->host ? (int*)c->host : local;
+  FW_CUDA(c, cudaMemcpyAsync(flag, c->d_flags, sizeof(local), cudaMemcpyDeviceToHost, c->stream));
   FW_CUDA(c, cudaStreamSynchronize(c->stream));
+  return report_flags(c, flag);
+}
+
+// `bytes` of device memory into pageable host memory with the error flags in
+// the same trip; small reads go through the context's page-locked block, so
+// that the whole is one wait (the pageable copy and the flags took one each).
+int read_pageable(fw_ctx* c, void* dst, const void* src, size_t bytes) {
+  const bool flags = raises_flags(c) && c->host, small = c->host && bytes <= kHostRead;
+  if (flags)
+    FW_CUDA(c, cudaMemcpyAsync(c->host, c->d_flags, sizeof(int) * fw_ctx::kFlags, cudaMemcpyDeviceToHost, c->stream));
+  FW_CUDA(c, cudaMemcpyAsync(small ? c->host + 256 : dst, src, bytes, cudaMemcpyDeviceToHost, c->stream));
+  FW_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (small) memcpy(dst, c->host + 256, bytes);
+  return flags ? report_flags(c, (const int*)c->host) : check_device_error(c);
+}
+
+int report_flags(fw_ctx* c, const int* flag) {
   if (flag[fw_ctx::kFlagFlex] & 1)
     return fail(c, FW_ERR_ARG, "FEM-FEM contact: a node received more than %d contact forces in one substep",
                 kFlexListCap);
@@ -3032,6 +3121,7 @@ int fw_create(fw_ctx** out, int device) {
     return FW_ERR_CUDA;
   }
   c->stream = c->own_stream;
+  c->host = take_host_block();
   *out = c;
   return FW_OK;
 }
@@ -3056,6 +3146,7 @@ void fw_destroy(fw_ctx* c) {
   for (void* p : c->allocs) cudaFree(p);
   for (void* p : {(void*)c->d_echunk, (void*)c->d_epart, (void*)c->d_efirst, (void*)c->d_eout})
     if (p) cudaFree(p);
+  give_host_block(c->host);  // the stream is idle: nothing writes it any more
   for (cudaStream_t st : c->side_streams) cudaStreamDestroy(st);
   for (cudaEvent_t ev : c->side_events) cudaEventDestroy(ev);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
@@ -3216,6 +3307,7 @@ int fw_add_voxel_pair(fw_ctx* c, int32_t body, float penalty, const float* lo, c
   p.table = (int)c->h_occ.size();
   p.n0 = nx;
   p.n1 = ny;
+  p.pad = nx > 0xFFFF || ny > 0xFFFF ? 1 : 0;
   p.f[0] = lb_x;
   p.f[1] = lb_y;
   p.f[2] = dx;
@@ -3805,6 +3897,13 @@ int fw_finalize(fw_ctx* c) {
   k_prepare_elements<<<(E + kBlock - 1) / kBlock, kBlock, 0, c->stream>>>(d, dE, dnu, drho, 0, E);
   k_prepare_mass<<<(N + kBlock - 1) / kBlock, kBlock, 0, c->stream>>>(d, 0, N);
   c->launches += 2;
+  bool table = false;  // of the nearest free voxel cells
+  for (const Pair& p : pairs) table |= p.kind == fw::PAIR_VOXEL && !p.pad;
+  if (table) {
+    if ((rc = dalloc(c, &d.vox, c->h_occ.size()))) return rc;
+    k_voxel_table<<<(unsigned)pairs.size(), 256, 0, c->stream>>>(d, 0);
+    c->launches += 1;
+  }
   if ((rc = check_kernel(c, "prepare"))) return rc;
   if (c->has_springs) {  // a spring-mass domain's nodes carry its mass (femspringmanager.py:844-845)
     std::vector<float> sm(N);
@@ -4152,6 +4251,7 @@ int fw_arena_init(fw_ctx* c, int64_t max_nodes, int64_t max_elems, int32_t max_b
       (rc = dalloc(c, &d.aabb_ring, 8 * (size_t)B)) || (rc = dalloc(c, &c->a_young, E)) ||
       (rc = dalloc(c, &c->a_poisson, E)) || (rc = dalloc(c, &c->a_rho, E)) || (rc = dalloc(c, &d.scene_bad, S)))
     return rc;
+  if (max_occ > 0 && (rc = dalloc(c, &d.vox, max_occ))) return rc;
   FW_CUDA(c, cudaMemsetAsync(d.scene_bad, 0, sizeof(int32_t) * S, c->stream));
   c->stage_cap = (size_t)64 << 20;  // packs up to 64 MB commit in one copy (larger ones part by part)
   if ((rc = dalloc(c, &c->d_stage, c->stage_cap))) return rc;
@@ -4346,6 +4446,7 @@ int fw_arena_commit_pack(fw_ctx* c, const fw_pack* pk, int32_t* scene_out) {
   r.count = std::max<int64_t>({3 * a.ne, a.nn, a.nb, a.np, a.nhh, a.nt, a.npp});
   k_arena_reloc<<<(int)std::min<int64_t>((r.count + kBlock - 1) / kBlock, 8 * c->sms), kBlock, 0, c->stream>>>(d, r);
   const int e_lo = (int)e0, e_hi = (int)(e0 + a.ne), n_lo = (int)n0, n_hi = (int)(n0 + a.nn);
+  if (a.np > 0 && a.no > 0) k_voxel_table<<<(unsigned)a.np, 256, 0, c->stream>>>(d, (int)a.p0);
   k_prepare_elements<<<(int)((a.ne + kBlock - 1) / kBlock), kBlock, 0, c->stream>>>(d, c->a_young + e0, c->a_poisson + e0,
                                                                                   c->a_rho + e0, e_lo, e_hi);
   k_prepare_mass<<<(int)((a.nn + kBlock - 1) / kBlock), kBlock, 0, c->stream>>>(d, n_lo, n_hi);
@@ -4829,9 +4930,19 @@ int fw_read_nodes(fw_ctx* c, int32_t field, int32_t first, int32_t count, float*
     case FW_FIELD_MASS: src = c->d.mass + first; per = sizeof(float); break;
     default: return fail(c, FW_ERR_ARG, "fw_read_nodes: unknown field %d", field);
   }
+  if (count == 0) return fw_synchronize(c);
+  if (!on_device) {
+    cudaPointerAttributes at{};
+    const bool pinned = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    if (!pinned) return read_pageable(c, dst, src, per * count);
+  }
   FW_CUDA(c, cudaMemcpyAsync(dst, src, per * count,
                              on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, c->stream));
-  FW_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (!raises_flags(c)) {
+    FW_CUDA(c, cudaStreamSynchronize(c->stream));
+    return FW_OK;
+  }
   return check_device_error(c);
 }
 

@@ -44,11 +44,11 @@ class _DeviceNodeArray:
     def numpy(self):
         m = self._mgr
         shape = (m.MAX_NODES, self._width) if self._width > 1 else (m.MAX_NODES,)
-        out = np.zeros(shape, np.float32)
-        vals = m._native.read_nodes(self._field, m._n0, m._nn)
+        out = np.empty(shape, np.float32)
+        m._native.read_nodes_ptr(self._field, m._n0, m._nn, out.ctypes.data)
+        out[m._nn:] = 0.0
         if self._transform is not None:
-            vals = self._transform(vals)
-        out[: m._nn] = vals
+            out[: m._nn] = self._transform(out[: m._nn])
         return out
 
     @property

@@ -167,3 +167,36 @@ def test_wait_runs_out_and_the_context_recovers():
     b._native.set_option(_native.FW_OPT_TEST_WITHHOLD, -1)
     b.advance(10)
     b.synchronize()
+
+
+def _terrain_scene(nx, ny, kind):
+    """A block on (and partly inside) a voxel grid of nx x ny cells: solid, solid with cells of neither state, or
+    random."""
+    rng = np.random.default_rng(nx * 100 + ny)
+    if kind == "random":
+        occ = (rng.random((nx, ny)) < 0.4).astype(np.int32)
+    else:
+        top = rng.integers(ny // 2, ny + 1, nx)
+        occ = (np.arange(ny)[None, :] < top[:, None]).astype(np.int32)
+        if kind == "marked":
+            occ[rng.random((nx, ny)) < 0.1] = 5
+    lb = np.array([0.1, -0.02 * ny + 0.03], np.float32)
+    vox = fw.VoxelGridDomain(2, nx, ny, lb, lb + np.float32([0.02 * nx, 0.02 * ny]), occupancy_np=occ)
+    return _rectangle(24, 11, MATS["elastic"], vox, cell=0.03)
+
+
+@pytest.mark.parametrize("kind", ["solid", "marked", "random"])
+@pytest.mark.parametrize("nx,ny", [(1, 1), (37, 1), (1, 29), (31, 64), (130, 33)])
+def test_voxel_contact_matches_the_oracle(nx, ny, kind):
+    import oracle
+
+    o = oracle.OracleLoop(_terrain_scene(nx, ny, kind), 0.0, useAdapativeDT=True, threads=4)
+    loops = [fw.ExplicitLoop(0.0, _terrain_scene(nx, ny, kind), path=p) for p in ("auto", "gather")]
+    loops.append(fw.ExplicitLoop(0.0, _terrain_scene(nx, ny, kind), front_warps=6))
+    o.advance(60)
+    x, v, _ = o.state()
+    for lp in loops:
+        lp.advance_n(60)
+        n = lp._packed.N
+        assert np.array_equal(lp.femSpringManager.coords.numpy()[:n].astype(np.float64), x)
+        assert np.array_equal(lp.femSpringManager.V.numpy()[:n].astype(np.float64), v)
