@@ -107,6 +107,7 @@ struct CluRun {
 };
 
 struct CluScene {
+  int64_t blob0;  // arenas: its patches' byte offsets count from here
   int scene;
   int patch0;     // its patches: patch[patch0 .. + cluster size)
   int n0, e0;     // its first node and triangle
@@ -152,7 +153,7 @@ struct CluLaunch {
   float2* rec_v;
   int* rec_gates;
   int rec_stride;
-  const CluRun* runs;            // per scene of the world (null: nsteps substeps of the scene's dt)
+  const CluRun* runs;            // per scene of the launch (null: nsteps substeps of the scene's dt)
   // grid form
   ulonglong2* ghalo;             // [2][n_halo]
   unsigned long long* gbox;      // [kCluBoxRing][ctas][nb][4]
@@ -468,13 +469,15 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
   const CluPatch& Pg = r.patch[sc.patch0 + rank];
   const int S = sc.scene, no = Pg.no, ne = Pg.ne, nbnd = Pg.nbnd, first_cut = Pg.n_int,
             halo0 = Pg.halo0;
-  const int32_t* gid = reinterpret_cast<const int32_t*>(r.blob + Pg.gid);
-  const int32_t* eid = reinterpret_cast<const int32_t*>(r.blob + Pg.eid);
-  const uint2* tri = reinterpret_cast<const uint2*>(r.blob + Pg.tri);
+  const unsigned char* blob = r.blob + sc.blob0;
+  const int32_t* gid = reinterpret_cast<const int32_t*>(blob + Pg.gid);
+  const int32_t* eid = reinterpret_cast<const int32_t*>(blob + Pg.eid);
+  const uint2* tri = reinterpret_cast<const uint2*>(blob + Pg.tri);
+  const CluRun* runs = r.runs ? r.runs + (GRID ? 0 : blockIdx.x / C) : nullptr;
   int nsteps = n_all;
-  if (r.runs) {
+  if (runs) {
     nsteps = 0;
-    for (int j = 0; j < kCluRuns; ++j) nsteps += r.runs[S].n[j];
+    for (int j = 0; j < kCluRuns; ++j) nsteps += runs->n[j];
   }
   if (!d.scene_active[S] || nsteps <= 0) {  // every CTA of the scene leaves: the state stays (or moves over)
     if (x_in != x_out) {
@@ -493,8 +496,8 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
     s_abort = 0;
     s_cfl = 0x7f800000;
   }
-  const uint32_t* pos = reinterpret_cast<const uint32_t*>(r.blob + Pg.pos);
-  const uint32_t* info = reinterpret_cast<const uint32_t*>(r.blob + Pg.info);
+  const uint32_t* pos = reinterpret_cast<const uint32_t*>(blob + Pg.pos);
+  const uint32_t* info = reinterpret_cast<const uint32_t*>(blob + Pg.info);
   // a patch's triangles share one material unless the launch keeps it per triangle
   CluTri tr{};
   if (ne > 0) {
@@ -590,8 +593,8 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
     }
   {
     const int nh = Pg.nh, npush = Pg.npush;
-    const int32_t* hid = reinterpret_cast<const int32_t*>(r.blob + Pg.hid);
-    const uint32_t* push = reinterpret_cast<const uint32_t*>(r.blob + Pg.push);
+    const int32_t* hid = reinterpret_cast<const int32_t*>(blob + Pg.hid);
+    const uint32_t* push = reinterpret_cast<const uint32_t*>(blob + Pg.push);
     const int W = blockDim.x;
     if (!GRID) {
       for (int i = t; i < nh; i += W) {  // substep 0's halo; the other copy holds no tag that is waited for
@@ -618,9 +621,12 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
     if (nbnd == 0)
       for (int b = t; b <= sc.nb; b += W) s.bst()[b] = 0;
   }
-  float dt = r.runs ? r.runs[S].dt[0] : (d.uniform_dt ? d.dt_uniform : d.scene_dt[S]);
-  int run = 0, run_end = r.runs ? r.runs[S].n[0] : nsteps;  // dt holds for substeps [.., run_end)
+  float dt = runs ? runs->dt[0] : (d.uniform_dt ? d.dt_uniform : d.scene_dt[S]);
+  int run = 0, run_end = runs ? runs->n[0] : nsteps;  // dt holds for substeps [.., run_end)
   const float damp = d.scene_damp[S];
+  // a scene just committed to an arena: its first substep is the zero-dt
+  // construction step (no contact, no damping, not counted)
+  const int init = d.scene_mode_req[S] ? 1 : 0;
   const float* bcfl = d.cfl_ord ? d.body_cfl : nullptr;
   float cfl = __int_as_float(0x7f800000);
   bool bad = false;
@@ -648,13 +654,14 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
   if (control) {
     // ---- control warps: the boxes and the contact forces of the substep's start state
     const int ct = t - T, CT = 32 * r.ctl;
+    const int g0 = counter0 - init;
     for (int k = 0; k < nsteps; ++k) {
       while (k == run_end) {
-        dt = r.runs[S].dt[++run];
-        run_end += r.runs[S].n[run];
+        dt = runs->dt[++run];
+        run_end += runs->n[run];
       }
       if (sc.np > 0) {
-        const int g = counter0 + k;
+        const int g = g0 + k;
         if (ct < 32) {  // the first one keeps the boxes
           if (!(k == 1 && (int)blockIdx.x == r.withhold_cta)) clu_publish<GRID>(r, s, rank, sc.nb, bodies, k, lane);
           if (k % kCluBoxSync == 0 && k > 0 && C > 1)  // everyone has come this far
@@ -680,7 +687,7 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
           for (int p = p_lo; p < p_hi; ++p) {
             const Pair& pr = s.pairs()[p];
             float2 cf;
-            const bool hit = pr.body - sc.body0 == body && fw::contact_force(pr, d.heights, d.occ, d.vox, x, v, dt, cf);
+            const bool hit = pr.body - sc.body0 == body && k >= init && fw::contact_force(pr, d.heights, d.occ, d.vox, x, v, dt, cf);
             bool on = k == 0 ? s.gate()[p] != 0
                              : x.x >= pr.glo[0] && x.x <= pr.ghi[0] && x.y >= pr.glo[1] && x.y <= pr.ghi[1];
             if (k > 0 && __any_sync(0xFFFFFFFFu, hit && !on))  // a force from outside the gate box: the gate itself
@@ -700,8 +707,8 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
   } else {
     for (int k = 0; k < nsteps; ++k) {
       while (k == run_end) {
-        dt = r.runs[S].dt[++run];
-        run_end += r.runs[S].n[run];
+        dt = runs->dt[++run];
+        run_end += runs->n[run];
       }
       // ---- corner forces: interior triangles, then the cut ones as the halo arrives
       if (ONE) {
@@ -764,7 +771,8 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
           f = p2.add(f, make_float2(cq.x, cq.y));
           f = p2.add(f, make_float2(cq.z, cq.w));
         }
-        clu_integrate(p2, (int)(nd.w & fw::NODE_BC_MASK), f, nd.im, nd.b, dt, damp, nd.x, nd.v);
+        clu_integrate(p2, (int)(nd.w & fw::NODE_BC_MASK), f, nd.im, nd.b, k < init ? 0.0f : dt, k < init ? 0.0f : damp, nd.x,
+                      nd.v);
         if (!ONE) nd.to = (nd.w >> kCluPushCntShift) & 7u ? s.push()[nd.w >> kCluPushOffShift] : 0u;
         if (nd.to && send) {
           clu_send<GRID>(r, nd.to, copy, tag, nd.x);
@@ -793,12 +801,15 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
     clu_publish<GRID>(r, s, rank, sc.nb, bodies, nsteps, lane);
     __syncwarp();
     if (rank == 0) {
-      const int after = counter0 + nsteps;
+      const int after = counter0 + nsteps - init;
       for (int b = 0; b < sc.nb; ++b) {
         const int4 bb = clu_box<GRID>(r, s, b, nsteps, &s_abort);
         if (lane == 0) *reinterpret_cast<int4*>(d.aabb_ring + ((size_t)(after & 1) * d.B + sc.body0 + b) * 4) = bb;
       }
-      if (lane == 0) d.scene_counter[S] = after;
+      if (lane == 0) {
+        d.scene_counter[S] = after;
+        if (init) d.scene_mode_req[S] = 0;
+      }
     }
   }
   if (bad) d.scene_bad[S] = 1;

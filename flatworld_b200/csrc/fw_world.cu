@@ -45,6 +45,8 @@ namespace {
 constexpr int kBlock = 256;     // default block size of the gather kernels
 constexpr int kMaxBlock = 512;  // launch bound (block sizes are a runtime option)
 constexpr int kGraphSteps = 32;
+constexpr int kCluServedNodes = 256;  // nodes of a served scene's cluster patch: latency before throughput
+constexpr size_t kCluSharedBytes = 232448 - 64;  // of a CTA on sm_100
 constexpr int kCluMinSteps = 3;  // substeps of a call from which a stream world's scenes are stepped on chip
 
 struct Dev {
@@ -1255,6 +1257,9 @@ struct fw_ctx {
     int64_t n0 = 0, nn = 0, e0 = 0, ne = 0, b0 = 0, nb = 0, p0 = 0, np = 0, h0 = 0, nh = 0, o0 = 0, no = 0;
     // stream arenas: patches, halo nodes, patch triangles, corner-list offsets
     int64_t pp0 = 0, npp = 0, hh0 = 0, nhh = 0, t0 = 0, nt = 0, cp0 = 0, ncp = 0;
+    // ... and, where it fits a cluster, its cluster patches and their bytes
+    CluLaunch clu{};
+    int64_t cq0 = 0, ncq = 0, cb0 = 0, ncb = 0;
   };
   bool arena = false;
   FreeList fl_nodes, fl_elems, fl_bodies, fl_pairs, fl_heights, fl_occ;
@@ -1262,7 +1267,12 @@ struct fw_ctx {
   // records of each committed scene's patches; owned-node records use the
   // scene's node range and corner lists its 3 x triangle range
   bool a_stream = false;
-  FreeList fl_patch, fl_halo, fl_ptri, fl_csrp;
+  FreeList fl_patch, fl_halo, fl_ptri, fl_csrp, fl_cpatch, fl_cblob;
+  CluPatch* d_cpatch = nullptr;
+  unsigned char* d_cblob = nullptr;
+  CluScene* d_cscene = nullptr;  // the scenes of a call, in launch order
+  bool clu_size_ok[kCluMaxCtas + 1] = {};  // cluster sizes the device can hold
+  size_t clu_cap = 0;
   int32_t* d_plist = nullptr;     // the active scenes' patches (CTA -> patch)
   int32_t* d_budget = nullptr;    // fw_step_served_budget: per-scene substep budgets
   int32_t* d_budget2 = nullptr;   // ... of the second segment
@@ -1317,7 +1327,8 @@ struct fw_ctx {
   int32_t* d_rest_scenes = nullptr;
   int4* d_rest_rng = nullptr;
   int rest_patches = 0;
-  CluRun* d_runs = nullptr;  // fw_step_runs: every scene's runs
+  CluRun* d_runs = nullptr;  // fw_step_runs: every scene's runs, in the groups' order
+  std::vector<int> clu_order;  // the scenes in the groups' order
   int clu_patches = 0;
   uint64_t clu_last_key = 0;
   HostLists lists;
@@ -1563,6 +1574,7 @@ int arena_stream_steps(fw_ctx* c, int n);
 
 int launch_cluster(fw_ctx* c, int n, const float2* x_in, float2* x_out, const float4* j2_in, float4* j2_out,
                    const CluRun* runs = nullptr, bool direct = false);
+int arena_cluster_steps(fw_ctx* c, int n);
 
 int build_resident(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<int32_t>& slot,
                    const std::vector<float2>& x0, bool has_j2);
@@ -2103,22 +2115,52 @@ bool clu_fits(const CluLaunch& r, int threads, size_t smem) {
   return e == cudaSuccess && n >= 1;
 }
 
+// Streams and events for the groups after the first, which run beside it.
+int clu_side_streams(fw_ctx* c) {
+  const size_t G = c->clu.size();
+  while (c->side_streams.size() + 1 < G) {
+    cudaStream_t st = nullptr;
+    FW_CUDA(c, cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    c->side_streams.push_back(st);
+  }
+  while (G > 1 && c->side_events.size() < G) {
+    cudaEvent_t ev = nullptr;
+    FW_CUDA(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    c->side_events.push_back(ev);
+  }
+  return FW_OK;
+}
+
+// Shared memory a CTA may have, the kernels' attributes, and the cluster sizes
+// the device can hold with that much of it.
+int clu_prepare(fw_ctx* c, size_t* cap, bool* size_ok) {
+  int optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+  *cap = (size_t)optin - kCluStatic;
+  for (int grid = 0; grid < 2; ++grid)
+    for (int one = 0; one < 2; ++one)
+      for (int threads : {512, 1024}) {
+        CluKernel k = clu_kernel(threads, one, grid);
+        FW_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*cap));
+        if (!grid) FW_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      }
+  for (int k = 1; size_ok && k <= kCluMaxCtas; k *= 2) {
+    CluLaunch r{};
+    r.ctas = k;
+    size_ok[k] = clu_fits(r, kCluMaxThreads, *cap);
+  }
+  return FW_OK;
+}
+
 // Cut the world's scenes for clusters where they fit, group them into
 // launches, and (stream worlds) list what is left.  Leaves c->clu empty when
 // nothing fits.
 int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<int32_t>& slot,
                   const std::vector<float2>& x0, const std::vector<uint32_t>& word, bool single) {
   if (!c->clu_opt || c->shape_asked) return FW_OK;
-  int optin = 0;
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  const size_t cap = (size_t)optin - kCluStatic;
-  for (int grid = 0; grid < 2; ++grid)
-    for (int one = 0; one < 2; ++one)
-      for (int threads : {512, 1024}) {
-        CluKernel k = clu_kernel(threads, one, grid);
-        FW_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
-        if (!grid) FW_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-      }
+  size_t cap = 0;
+  bool size_ok[kCluMaxCtas + 1] = {};
+  if (int rp = clu_prepare(c, &cap, single ? nullptr : size_ok)) return rp;
   const int S = c->S;
   std::vector<CluScene> scenes(S);
   std::vector<int> nn(S, 0);
@@ -2128,7 +2170,7 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
     for (int b = 0; b < c->B; ++b) {
       CluScene& sc = scenes[c->h_scene[b]];
       if (sc.body0 < 0) {
-        sc = CluScene{c->h_scene[b], 0, c->h_noff[b], c->h_eoff[b], b, 0, 0, 0};
+        sc = CluScene{0, c->h_scene[b], 0, c->h_noff[b], c->h_eoff[b], b, 0, 0, 0};
         ok[sc.scene] = 1;
       }
       const int s = sc.scene;
@@ -2192,12 +2234,6 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
     std::vector<unsigned char> blob;
   };
   std::vector<Cut> cuts(S);
-  bool size_ok[kCluMaxCtas + 1] = {};  // cluster sizes that fit the device with all of an SM's shared memory
-  for (int k = 1; !single && k <= kCluMaxCtas; k *= 2) {
-    CluLaunch r{};
-    r.ctas = k;
-    size_ok[k] = clu_fits(r, kCluMaxThreads, cap);
-  }
   parallel_for(S, host_threads(), [&](int s) {
     if (!ok[s]) return;
     const int most = single ? sms : kCluMaxCtas;
@@ -2283,6 +2319,7 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
     }
     c->clu.back().r = widened(c->clu.back().r);
     lists.back().push_back(sc);
+    c->clu_order.push_back(m.s);
     ok[m.s] = 2;
   }
   for (size_t k = 0; k < c->clu.size(); ++k) {
@@ -2334,18 +2371,7 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
     FW_CUDA(c, cudaStreamSynchronize(c->stream));
   }
   c->clu_patches = (int)patches.size();
-  const size_t G = c->clu.size();
-  while (c->side_streams.size() + 1 < G) {
-    cudaStream_t st = nullptr;
-    FW_CUDA(c, cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    c->side_streams.push_back(st);
-  }
-  while (G > 1 && c->side_events.size() < G) {
-    cudaEvent_t ev = nullptr;
-    FW_CUDA(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    c->side_events.push_back(ev);
-  }
-  return FW_OK;
+  return clu_side_streams(c);
 }
 
 // The resident patches, laid out when they are first needed (> 0: they do not fit).
@@ -2414,6 +2440,7 @@ int launch_cluster(fw_ctx* c, int n, const float2* x_in, float2* x_out, const fl
     if (k > 0) FW_CUDA(c, cudaStreamWaitEvent(st, c->side_events[0], 0));
     CluLaunch r = g.r;
     r.runs = runs;
+    if (runs) runs += g.scenes;
     r.wait_limit = c->wait_limit > 0 ? c->wait_limit : kCluWaitLimit;
     r.withhold_cta = c->withhold_cta;
     if (c->res.rec_x) {
@@ -2839,7 +2866,7 @@ __global__ void k_arena_reloc(Dev d, ArenaReloc r) {
 
 // Parts of a pack copied from the device staging buffer to their arena
 // ranges: part k = stage[off[k] .. +len[k]) -> dst[k] (blockIdx.y = part).
-constexpr int kScatterParts = 27;  // the pack's parts and the rest positions again (as the current ones)
+constexpr int kScatterParts = 29;  // the pack's parts and the rest positions again (as the current ones)
 struct ArenaScatter {
   unsigned char* dst[kScatterParts];
   uint32_t off[kScatterParts];
@@ -2878,6 +2905,83 @@ int stream_attrs(fw_ctx* c, int optin) {
   return FW_OK;
 }
 
+// n substeps of an arena's active scenes that have cluster patches: each through
+// its own runs (its budget at its dt, then the next budget), one launch per
+// cluster size.
+int arena_cluster_steps(fw_ctx* c, int n) {
+  struct Item {
+    int s;
+    CluRun run;
+  };
+  std::vector<Item> items;
+  int64_t tris = 0;
+  for (size_t s = 0; s < c->ascenes.size(); ++s) {
+    const fw_ctx::ArenaScene& a = c->ascenes[s];
+    if (!a.live || !c->cur_active[s] || !a.clu.ctas) continue;
+    CluRun run{};
+    run.n[0] = c->d.scene_budget ? std::max(0, std::min(n, c->h_budget[s])) : n;
+    run.dt[0] = c->d.uniform_dt ? c->d.dt_uniform : c->cur_dt[s];
+    if (c->d.scene_budget_next) {
+      run.n[1] = std::max(0, std::min(n - run.n[0], c->h_budget2[s]));
+      run.dt[1] = c->h_dt2[s];
+    }
+    if (run.n[0] + run.n[1] == 0) continue;
+    items.push_back(Item{(int)s, run});
+    tris += a.ne;
+  }
+  c->clu.clear();
+  if (items.empty()) return FW_OK;
+  // the largest scenes first, so that the small ones fill in behind them
+  std::stable_sort(items.begin(), items.end(), [&](const Item& p, const Item& q) {
+    const CluLaunch &a = c->ascenes[p.s].clu, &b = c->ascenes[q.s].clu;
+    return a.ctas != b.ctas ? a.ctas > b.ctas : a.ne > b.ne;
+  });
+  const bool shared = tris > (int64_t)c->sms * 900;
+  std::vector<CluScene> scenes;
+  std::vector<CluRun> runs;
+  for (const Item& it : items) {
+    const fw_ctx::ArenaScene& a = c->ascenes[it.s];
+    auto widened = [&](CluLaunch r) {
+      const CluLaunch& b = a.clu;
+      r.no = std::max(r.no, b.no); r.nh = std::max(r.nh, b.nh); r.ne = std::max(r.ne, b.ne); r.deg = std::max(r.deg, b.deg);
+      r.npush = std::max(r.npush, b.npush); r.nbnd = std::max(r.nbnd, b.nbnd);
+      r.nb = std::max(r.nb, b.nb); r.np = std::max(r.np, b.np);
+      r.has_j2 |= b.has_j2; r.per_tri |= b.per_tri;
+      clu_threads(r, shared);
+      return r;
+    };
+    bool join = !c->clu.empty() && c->clu.back().r.ctas == a.clu.ctas && 4 * a.clu.ne > c->clu.back().r.ne;
+    if (join && clu_smem(widened(c->clu.back().r)) > c->clu_cap) join = false;
+    if (!join) {
+      fw_ctx::CluGroup g;
+      g.r.ctas = a.clu.ctas;
+      c->clu.push_back(g);
+    }
+    fw_ctx::CluGroup& g = c->clu.back();
+    g.r = widened(g.r);
+    g.scenes += 1;
+    scenes.push_back(CluScene{a.cb0, it.s, (int)a.cq0, (int)a.n0, (int)a.e0, (int)a.b0, (int)a.nb, (int)a.p0, (int)a.np});
+    runs.push_back(it.run);
+  }
+  // staged before the calls return
+  FW_CUDA(c, cudaMemcpyAsync(c->d_cscene, scenes.data(), sizeof(CluScene) * scenes.size(), cudaMemcpyHostToDevice, c->stream));
+  FW_CUDA(c, cudaMemcpyAsync(c->d_runs, runs.data(), sizeof(CluRun) * runs.size(), cudaMemcpyHostToDevice, c->stream));
+  const CluScene* at = c->d_cscene;
+  for (fw_ctx::CluGroup& g : c->clu) {
+    g.r.scene = at;
+    at += g.scenes;
+    g.r.patch = c->d_cpatch;
+    g.r.blob = c->d_cblob;
+    g.r.err = c->d_flags + fw_ctx::kFlagCluster;
+    g.threads = clu_threads(g.r, shared);
+    g.smem = clu_layout(g.r);
+  }
+  int rc = clu_side_streams(c);
+  if (!rc) rc = launch_cluster(c, n, c->d.x, c->d.x, c->d.j2state, c->d.j2state, c->d_runs, true);
+  c->clu.clear();
+  return rc;
+}
+
 // n substeps of a stream arena: k_control + k_stream over the active scenes'
 // patches each, then (n odd) the carry back into the first buffers.
 int arena_stream_steps(fw_ctx* c, int n) {
@@ -2886,7 +2990,7 @@ int arena_stream_steps(fw_ctx* c, int n) {
     c->h_slist.clear();
     for (size_t s2 = 0; s2 < c->ascenes.size(); ++s2) {
       const fw_ctx::ArenaScene& a = c->ascenes[s2];
-      if (!a.live || !c->cur_active[s2]) continue;
+      if (!a.live || !c->cur_active[s2] || (c->clu_opt && a.clu.ctas)) continue;
       c->h_slist.push_back((int32_t)s2);
       for (int64_t k = 0; k < a.npp; ++k) c->h_plist.push_back((int32_t)(a.pp0 + k));
     }
@@ -2902,7 +3006,10 @@ int arena_stream_steps(fw_ctx* c, int n) {
     c->chunks_dirty = false;
   }
   c->host_counter += n;
-  if (c->st_list_n == 0 || n <= 0) return FW_OK;
+  if (n <= 0) return FW_OK;
+  if (c->clu_opt && c->d_cpatch)
+    if (int rc = arena_cluster_steps(c, n)) return rc;
+  if (c->st_list_n == 0) return FW_OK;
   float2 *xa = c->d.x, *xb = c->d.x_alt;
   float4 *ja = c->d.j2state, *jb = c->d.j2_alt;
   const StreamKernel k = stream_kernel(c->st_nodes, c->st_minb, c->st_bulk);
@@ -2942,12 +3049,13 @@ int arena_stream_steps(fw_ctx* c, int n) {
 struct fw_pack {
   enum Part {
     X0, V0, BCV, WORD, CBEG, CEND, SLOT, CPOS, CONN, EMAT, J2PAR, YOUNG, POISSON, RHO, POFF, PCNT, PAIRS,
-    HEIGHTS, OCC, RN, RH, RE, RC, RCP, RCS, PATCH, NPARTS
+    HEIGHTS, OCC, RN, RH, RE, RC, RCP, RCS, PATCH, CPATCH, CBLOB, NPARTS
   };
   int64_t Ns = 0, Es = 0, Bs = 0, Np = 0, Nh = 0, No = 0;
   int64_t Ps = 0, Hs = 0, Ts = 0, CPs = 0;  // stream records (patch_nodes > 0)
   int patch_nodes = 0;
   int no_max = 0, nh_max = 0, ne_max = 0;
+  CluLaunch clu{};  // cluster size and maxima of its cluster patches (ctas 0: none)
   float damp = 0.f;
   unsigned char* block = nullptr;
   bool pinned = false;
@@ -3038,15 +3146,63 @@ int build_pack(fw_ctx* c, int patch_nodes, bool pinned, fw_pack** out) {
     pcnt[pr.body]++;
   }
   for (int b = 1; b < Bs; ++b) poff[b] = poff[b - 1] + pcnt[b - 1];
+  // cluster patches, beside the stream records below
+  CluLaunch clu{};
+  std::vector<CluPatch> cpatch;
+  std::vector<unsigned char> cblob;
+  auto cut = [&] {
+    if (!patch_nodes || Bs > kCluMaxBodies || pairs.size() > (size_t)kCluMaxPairs) return;
+    bool per_tri = Bs > 1;
+    int64_t at = 0;
+    for (int b = 0; b < Bs; ++b) {  // bodies one after the other
+      if (c->h_noff[b] != at) return;
+      at += c->h_ncnt[b];
+    }
+    for (int64_t e = 1; e < Es && !per_tri; ++e)
+      per_tri = c->h_E[e] != c->h_E[0] || c->h_nu[e] != c->h_nu[0] || c->h_type[e] != c->h_type[0] ||
+                c->h_sy[e] != c->h_sy[0] || c->h_H[e] != c->h_H[0];
+    const CluScene sc{0, 0, 0, 0, 0, 0, Bs, 0, (int)pairs.size()};
+    std::vector<int> part(Ns, 0);
+    int ctas = 1;
+    while (ctas < kCluMaxCtas && (Ns + ctas - 1) / ctas > kCluServedNodes) ctas *= 2;
+    for (; ctas <= kCluMaxCtas && ctas <= Ns; ctas *= 2) {
+      if (Ns > ctas * (int64_t)kCluMaxThreads && Ns * 32 + Es * 56 > ctas * (int64_t)kCluSharedBytes) continue;
+      cpatch.clear();
+      cblob.clear();
+      if (!make_cluster_patches(c, sc, (int)Ns, off, slot, x0, word, ctas, part, 1, cpatch, cblob)) continue;
+      CluLaunch r{};
+      r.ctas = ctas;
+      for (const CluPatch& q : cpatch) clu_widen(r, q);
+      r.nb = Bs;
+      r.np = (int)pairs.size();
+      r.per_tri = per_tri;
+      r.one = 0;  // the larger of the two carve-ups
+      clu_threads(r, true);
+      if (clu_smem(r) > kCluSharedBytes) continue;
+      clu = r;
+      return;
+    }
+    cpatch.clear();
+    cblob.clear();
+  };
+  std::thread cutter(cut);
+  struct Join {
+    std::thread& t;
+    ~Join() { t.join(); }
+  };
   // stream records
   PatchSet ps;
   if (patch_nodes) {
+    Join wait{cutter};
     std::string why;
     std::vector<int32_t> bscene(Bs, 0);
     if (make_patches((int)Ns, (int)Es, conn.data(), off, slot, x0, c->h_noff, c->h_ncnt, bscene, patch_nodes, ps, why))
       return fail(c, FW_ERR_ARG, "%s", why.c_str());
+  } else {
+    cutter.join();
   }
   fw_pack* pk = new fw_pack();
+  pk->clu = clu;
   pk->Ns = Ns; pk->Es = Es; pk->Bs = Bs; pk->Np = (int64_t)pairs.size();
   pk->Nh = (int64_t)c->h_heights.size(); pk->No = (int64_t)c->h_occ.size();
   pk->damp = c->h_damp.empty() ? 0.f : c->h_damp[0];
@@ -3066,7 +3222,8 @@ int build_pack(fw_ctx* c, int patch_nodes, bool pinned, fw_pack** out) {
       {ps.rn.data(), sizeof(int32_t) * ps.rn.size()}, {ps.rh.data(), sizeof(int32_t) * ps.rh.size()},
       {ps.re.data(), sizeof(int32_t) * ps.re.size()}, {ps.rc.data(), sizeof(uint2) * ps.rc.size()},
       {ps.rcp.data(), sizeof(uint16_t) * ps.rcp.size()}, {ps.rcs.data(), sizeof(uint16_t) * ps.rcs.size()},
-      {ps.patches.data(), sizeof(StreamPatch) * ps.patches.size()}};
+      {ps.patches.data(), sizeof(StreamPatch) * ps.patches.size()},
+      {cpatch.data(), sizeof(CluPatch) * cpatch.size()}, {cblob.data(), cblob.size()}};
   size_t total = 0;
   for (int k = 0; k < fw_pack::NPARTS; ++k) {
     pk->off[k] = total;
@@ -3090,7 +3247,8 @@ int build_pack(fw_ctx* c, int patch_nodes, bool pinned, fw_pack** out) {
   int64_t dev = 48 * Ns + 136 * Es + 64 * pk->Np + 4 * pk->Nh + pk->No;
   if (patch_nodes)
     dev += (int64_t)sizeof(StreamPatch) * pk->Ps + 4 * pk->Hs + (4 + 8 + (int64_t)sizeof(StreamElem)) * pk->Ts +
-           2 * pk->CPs + 6 * Es + (4 + (int64_t)sizeof(StreamNode)) * Ns;
+           2 * pk->CPs + 6 * Es + (4 + (int64_t)sizeof(StreamNode)) * Ns + (int64_t)cblob.size() +
+           (int64_t)(sizeof(CluPatch) * cpatch.size());
   pk->dev_bytes = dev;
   // clear the stage for the next scene
   c->h_x.clear(); c->h_v.clear(); c->h_bc.clear(); c->h_bcv.clear();
@@ -4145,6 +4303,7 @@ int fw_set_option(fw_ctx* c, int32_t option, int32_t value) {
       if (value != 0 && value != 1) return fail(c, FW_ERR_ARG, "FW_OPT_CLUSTER must be 0 or 1");
       if (c->finalized && value) return fail(c, FW_ERR_STATE, "FW_OPT_CLUSTER: clusters are laid out by fw_finalize");
       c->clu_opt = value;
+      c->chunks_dirty = true;  // an arena's lists
       return value ? FW_OK : cluster_off(c);
     }
     default:
@@ -4316,6 +4475,14 @@ int fw_arena_init(fw_ctx* c, int64_t max_nodes, int64_t max_elems, int32_t max_b
     c->fl_halo.init(Hcap);
     c->fl_ptri.init(Tcap);
     c->fl_csrp.init(CPcap);
+    if (c->clu_opt) {
+      const int64_t Qcap = N / kCluServedNodes * 2 + 16 * (int64_t)S, Bcap = 24 * N + 32 * E + 256 * Qcap;
+      if ((rc = dalloc(c, &c->d_cpatch, Qcap)) || (rc = dalloc(c, &c->d_cblob, Bcap)) || (rc = dalloc(c, &c->d_cscene, S)) ||
+          (rc = dalloc(c, &c->d_runs, S)) || (rc = clu_prepare(c, &c->clu_cap, c->clu_size_ok)))
+        return rc;
+      c->fl_cpatch.init(Qcap);
+      c->fl_cblob.init(Bcap);
+    }
     stream_smem(1, 1, 1, &c->st_smem, &c->st_smem_bulk);
     if ((rc = stream_attrs(c, shared_optin(c)))) return rc;
     c->st_list_n = 0;
@@ -4378,6 +4545,16 @@ int fw_arena_commit_pack(fw_ctx* c, const fw_pack* pk, int32_t* scene_out) {
       return fail(c, FW_ERR_ARG, "arena: a patch of this scene needs %zu B of shared memory", smem);
     }
   }
+  // cluster patches, where the device and the arena have room; else the stream kernels step the scene
+  a.clu = pk->clu;
+  a.ncq = (int64_t)(pk->len[fw_pack::CPATCH] / sizeof(CluPatch));
+  a.ncb = (int64_t)pk->len[fw_pack::CBLOB];
+  if (!c->d_cpatch || !a.clu.ctas || !c->clu_size_ok[a.clu.ctas] || clu_smem(a.clu) > c->clu_cap) a.clu.ctas = 0;
+  if (a.clu.ctas && !c->fl_cpatch.take(a.ncq, &a.cq0)) a.clu.ctas = 0;
+  else if (a.clu.ctas && !c->fl_cblob.take(a.ncb, &a.cb0)) {
+    c->fl_cpatch.give(a.cq0, a.ncq);
+    a.clu.ctas = 0;
+  }
   const int s = c->free_scene_ids.back();
   c->free_scene_ids.pop_back();
   a.live = true;
@@ -4402,6 +4579,10 @@ int fw_arena_commit_pack(fw_ctx* c, const fw_pack* pk, int32_t* scene_out) {
     dst[fw_pack::RN] = B(c->sd.nodes + n0); dst[fw_pack::RH] = B(c->sd.halo + a.hh0); dst[fw_pack::RE] = B(c->sd.eid + a.t0);
     dst[fw_pack::RC] = B(c->sd.conn + a.t0); dst[fw_pack::RCP] = B(c->sd.csrp + a.cp0);
     dst[fw_pack::RCS] = B(c->sd.csrs + 3 * e0); dst[fw_pack::PATCH] = B(c->sd.patch + a.pp0);
+  }
+  if (a.clu.ctas) {
+    dst[fw_pack::CPATCH] = B(c->d_cpatch + a.cq0);
+    dst[fw_pack::CBLOB] = B(c->d_cblob + a.cb0);
   }
   if (pk->bytes <= c->stage_cap) {
     FW_CUDA(c, cudaMemcpyAsync(c->d_stage, pk->block, pk->bytes, cudaMemcpyHostToDevice, c->stream));
@@ -4507,6 +4688,10 @@ int fw_arena_remove(fw_ctx* c, int32_t s) {
     c->fl_halo.give(a.hh0, a.nhh);
     c->fl_ptri.give(a.t0, a.nt);
     c->fl_csrp.give(a.cp0, a.ncp);
+  }
+  if (a.clu.ctas) {
+    c->fl_cpatch.give(a.cq0, a.ncq);
+    c->fl_cblob.give(a.cb0, a.ncb);
   }
   a = fw_ctx::ArenaScene{};
   c->energy_dirty = true;
@@ -4882,12 +5067,12 @@ int fw_step_runs(fw_ctx* c, int32_t n_runs, const int32_t* counts, const float* 
   if (c->path != FW_PATH_STREAM || c->clu.empty() || !c->rest_scenes.empty())
     return fail(c, FW_ERR_STATE, "fw_step_runs: not every scene of the world is stepped on chip (FW_OPT_CLUSTER)");
   std::vector<CluRun> runs(c->S, CluRun{});
-  for (int s = 0; s < c->S; ++s)
+  for (int j = 0; j < c->S; ++j)
     for (int k = 0; k < n_runs; ++k) {
-      const int n = counts[(size_t)s * n_runs + k];
+      const int s = c->clu_order[j], n = counts[(size_t)s * n_runs + k];
       if (n < 0) return fail(c, FW_ERR_ARG, "fw_step_runs: scene %d: count < 0", s);
-      runs[s].n[k] = n;
-      runs[s].dt[k] = dts[(size_t)s * n_runs + k];
+      runs[j].n[k] = n;
+      runs[j].dt[k] = dts[(size_t)s * n_runs + k];
     }
   int rc;
   if (!c->d_runs && (rc = dalloc(c, &c->d_runs, c->S))) return rc;
