@@ -151,7 +151,7 @@ struct CluLaunch {
   int withhold_cta;              // test hook: this CTA sends nothing after its first substep (-1: none)
   float2* rec_x;                 // adjoint recompute (one scene): state at the start of each substep
   float2* rec_v;
-  int* rec_gates;
+  int* rec_gates;                // 1 where a pair gave a force (a pair that gave none has no adjoint either)
   int rec_stride;
   const CluRun* runs;            // per scene of the launch (null: nsteps substeps of the scene's dt)
   // grid form
@@ -669,12 +669,6 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
               for (long long it = 0; !ll_has(clu_peek_box<GRID>(r, s, c, k % kCluBoxRing, 0, 0), r.ep0 + (uint32_t)k + 1u) &&
                                      clu_again(it, r.wait_limit, r.err, &s_abort);) {
               }
-          if (r.rec_gates && rank == 0)
-            for (int p = 0; p < sc.np; ++p) {
-              const Pair& pr = s.pairs()[p];
-              const bool on = k == 0 ? s.gate()[p] != 0 : clu_gate(pr, clu_box<GRID>(r, s, pr.body - sc.body0, k, &s_abort), g);
-              if (lane == 0) r.rec_gates[(size_t)k * r.rec_stride + p] = on ? 1 : 0;
-            }
         }
         // the others' contact forces (a single control warp does both)
         const int first = r.ctl > 1 ? (ct & ~31) - 32 : 0, step = r.ctl > 1 ? CT - 32 : 32;
@@ -695,6 +689,7 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
             if (hit && on) {
               f.x += cf.x;
               f.y += cf.y;
+              if (r.rec_gates) r.rec_gates[(size_t)k * r.rec_stride + p] = 1;  // zero before the launch
             }
           }
           if (valid) s.cf()[i] = f;
@@ -843,6 +838,217 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
     if (!ok) __nanosleep(20000);  // what was sent to a CTA that gave up has landed by then
   }
 }
+
+// ------------------------------------------------------------------ adjoint
+// Reverse pass of one recorded segment on the grid form's patches, a thread per
+// triangle and per node: the adjoint state of a node (FP64) and the static data
+// and dL/dE of a triangle stay in registers, the force adjoints that neighbours
+// read are pushed into their halo slots (four tagged words each), and the
+// positions of the next substep are fetched while this one's triangles are
+// evaluated.  The arithmetic and its order are those of k_adj_prep /
+// k_adj_elements / k_adj_nodes.  Bound, like the forward step, by the latency of
+// one substep's chain.
+struct CluAdj {
+  CluLaunch r;  // patches, err, wait limit, tags
+  int x, fb, f, push, pairs;  // byte offsets in shared memory: positions (owned, halo), force adjoints, corner slots
+  ulonglong2* words;          // [2][n_halo][2] force adjoints
+  const float2* rec_x;
+  const float2* rec_v;
+  const int* rec_gates;
+  int gate_stride;
+};
+
+inline size_t clu_adj_layout(CluAdj& q) {
+  size_t o = 0;
+  auto take = [&](int& at, size_t bytes) {
+    at = (int)o;
+    o += (bytes + 15) & ~(size_t)15;
+  };
+  const CluLaunch& r = q.r;
+  take(q.x, sizeof(float2) * (size_t)(r.no + r.nh));
+  take(q.fb, sizeof(double2) * (size_t)r.no);
+  take(q.f, sizeof(float2) * (size_t)r.fs * r.no);
+  take(q.push, sizeof(uint32_t) * (size_t)r.npush);
+  take(q.pairs, sizeof(Pair) * (size_t)r.np);
+  return o;
+}
+
+template <int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+k_cluster_adj(const __grid_constant__ Dev d, const __grid_constant__ CluAdj q, const __grid_constant__ Adj a, int nsteps,
+              float dt, float damp) {
+  __shared__ int s_abort;
+  const CluLaunch& r = q.r;
+  const int t = threadIdx.x, T = blockDim.x, N = d.N;
+  const CluScene sc = r.scene[0];
+  const CluPatch& P = r.patch[sc.patch0 + blockIdx.x];
+  const int no = P.no, nh = P.nh, ne = P.ne, nbnd = P.nbnd;
+  float2* xs = reinterpret_cast<float2*>(clu_mem + q.x);
+  double2* fbs = reinterpret_cast<double2*>(clu_mem + q.fb);
+  float2* fs = reinterpret_cast<float2*>(clu_mem + q.f);
+  uint32_t* push = reinterpret_cast<uint32_t*>(clu_mem + q.push);
+  Pair* pairs = reinterpret_cast<Pair*>(clu_mem + q.pairs);
+  // ---- load
+  if (t == 0) s_abort = 0;
+  const bool tri = t < ne, node = t < no, halo = t < nh;
+  CluTri m{};
+  double Eb = 0.0;
+  float young = 1.f;
+  int eg = 0;
+  if (tri) {
+    eg = sc.e0 + reinterpret_cast<const int32_t*>(r.blob + P.eid)[t];
+    const ElemMat em = d.emat[eg];
+    m.ji = d.jinv[eg];
+    m.rec = clu_rec(r, reinterpret_cast<const uint2*>(r.blob + P.tri)[t], reinterpret_cast<const uint32_t*>(r.blob + P.pos)[t],
+                    em.area);
+    m.lam = em.lam;
+    m.mu = em.mu;
+    m.word = em.word;
+    young = a.young[eg];
+    if (m.rec.y & 0x8000u) Eb = a.Eb[eg];
+  }
+  const bool cut = P.n_int <= (t | 31);
+  double2 xb = make_double2(0.0, 0.0), vb = xb, fb = xb;
+  double step = 0.0, keep = 0.0;
+  uint32_t w = 0;
+  int gn = 0, gh = 0;
+  const double h = (double)dt;
+  if (node) {
+    gn = sc.n0 + reinterpret_cast<const int32_t*>(r.blob + P.gid)[t];
+    w = reinterpret_cast<const uint32_t*>(r.blob + P.info)[t];
+    xb = a.xb[gn];
+    vb = a.vb[gn];
+    step = h / (double)d.mass[gn];
+    keep = 1.0 - step * (double)damp;
+  }
+  if (halo) gh = sc.n0 + reinterpret_cast<const int32_t*>(r.blob + P.hid)[t];
+  for (int i = t; i < P.npush; i += T) {
+    const uint32_t to = reinterpret_cast<const uint32_t*>(r.blob + P.push)[i];
+    push[i] = (uint32_t)r.patch[sc.patch0 + (to >> 24)].halo0 + (to & 0xFFFFFFu);
+  }
+  for (int i = t; i < r.fs * r.no; i += T) fs[i] = make_float2(0.f, 0.f);
+  for (int i = t; i < sc.np; i += T) pairs[i] = d.pairs[sc.pair0 + i];
+  const int bc = (int)(w & fw::NODE_BC_MASK);
+  const bool vfixed = (bc & (fw::BC_U | fw::BC_V)) != 0, fdead = vfixed || (bc & fw::BC_A) != 0;
+  int p_lo = 0, p_hi = 0;  // the pairs of a boundary node's body
+  if (t < nbnd) {
+    const int b = sc.body0 + ((int)(w >> kCluBodyShift) & 15);
+    p_lo = d.body_pair_off[b] - sc.pair0;
+    p_hi = p_lo + d.body_pair_cnt[b];
+  }
+  auto prep = [&] {  // the adjoints of the node force and of the previous velocity
+    const double2 vt = make_double2(vb.x + h * xb.x, vb.y + h * xb.y);
+    fb = fdead ? make_double2(0.0, 0.0) : make_double2(step * vt.x, step * vt.y);
+    vb = vfixed ? make_double2(0.0, 0.0) : make_double2(keep * vt.x, keep * vt.y);
+  };
+  prep();
+  size_t row = (size_t)(nsteps - 1) * N;
+  float2 xn = node ? q.rec_x[row + gn] : make_float2(0.f, 0.f), xh = halo ? q.rec_x[row + gh] : make_float2(0.f, 0.f);
+  __syncthreads();
+  for (int rr = 0; rr < nsteps; ++rr) {
+    const int j = nsteps - 1 - rr;
+    const uint32_t tag = r.ep0 + (uint32_t)rr + 1u;
+    ulonglong2* copy = q.words + (size_t)(rr & 1) * r.n_halo * 2;
+    const float2 xi = xn;
+    if (node) {
+      const uint32_t n_to = (w >> kCluPushCntShift) & 7u;
+      for (uint32_t k = 0; k < n_to; ++k) {
+        ulonglong2* to = copy + 2 * (size_t)push[(w >> kCluPushOffShift) + k];
+        asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(to), "l"(ll_pack(tag, lo32(fb.x))),
+                     "l"(ll_pack(tag, hi32(fb.x)))
+                     : "memory");
+        asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(to + 1), "l"(ll_pack(tag, lo32(fb.y))),
+                     "l"(ll_pack(tag, hi32(fb.y)))
+                     : "memory");
+      }
+      fbs[t] = fb;
+      xs[t] = xn;
+    }
+    if (halo) xs[r.no + t] = xh;
+    __syncthreads();  // positions and force adjoints of substep j
+    float2 vi = make_float2(0.f, 0.f);
+    if (t < nbnd && p_hi > p_lo) vi = q.rec_v[row + gn];
+    if (j > 0) {  // the next substep's positions, on their way meanwhile
+      const size_t up = row - N;
+      if (node) xn = q.rec_x[up + gn];
+      if (halo) xh = q.rec_x[up + gh];
+    }
+    if (tri) {
+      const uint4 c = m.rec;
+      const int i0 = c.y & 0x7FFFu, i1 = c.y >> 16, i2 = c.z & 0xFFFFu;
+      double2 b0, b1, b2;
+      if (cut) {  // poll the halo corners together
+        const bool h0 = i0 >= r.no, h1 = i1 >= r.no, h2 = i2 >= r.no;
+        const ulonglong2* base = copy + 2 * ((ptrdiff_t)P.halo0 - r.no);
+        for (long long it = 0;;) {
+          const unsigned long long done = ll_pack(tag, 0u);
+          ulonglong2 u[6];
+#pragma unroll
+          for (int k = 0; k < 6; ++k) {
+            const bool hk = k < 2 ? h0 : (k < 4 ? h1 : h2);
+            const int ik = k < 2 ? i0 : (k < 4 ? i1 : i2);
+            u[k] = make_ulonglong2(done, done);
+            if (hk)
+              asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                           : "=l"(u[k].x), "=l"(u[k].y)
+                           : "l"(base + 2 * (ptrdiff_t)ik + (k & 1))
+                           : "memory");
+          }
+          bool here = true;
+#pragma unroll
+          for (int k = 0; k < 6; ++k) here = here && ll_has(u[k].x, tag) && ll_has(u[k].y, tag);
+          b0 = make_double2(join64((uint32_t)u[0].x, (uint32_t)u[0].y), join64((uint32_t)u[1].x, (uint32_t)u[1].y));
+          b1 = make_double2(join64((uint32_t)u[2].x, (uint32_t)u[2].y), join64((uint32_t)u[3].x, (uint32_t)u[3].y));
+          b2 = make_double2(join64((uint32_t)u[4].x, (uint32_t)u[4].y), join64((uint32_t)u[5].x, (uint32_t)u[5].y));
+          if (here || !clu_again(it, r.wait_limit, r.err, &s_abort)) break;
+        }
+        if (!h0) b0 = fbs[i0];
+        if (!h1) b1 = fbs[i1];
+        if (!h2) b2 = fbs[i2];
+      } else {
+        b0 = fbs[i0];
+        b1 = fbs[i1];
+        b2 = fbs[i2];
+      }
+      fw::Dual f[6];
+      fw::element_forces_jvp(xs[i0], xs[i1], xs[i2], make_float2((float)b0.x, (float)b0.y), make_float2((float)b1.x, (float)b1.y),
+                             make_float2((float)b2.x, (float)b2.y), m.ji, fw::elem_type(m.word), m.lam, m.mu,
+                             __uint_as_float(c.x), f);
+      const uint32_t o0 = c.z >> 16, o1 = c.w & 0xFFFFu, o2 = c.w >> 16;
+      if (o0 != kCluNoSlot) fs[o0] = make_float2(f[0].d, f[1].d);
+      if (o1 != kCluNoSlot) fs[o1] = make_float2(f[2].d, f[3].d);
+      if (o2 != kCluNoSlot) fs[o2] = make_float2(f[4].d, f[5].d);
+      if (c.y & 0x8000u) {
+        const double dot = b0.x * f[0].v + b0.y * f[1].v + b1.x * f[2].v + b1.y * f[3].v + b2.x * f[4].v + b2.y * f[5].v;
+        Eb += dot / (double)young;
+      }
+    }
+    __syncthreads();  // every corner's share of substep j
+    if (s_abort) break;
+    if (node) {
+      const float4* c = reinterpret_cast<const float4*>(fs + t * r.fs);
+      for (int k = 0; 2 * k < r.fs; ++k) {
+        const float4 cq = c[k];
+        xb.x += cq.x;
+        xb.y += cq.y;
+        xb.x += cq.z;
+        xb.y += cq.w;
+      }
+      for (int p = p_lo; p < p_hi; ++p)
+        if (q.rec_gates[(size_t)j * q.gate_stride + p]) fw::contact_vjp(pairs[p], d.heights, d.occ, xi, vi, dt, fb, xb, vb);
+      if (j > 0) prep();
+    }
+    row -= N;
+  }
+  if (node) {
+    a.xb[gn] = xb;
+    a.vb[gn] = vb;
+  }
+  if (tri && (m.rec.y & 0x8000u)) a.Eb[eg] = Eb;
+}
+
+using CluAdjKernel = void (*)(const Dev, const CluAdj, const Adj, int, float, float);
+inline CluAdjKernel clu_adj_kernel(int threads) { return threads <= 512 ? k_cluster_adj<512> : k_cluster_adj<768>; }
 
 using CluKernel = void (*)(const Dev, const CluLaunch, const float2*, float2*, const float4*, float4*, int);
 inline CluKernel clu_kernel(int threads, int one, int grid) {

@@ -1334,6 +1334,10 @@ struct fw_ctx {
   HostLists lists;
   std::vector<cudaStream_t> side_streams;  // the groups after the first run beside it
   std::vector<cudaEvent_t> side_events;
+  CluAdj clu_adj{};                // the reverse pass on the grid form's patches (k_cluster_adj); words null: not used
+  int clu_adj_threads = 0;
+  uint32_t clu_adj_epoch = 0;
+  size_t clu_adj_smem = 0;
   bool res_adj = false;            // the reverse pass runs resident (k_res_adj)
   size_t res_adj_smem = 0;
   unsigned long long* fll = nullptr;  // [2][N][4] flag-in-data force adjoints of the reverse pass
@@ -4327,6 +4331,47 @@ int fw_get_option(const fw_ctx* c, int32_t option, int32_t* value) {
   }
 }
 
+// A snapshot's arrays, between the context and a slot, in one launch (six copies
+// took 38 us a snapshot for 4225 nodes, most of it their launches).
+struct StateCopy {
+  uint32_t* dst[6];
+  const uint32_t* src[6];
+  uint32_t words[6];
+};
+
+static __global__ void k_copy_state(StateCopy s) {
+  const int part = blockIdx.y;
+  const uint32_t n = s.words[part], n4 = n / 4;
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (uint32_t i = t; i < n4; i += stride) reinterpret_cast<uint4*>(s.dst[part])[i] = reinterpret_cast<const uint4*>(s.src[part])[i];
+  for (uint32_t i = 4 * n4 + t; i < n; i += stride) s.dst[part][i] = s.src[part][i];
+}
+
+static int copy_state(fw_ctx* c, const fw_ctx::Snap& sn, bool save) {
+  // every array is an allocation of its own: 16-byte aligned
+  struct Part {
+    void *live, *kept;
+    size_t bytes;
+  } parts[6] = {{c->d.x, sn.x, sizeof(float2) * (size_t)c->N},
+                {c->d.v, sn.v, sizeof(float2) * (size_t)c->N},
+                {c->d.j2state, sn.j2, sizeof(float4) * (size_t)(c->d.has_j2 ? c->E : 0)},
+                {c->d.scene_counter, sn.counter, sizeof(int32_t) * (size_t)c->S},
+                {c->d.aabb_ring, sn.ring, sizeof(int32_t) * 8 * (size_t)c->B},
+                {c->d.scene_mode_req, sn.mode_req, sizeof(int32_t) * (size_t)c->S}};
+  StateCopy s{};
+  size_t most = 0;
+  for (int k = 0; k < 6; ++k) {
+    s.dst[k] = (uint32_t*)(save ? parts[k].kept : parts[k].live);
+    s.src[k] = (const uint32_t*)(save ? parts[k].live : parts[k].kept);
+    s.words[k] = (uint32_t)(parts[k].bytes / 4);
+    most = std::max(most, parts[k].bytes / 16);
+  }
+  const unsigned gx = (unsigned)std::min<size_t>(std::max<size_t>((most + 255) / 256, 1), 4 * (size_t)c->sms);
+  k_copy_state<<<dim3(gx, 6), 256, 0, c->stream>>>(s);
+  c->launches += 1;
+  return check_kernel(c, "state copy");
+}
+
 int fw_snapshot(fw_ctx* c, int32_t slot) {
   if (c && c->has_rigid) return fail(c, FW_ERR_STATE, "snapshots do not hold the rigid bodies' state");
   if (c && c->has_flex)
@@ -4344,12 +4389,7 @@ int fw_snapshot(fw_ctx* c, int32_t slot) {
         (rc = dalloc(c, &sn.mode_req, c->S)))
       return rc;
   }
-  FW_CUDA(c, cudaMemcpyAsync(sn.x, c->d.x, sizeof(float2) * c->N, cudaMemcpyDeviceToDevice, c->stream));
-  FW_CUDA(c, cudaMemcpyAsync(sn.v, c->d.v, sizeof(float2) * c->N, cudaMemcpyDeviceToDevice, c->stream));
-  FW_CUDA(c, cudaMemcpyAsync(sn.j2, c->d.j2state, sizeof(float4) * E, cudaMemcpyDeviceToDevice, c->stream));
-  FW_CUDA(c, cudaMemcpyAsync(sn.counter, c->d.scene_counter, sizeof(int32_t) * c->S, cudaMemcpyDeviceToDevice, c->stream));
-  FW_CUDA(c, cudaMemcpyAsync(sn.ring, c->d.aabb_ring, sizeof(int32_t) * 8 * c->B, cudaMemcpyDeviceToDevice, c->stream));
-  FW_CUDA(c, cudaMemcpyAsync(sn.mode_req, c->d.scene_mode_req, sizeof(int32_t) * c->S, cudaMemcpyDeviceToDevice, c->stream));
+  if ((rc = copy_state(c, sn, true))) return rc;
   sn.host_counter = c->host_counter;
   sn.valid = true;
   return FW_OK;
@@ -4364,13 +4404,7 @@ int fw_restore(fw_ctx* c, int32_t slot) {
   if (slot < 0 || slot >= (int)c->snaps.size() || !c->snaps[slot].valid)
     return fail(c, FW_ERR_ARG, "fw_restore: slot %d holds no snapshot", slot);
   fw_ctx::Snap& sn = c->snaps[slot];
-  const size_t E = c->d.has_j2 ? c->E : 1;
-  FW_CUDA(c, cudaMemcpyAsync(c->d.x, sn.x, sizeof(float2) * c->N, cudaMemcpyDeviceToDevice, c->stream));
-  FW_CUDA(c, cudaMemcpyAsync(c->d.v, sn.v, sizeof(float2) * c->N, cudaMemcpyDeviceToDevice, c->stream));
-  FW_CUDA(c, cudaMemcpyAsync(c->d.j2state, sn.j2, sizeof(float4) * E, cudaMemcpyDeviceToDevice, c->stream));
-  FW_CUDA(c, cudaMemcpyAsync(c->d.scene_counter, sn.counter, sizeof(int32_t) * c->S, cudaMemcpyDeviceToDevice, c->stream));
-  FW_CUDA(c, cudaMemcpyAsync(c->d.aabb_ring, sn.ring, sizeof(int32_t) * 8 * c->B, cudaMemcpyDeviceToDevice, c->stream));
-  FW_CUDA(c, cudaMemcpyAsync(c->d.scene_mode_req, sn.mode_req, sizeof(int32_t) * c->S, cudaMemcpyDeviceToDevice, c->stream));
+  if (int rc = copy_state(c, sn, false)) return rc;
   c->host_counter = sn.host_counter;
   return FW_OK;
 }
@@ -4833,12 +4867,37 @@ int fw_adj_begin(fw_ctx* c, int32_t max_segment_steps) {
     if ((rc = dalloc(c, &a.sb, 4 * (size_t)c->E))) return rc;
   }
   if (a.sb) FW_CUDA(c, cudaMemsetAsync(a.sb, 0, sizeof(double) * 4 * (size_t)c->E, c->stream));
+  // Reverse pass on the grid form's patches where a CTA has a thread per
+  // triangle and node (64 x 64 quads: 4.4 / 2.4 us a reverse substep against
+  // k_res_adj); larger patches and J2 worlds go on below.
+  if (!c->clu.empty() && c->clu[0].r.grid && !c->d.has_j2 && !c->clu_adj.words) {
+    CluAdj q{};
+    q.r = c->clu[0].r;
+    const int threads = (std::max({q.r.ne, q.r.no, q.r.nh}) + 31) / 32 * 32;
+    int optin = 0, sms = 148, per_sm = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    const size_t need = clu_adj_layout(q);
+    if (threads <= 768 && need + kCluStatic <= (size_t)optin) {
+      CluAdjKernel k = clu_adj_kernel(threads);
+      FW_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)optin - kCluStatic)));
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, need) == cudaSuccess &&
+          per_sm * sms >= q.r.ctas) {
+        if ((rc = dalloc(c, &q.words, 4 * (size_t)q.r.n_halo))) return rc;
+        FW_CUDA(c, cudaMemsetAsync(q.words, 0, sizeof(ulonglong2) * 4 * (size_t)q.r.n_halo, c->stream));
+        c->clu_adj = q;
+        c->clu_adj_threads = threads;
+        c->clu_adj_smem = need;
+      }
+    }
+    cudaGetLastError();
+  }
   // Resident reverse pass when the world runs resident and the adjoint state
   // fits on chip too (J2 worlds reverse on the gather kernels).
-  if (c->path == FW_PATH_RESIDENT && !c->res_adj && !c->d.has_j2) {
+  if (c->path == FW_PATH_RESIDENT && !c->res_adj && !c->d.has_j2 && !c->clu_adj.words) {
     if (!c->clu.empty() && (rc = own_resident(c)) < 0) return rc;
   }
-  if (c->path == FW_PATH_RESIDENT && !c->res_adj && !c->d.has_j2 && c->res.err) {
+  if (c->path == FW_PATH_RESIDENT && !c->res_adj && !c->d.has_j2 && !c->clu_adj.words && c->res.err) {
     int optin = 0, sms = 148;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
@@ -4886,8 +4945,49 @@ int fw_adj_segment(fw_ctx* c, int32_t n_steps, float dt) {
   c->d.uniform_dt = 1;
   c->d.dt_uniform = dt;
   int rc;
+  if (c->clu_adj.words && c->clu.empty()) c->clu_adj.words = nullptr;  // the forms' patches were given up (cluster_off)
+  if (c->clu_adj.words) {
+    // recompute on the grid form, recording positions and gates, then reverse on the same patches
+    if (c->d.P > 0) FW_CUDA(c, cudaMemsetAsync(a.gates, 0, sizeof(int32_t) * (size_t)P * n_steps, c->stream));
+    c->res.rec_x = a.traj;
+    c->res.rec_v = a.trajv;
+    c->res.rec_gates = c->d.P > 0 ? a.gates : nullptr;
+    c->res.rec_stride = P;
+    rc = launch_resident(c, n_steps);
+    c->res.rec_x = nullptr;
+    c->res.rec_v = nullptr;
+    c->res.rec_gates = nullptr;
+    if (rc) return rc;
+    CluAdj q = c->clu_adj;
+    q.r.wait_limit = c->wait_limit > 0 ? c->wait_limit : kCluWaitLimit;
+    if (c->clu_adj_epoch > 0xF0000000u) {
+      FW_CUDA(c, cudaMemsetAsync(q.words, 0, sizeof(ulonglong2) * 4 * (size_t)q.r.n_halo, c->stream));
+      c->clu_adj_epoch = 0;
+    }
+    q.r.ep0 = c->clu_adj_epoch;
+    c->clu_adj_epoch += (uint32_t)n_steps + 1u;
+    q.rec_x = a.traj;
+    q.rec_v = a.trajv;
+    q.rec_gates = a.gates;
+    q.gate_stride = P;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(q.r.ctas);
+    cfg.blockDim = dim3(c->clu_adj_threads);
+    cfg.dynamicSmemBytes = c->clu_adj_smem;
+    cfg.stream = c->stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    FW_CUDA(c, cudaLaunchKernelEx(&cfg, clu_adj_kernel(c->clu_adj_threads), (const Dev)c->d, (const CluAdj)q, (const Adj)a,
+                                  (int)n_steps, dt, c->h_damp.empty() ? 0.0f : c->h_damp[0]));
+    c->launches += 1;
+    return check_kernel(c, "adjoint segment");
+  }
   if (c->res_adj) {
     // recompute on the resident step, recording positions and gates, then the resident reverse
+    if (!c->clu.empty()) FW_CUDA(c, cudaMemsetAsync(a.gates, 0, sizeof(int32_t) * (size_t)P * n_steps, c->stream));
     c->res.rec_x = a.traj;
     c->res.rec_v = a.trajv;
     c->res.rec_gates = a.gates;

@@ -200,3 +200,24 @@ def test_voxel_contact_matches_the_oracle(nx, ny, kind):
         n = lp._packed.N
         assert np.array_equal(lp.femSpringManager.coords.numpy()[:n].astype(np.float64), x)
         assert np.array_equal(lp.femSpringManager.V.numpy()[:n].astype(np.float64), v)
+
+
+@pytest.mark.parametrize("n,ground", [(3, "plane"), (16, "plane"), (41, "bump"), (70, "bump"), (150, "plane")])
+def test_reverse_pass_matches_the_gather_reverse(n, ground):
+    """One patch, several, and meshes whose patches hold more than 512 triangles; contact on."""
+    from flatworld_b200.diff import DiffSim
+
+    def build():
+        g = _plane(0.1 / n) if ground == "plane" else _bump(-1.0, 6.0)  # a quarter of a cell deep, whatever the mesh
+        return _rectangle(n, n, MATS["neohookean"], g, cell=0.4 / n)
+
+    dt = 0.05 * (0.4 / n) / 10.0
+    a, b = DiffSim(build(), dt, 37, 15, damping=0.01), DiffSim(build(), dt, 37, 15, damping=0.01, path="gather")
+    rng = np.random.default_rng(n)
+    young = (5e4 * np.exp(0.1 * rng.standard_normal(a.E))).astype(np.float32)
+    v0 = rng.standard_normal((a.N, 2)).astype(np.float32)
+    seed = rng.standard_normal((a.N, 2)).astype(np.float32)
+    xa, xb = a.forward(young, v0), b.forward(young, v0)
+    assert np.array_equal(xa, xb)
+    for u, v in zip(a.backward(seed, 0.1 * seed), b.backward(seed, 0.1 * seed)):
+        assert np.abs(v).max() > 0 and np.array_equal(u, v)
