@@ -95,7 +95,8 @@ constexpr int kCluPushOffShift = 17;   // 15 bits
 struct CluPatch {
   int no, nh, ne, n_int;  // owned and halo nodes, triangles, interior triangles
   int npush, deg, n_j2, nbnd;  // nbnd: boundary nodes (the first ones)
-  int halo0, pad[3];           // grid form: its first halo slot in CluLaunch::ghalo
+  int halo0, tri0;             // grid form: its first halo slot in CluLaunch::ghalo, its first triangle record in gji and grec
+  int slot_shift, pad;         // corner slots in the blob: corner << slot_shift | node
   int64_t gid, info, hid, push, eid, tri, pos;  // byte offsets into the blob
 };
 
@@ -158,6 +159,13 @@ struct CluLaunch {
   ulonglong2* ghalo;             // [2][n_halo]
   unsigned long long* gbox;      // [kCluBoxRing][ctas][nb][4]
   int n_halo;
+  // ... of patches whose triangle records do not fit beside the nodes: records
+  // in global memory (L2), in patch order, read once a substep
+  float4* gji;
+  uint4* grec;
+  float4* glm;                   // lam, mu, word (per_tri)
+  float4* gj2;
+  int tri_l2;
   uint32_t ep0;                  // tags of this launch count up from here
 };
 
@@ -175,7 +183,7 @@ inline size_t clu_layout(CluLaunch& r) {
   take(r.at.halo, r.grid ? 0 : sizeof(ulonglong2) * 2 * (size_t)r.nh);
   r.fs = (r.deg + 1) / 4 * 4 + 2;  // >= deg, 2 mod 4
   take(r.at.f, sizeof(float2) * (size_t)r.fs * r.no);
-  const size_t nb = r.np ? r.nbnd : 0, ne = r.one ? 0 : r.ne, no = r.one ? 0 : r.no;
+  const size_t nb = r.np ? r.nbnd : 0, ne = r.one || r.tri_l2 ? 0 : r.ne, no = r.one ? 0 : r.no;
   take(r.at.cf, sizeof(float2) * nb);
   take(r.at.bv, sizeof(float2) * nb);
   take(r.at.bb, sizeof(int) * (size_t)r.nbnd);
@@ -285,12 +293,12 @@ __device__ __forceinline__ bool clu_again(long long& it, long long limit, int* e
 }
 
 // Blob encodings, independent of a launch's maxima: a local corner is the owned
-// node, or kCluHalo + the halo node; a corner slot is corner * kCluSlotNodes + node.
+// node, or kCluHalo + the halo node; a corner slot is
+// corner << CluPatch::slot_shift | node (11 bits of node leave 31 corners, 12 leave 15).
 constexpr uint32_t kCluHalo = 0x4000u;
-constexpr uint32_t kCluSlotNodes = 2048u;
 __device__ __forceinline__ uint32_t clu_index(uint32_t c, int no) { return c & kCluHalo ? (c & 0x3FFFu) + no : c; }
-__device__ __forceinline__ uint32_t clu_slot(uint32_t p, int fs) {
-  return p == kCluNoSlot ? p : (p % kCluSlotNodes) * fs + p / kCluSlotNodes;
+__device__ __forceinline__ uint32_t clu_slot(uint32_t p, int fs, int shift) {
+  return p == kCluNoSlot ? p : (p & ((1u << shift) - 1u)) * fs + (p >> shift);
 }
 
 // A triangle's static data (and J2 state).
@@ -302,11 +310,11 @@ struct CluTri {
   float4 j2;
 };
 
-__device__ __forceinline__ uint4 clu_rec(const CluLaunch& r, uint2 c, uint32_t p, float area) {
+__device__ __forceinline__ uint4 clu_rec(const CluLaunch& r, uint2 c, uint32_t p, float area, int shift) {
   const uint32_t i0 = clu_index(c.x & 0x7FFFu, r.no) | (c.x & 0x8000u), i1 = clu_index(c.x >> 16, r.no);
   return make_uint4(__float_as_uint(area), i0 | (i1 << 16),
-                    clu_index(c.y & 0xFFFFu, r.no) | (clu_slot(c.y >> 16, r.fs) << 16),
-                    clu_slot(p & 0xFFFFu, r.fs) | (clu_slot(p >> 16, r.fs) << 16));
+                    clu_index(c.y & 0xFFFFu, r.no) | (clu_slot(c.y >> 16, r.fs, shift) << 16),
+                    clu_slot(p & 0xFFFFu, r.fs, shift) | (clu_slot(p >> 16, r.fs, shift) << 16));
 }
 
 // Corner forces of one triangle in substep k (the halo's tag); returns its
@@ -455,7 +463,7 @@ __device__ __forceinline__ bool clu_gate(const Pair& pr, int4 bb, int g) {
 // Steps every scene of the launch through nsteps substeps: the j-th group of
 // r.ctas CTAs holds scene r.scene[j].  Positions and J2 state are read from x_in / j2_in and
 // written to x_out / j2_out (the same buffers, or a stream world's pair).
-template <int MAXT, bool ONE, bool GRID>
+template <int MAXT, bool ONE, bool GRID, bool L2TRI = false>
 __global__ void __launch_bounds__(MAXT, 1)
 k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, const float2* x_in, float2* x_out,
           const float4* j2_in, float4* j2_out, int n_all) {
@@ -468,7 +476,7 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
   const CluScene sc = r.scene[GRID ? 0 : blockIdx.x / C];
   const CluPatch& Pg = r.patch[sc.patch0 + rank];
   const int S = sc.scene, no = Pg.no, ne = Pg.ne, nbnd = Pg.nbnd, first_cut = Pg.n_int,
-            halo0 = Pg.halo0;
+            halo0 = Pg.halo0, tri0 = Pg.tri0;
   const unsigned char* blob = r.blob + sc.blob0;
   const int32_t* gid = reinterpret_cast<const int32_t*>(blob + Pg.gid);
   const int32_t* eid = reinterpret_cast<const int32_t*>(blob + Pg.eid);
@@ -516,7 +524,7 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
       const int e = sc.e0 + eid[t];
       const ElemMat m = d.emat[e];
       tr.ji = d.jinv[e];
-      tr.rec = clu_rec(r, tri[t], pos[t], m.area);
+      tr.rec = clu_rec(r, tri[t], pos[t], m.area, Pg.slot_shift);
       tr.lam = m.lam;
       tr.mu = m.mu;
       tr.word = m.word;
@@ -552,9 +560,18 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
       for (int u = 0; u < U; ++u)
         if (e[u] >= 0) {
           const int q = q0 + u * W;
+          const uint4 rec = clu_rec(r, c[u], ps[u], m[u].area, Pg.slot_shift);
+          const float4 lm = make_float4(m[u].lam, m[u].mu, __int_as_float(m[u].word), 0.f);
+          if (L2TRI) {
+            r.gji[tri0 + q] = ji[u];
+            r.grec[tri0 + q] = rec;
+            if (r.per_tri) r.glm[tri0 + q] = lm;
+            if (r.has_j2) r.gj2[tri0 + q] = j2[u];
+            continue;
+          }
           s.jinv()[q] = ji[u];
-          s.rec()[q] = clu_rec(r, c[u], ps[u], m[u].area);
-          if (r.per_tri) s.lm()[q] = make_float4(m[u].lam, m[u].mu, __int_as_float(m[u].word), 0.f);
+          s.rec()[q] = rec;
+          if (r.per_tri) s.lm()[q] = lm;
           if (r.has_j2) {
             s.j2()[q] = j2[u];
             if (r.per_tri) s.j2p()[q] = d.j2par[e[u]];
@@ -709,6 +726,39 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
       if (ONE) {
         const bool cut = first_cut <= (t | 31);  // the warp holds cut triangles
         if (t < ne) cfl = fminf(cfl, clu_element<GRID>(p2, r, s, tr, cut, halo0, k, r.ep0 + (uint32_t)k + 1u, &s_abort, bcfl));
+      } else if (L2TRI) {
+        // each record is fetched from L2 while the one before it is evaluated
+        float4 nx_ji{};
+        uint4 nx_rec{};
+        if (t < ne) {
+          nx_ji = __ldcg(&r.gji[tri0 + t]);
+          nx_rec = __ldcg(&r.grec[tri0 + t]);
+        }
+        for (int q = t; q < ne; q += T) {
+          tr.ji = nx_ji;
+          tr.rec = nx_rec;
+          if (q + T < ne) {
+            nx_ji = __ldcg(&r.gji[tri0 + q + T]);
+            nx_rec = __ldcg(&r.grec[tri0 + q + T]);
+          }
+          if (r.per_tri) {
+            const float4 l = __ldcg(&r.glm[tri0 + q]);
+            tr.lam = l.x;
+            tr.mu = l.y;
+            tr.word = __float_as_int(l.z);
+          }
+          const bool mises = fw::elem_type(tr.word) == fw::MAT_MISES;
+          if (mises) {
+            tr.j2 = __ldcg(&r.gj2[tri0 + q]);
+            if (r.per_tri) {
+              const float2 jp = d.j2par[sc.e0 + eid[q]];
+              tr.sy = jp.x;
+              tr.H = jp.y;
+            }
+          }
+          cfl = fminf(cfl, clu_element<GRID>(p2, r, s, tr, first_cut <= (q | 31), halo0, k, r.ep0 + (uint32_t)k + 1u, &s_abort, bcfl));
+          if (mises) __stcg(&r.gj2[tri0 + q], tr.j2);
+        }
       } else {
         for (int q = t; q < ne; q += T) {
           const bool cut = first_cut <= (q | 31);
@@ -829,8 +879,8 @@ k_cluster(const __grid_constant__ Dev d, const __grid_constant__ CluLaunch r, co
       for (int q = t; q < ne; q += T)
         if (tri[q].x & 0x8000u) {
           const int e = sc.e0 + eid[q];
-          const int word = ONE ? tr.word : (r.per_tri ? __float_as_int(s.lm()[q].z) : tr.word);
-          if (fw::elem_type(word) == fw::MAT_MISES) j2_out[e] = ONE ? tr.j2 : s.j2()[q];
+          const int word = d.emat[e].word;
+          if (fw::elem_type(word) == fw::MAT_MISES) j2_out[e] = ONE ? tr.j2 : (L2TRI ? __ldcg(&r.gj2[tri0 + q]) : s.j2()[q]);
         }
   }
   if (!GRID && C > 1) {
@@ -900,7 +950,7 @@ k_cluster_adj(const __grid_constant__ Dev d, const __grid_constant__ CluAdj q, c
     const ElemMat em = d.emat[eg];
     m.ji = d.jinv[eg];
     m.rec = clu_rec(r, reinterpret_cast<const uint2*>(r.blob + P.tri)[t], reinterpret_cast<const uint32_t*>(r.blob + P.pos)[t],
-                    em.area);
+                    em.area, P.slot_shift);
     m.lam = em.lam;
     m.mu = em.mu;
     m.word = em.word;
@@ -1051,8 +1101,9 @@ using CluAdjKernel = void (*)(const Dev, const CluAdj, const Adj, int, float, fl
 inline CluAdjKernel clu_adj_kernel(int threads) { return threads <= 512 ? k_cluster_adj<512> : k_cluster_adj<768>; }
 
 using CluKernel = void (*)(const Dev, const CluLaunch, const float2*, float2*, const float4*, float4*, int);
-inline CluKernel clu_kernel(int threads, int one, int grid) {
+inline CluKernel clu_kernel(int threads, int one, int grid, int tri_l2 = 0) {
   if (grid) {
+    if (tri_l2) return k_cluster<1024, false, true, true>;
     if (one) return threads <= 512 ? k_cluster<512, true, true> : k_cluster<1024, true, true>;
     return threads <= 640 ? k_cluster<640, false, true> : k_cluster<1024, false, true>;
   }

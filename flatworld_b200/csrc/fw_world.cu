@@ -1989,7 +1989,8 @@ bool make_cluster_patches(const fw_ctx* c, const CluScene& sc, int nn, const std
     q.ne = (int)tri.size();
     q.n_int = pt.n_int;
     q.nbnd = (int)(first - ow.begin());
-    if (q.no >= (int)kCluSlotNodes || q.nh >= (int)kCluHalo || q.no + q.nh >= 0x7FFF) {
+    q.slot_shift = q.no > 2048 ? 12 : 11;
+    if (q.no > 4096 || q.nh >= (int)kCluHalo || q.no + q.nh >= 0x7FFF) {
       fits = false;
       return;
     }
@@ -2017,7 +2018,7 @@ bool make_cluster_patches(const fw_ctx* c, const CluScene& sc, int nn, const std
       for (int k = 0; k < dn; ++k) push.push_back(dest[d0 + k]);
       q.deg = std::max(q.deg, off[n + 1] - off[n]);
     }
-    if (q.deg > 30 || (int64_t)(q.deg + 4) * q.no >= (int64_t)kCluNoSlot) {
+    if (q.deg > (q.slot_shift == 11 ? 30 : 14) || (int64_t)(q.deg + 4) * q.no >= (int64_t)kCluNoSlot) {
       fits = false;
       return;
     }
@@ -2034,7 +2035,7 @@ bool make_cluster_patches(const fw_ctx* c, const CluScene& sc, int nn, const std
         if (part[cn[m]] != p) continue;
         const int32_t *b = slot.data() + off[cn[m]], *en = slot.data() + off[cn[m] + 1];
         const int32_t* it = std::lower_bound(b, en, 3 * e + m);  // a node's corners ascend
-        sl[m] = (uint32_t)(it - b) * kCluSlotNodes + at[m];
+        sl[m] = (uint32_t)(it - b) << q.slot_shift | at[m];
       }
       tr[k] = make_uint2((at[0] | (part[cn[0]] == p ? 0x8000u : 0u)) | (at[1] << 16), at[2] | (sl[0] << 16));
       pos[k] = sl[1] | (sl[2] << 16);
@@ -2099,7 +2100,7 @@ bool clu_fits(const CluLaunch& r, int threads, size_t smem) {
     int per_sm = 0, sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, clu_kernel(threads, r.one, 1), threads, smem);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, clu_kernel(threads, r.one, 1, r.tri_l2), threads, smem);
     cudaGetLastError();
     return e == cudaSuccess && per_sm * sms >= r.ctas;
   }
@@ -2145,6 +2146,8 @@ int clu_prepare(fw_ctx* c, size_t* cap, bool* size_ok) {
     for (int one = 0; one < 2; ++one)
       for (int threads : {512, 1024}) {
         CluKernel k = clu_kernel(threads, one, grid);
+        if (grid && !one && threads == 1024)
+          FW_CUDA(c, cudaFuncSetAttribute(clu_kernel(threads, 0, 1, 1), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*cap));
         FW_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*cap));
         if (!grid) FW_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
       }
@@ -2233,7 +2236,7 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
   struct Cut {
     int ctas = 0;
     size_t smem = 0;
-    int kind = 0;
+    int kind = 0, tri_l2 = 0;
     std::vector<CluPatch> patches;
     std::vector<unsigned char> blob;
   };
@@ -2246,7 +2249,8 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
     for (; ctas <= most && ctas <= nn[s]; ctas *= 2) {
       // more nodes than threads and not enough room for positions, node state,
       // corner forces and triangle records: not cut at all
-      if (nn[s] > ctas * kCluMaxThreads && (int64_t)nn[s] * 32 + (int64_t)n_tri[s] * 56 > (int64_t)ctas * (int64_t)cap) continue;
+      const int64_t room = (int64_t)ctas * (int64_t)cap, nodes = (int64_t)nn[s] * 32 + (int64_t)n_tri[s] * 24;
+      if (nn[s] > ctas * kCluMaxThreads && (single ? nodes : nodes + (int64_t)n_tri[s] * 32) > room) continue;
       Cut& k = cuts[s];
       k.patches.clear();
       k.blob.clear();
@@ -2262,6 +2266,15 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
       r.per_tri = scene_tri[s];
       const int threads = clu_threads(r, shared);
       k.smem = clu_smem(r);
+      // A mesh whose records do not fit beside its nodes leaves them in L2, read
+      // once a substep: us per substep against the gather kernels, 537600
+      // triangles 8.0 / 14.6, 655360 9.2 / 17.4, 798000 11.2 / 20.2 (409600,
+      // the records still on chip: 5.75 / 12.7).
+      if (single && k.smem > cap) {
+        r.tri_l2 = 1;
+        k.smem = clu_smem(r);
+      }
+      k.tri_l2 = r.tri_l2;
       if (k.smem > cap || !(single ? clu_fits(r, threads, k.smem) : size_ok[ctas])) continue;
       k.ctas = ctas;
       k.kind = scene_tri[s] * 2 + (r.has_j2 ? 1 : 0);
@@ -2284,9 +2297,12 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
   if (single && made.size() != (size_t)S) return FW_OK;
   int rc;
   int n_halo = 0;
+  int n_rec = 0;
   for (CluPatch& q : patches) {
     q.halo0 = n_halo;
     n_halo += q.nh;
+    q.tri0 = n_rec;
+    n_rec += q.ne;
   }
   CluPatch* dp = nullptr;
   unsigned char* db = nullptr;
@@ -2316,6 +2332,7 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
       fw_ctx::CluGroup g;
       g.r.ctas = m.ctas;
       g.r.grid = m.grid;
+      g.r.tri_l2 = single ? cuts[m.s].tri_l2 : 0;
       c->clu.push_back(g);
       lists.emplace_back();
       group_tri = m.tri;
@@ -2336,6 +2353,11 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
     g.r.err = c->d_flags + fw_ctx::kFlagCluster;
     g.r.withhold_cta = -1;
     g.r.wait_limit = kCluWaitLimit;
+    if (g.r.tri_l2) {
+      if ((rc = dalloc(c, &g.r.gji, n_rec)) || (rc = dalloc(c, &g.r.grec, n_rec)) || (rc = dalloc(c, &g.r.glm, n_rec)) ||
+          (rc = dalloc(c, &g.r.gj2, g.r.has_j2 ? n_rec : 1)))
+        return rc;
+    }
     if (g.r.grid) {
       g.r.n_halo = n_halo;
       const size_t nbox = 4 * (size_t)kCluBoxRing * g.r.ctas * g.r.nb;
@@ -2476,7 +2498,7 @@ int launch_cluster(fw_ctx* c, int n, const float2* x_in, float2* x_out, const fl
     cfg.stream = st;
     cfg.attrs = at;
     cfg.numAttrs = r.ctas > 1 ? 1 : 0;
-    FW_CUDA(c, cudaLaunchKernelEx(&cfg, clu_kernel(g.threads, r.one, r.grid), (const Dev)c->d, (const CluLaunch)r, x_in, x_out, j2_in, j2_out, n));
+    FW_CUDA(c, cudaLaunchKernelEx(&cfg, clu_kernel(g.threads, r.one, r.grid, r.tri_l2), (const Dev)c->d, (const CluLaunch)r, x_in, x_out, j2_in, j2_out, n));
     c->launches += 1;
     if (k > 0) {
       FW_CUDA(c, cudaEventRecord(c->side_events[k], st));

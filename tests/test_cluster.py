@@ -52,6 +52,8 @@ SINGLE = {
     "two patches": lambda: _rectangle(15, 8, MATS["neohookean"], _plane()),
     "a thread per triangle, J2": lambda: _rectangle(60, 31, MATS["mises"], _plane()),
     "several triangles per thread": lambda: _rectangle(260, 251, MATS["neohookean"], _plane(), cell=0.004),
+    "records in L2": lambda: _rectangle(640, 500, MATS["neohookean"], _plane(-0.0005), cell=0.002),
+    "records in L2, J2": lambda: _rectangle(520, 440, MATS["mises"], _plane(-0.0005), cell=0.002),
     "nodes of many corners": _disk,
     "no pairs": lambda: _rectangle(40, 17, MATS["mises"], None),
     "seven bodies": lambda: scenes.multi_block_scene(fw, 7),
