@@ -32,11 +32,12 @@ constexpr int kFlexMaxCells = 100000;                // SpatialHashManager max_c
 constexpr int kFlexListCap = 16;                     // contributions one node takes per substep
 constexpr double kFlexRebuildInterval = 1.0 / 500.0; // FemSpringManager._sh_rebuild_interval
 constexpr int kFlexScanThreads = 1024;
+constexpr int kFlexMaxFem = 14560;                   // 16 bytes of shared memory per FEM body: more never fit
 
 struct FlexGrid {
   int tc, cnx, cny, npairs;
   int simple;    // every element sits in every cell of its box (no cell cap, no pair truncation)
-  int n_active;  // work items of active (pair, side) segments this substep
+  int n_units;   // groups of work items that run this substep (FlexDev::unit)
   int pad2[2];
   float olx, oly, gsx, gsy;
   int estimate;  // ordered-int minimum of the element box diagonals
@@ -51,10 +52,10 @@ struct FlexScene {
   int scene, body0, n_fem;       // the scene and its bodies (FEM-local index = body - body0)
   int dom_off, n_dom, skip_bvh;  // its domains (dom_obj / dom_body / dom_box)
   int pair_off, n_pairs;         // its ContactFlexFlex pairs
-  int seg_base, n_seg;           // its (pair, side) segments; seg_off holds n_seg + 1 entries at seg_base + k
+  int seg_base, n_seg;           // its (pair, side) segments
   int be0, n_be;                 // its boundary edges (registration order)
   int max_pairs, pair_base;      // its (cell, element) pair capacity and slot base
-  int cell_base, pad;            // its cells: k * kFlexMaxCells
+  int cell_base, unit_base;      // its cells: k * kFlexMaxCells; its first work-item group
   int n_tied, n_untied;          // its work items of tied / untied pairs
 };
 
@@ -84,8 +85,6 @@ struct FlexDev {
   const int32_t* dom_obj;   // per domain of the scene: a broad-phase object (considerContact)
   const int32_t* dom_body;  // per domain: global body id, -1 for a ground, -2 - r for rigid r
   const float4* dom_box;    // per domain: a ground's static box
-  int32_t* pair_active;
-  int32_t* stamped;  // at body0 + g: the scene's domain g is in a broad-phase pair this substep
   FlexGrid* g;
   float4* ebox;
   int32_t* ecount;
@@ -96,12 +95,13 @@ struct FlexDev {
   int32_t* cursor;
   int32_t* sorted;
   int2* crange;  // (start, end) of cell (ix, iy) at ix * cny + iy: a column is contiguous
-  int2* ecell;   // per element: its lowest cell (ix, iy), clamped to the grid
+  int4* ecell;   // per element: its lowest and highest cell (ix, iy, ix, iy), clamped to the grid
+  int4* bcell;   // per body: the cell range of its elements
   int4* srec;    // per cell entry (cell order): element, its body, its two nodes
   int2* scell;   // per cell entry: the element's lowest cell
   int n_seg;            // (pair, side) segments of consecutive work items
   const int4* seg;      // per segment: first item, item count, pair (in the scene), target body
-  int32_t* seg_off;     // [n_seg + 1]: exclusive scan of the active segments' item counts
+  int4* unit;           // the work items that run: (first item, count <= kFlexUnit, target body)
   // tied pairs (ExplicitLoop(ties=...)): per pair, and per work item the edge
   // it found at the first substep (-1: none), its weights and normal gap
   const int32_t* pair_tied;
@@ -118,13 +118,13 @@ __device__ __forceinline__ FlexDev flex_view(const FlexDev& f0, int k) {
   f.scene = c.scene; f.body0 = c.body0; f.n_fem = c.n_fem; f.n_dom = c.n_dom; f.skip_bvh = c.skip_bvh;
   f.n_pairs = c.n_pairs; f.n_seg = c.n_seg; f.be0 = c.be0; f.n_be = c.n_be; f.max_pairs = c.max_pairs;
   f.dom_obj += c.dom_off; f.dom_body += c.dom_off; f.dom_box += c.dom_off;
-  f.pair_body += c.pair_off; f.pair_active += c.pair_off; f.pair_tied += c.pair_off;
+  f.pair_body += c.pair_off; f.pair_tied += c.pair_off;
   f.n_tied = c.n_tied; f.n_untied = c.n_untied;
   f.g += k;
   f.cell_count += c.cell_base; f.cell_start += c.cell_base; f.cell_end += c.cell_base;
   f.cursor += c.cell_base; f.crange += c.cell_base;
   f.sorted += c.pair_base; f.srec += c.pair_base; f.scell += c.pair_base;
-  f.seg += c.seg_base; f.seg_off += c.seg_base + k;
+  f.seg += c.seg_base; f.unit += c.unit_base;
   return f;
 }
 
@@ -163,32 +163,46 @@ __device__ __forceinline__ int flex_cell(float delta, float gs, int n) {
   return c;
 }
 
-// Exclusive scan of n ints (one CTA of kFlexScanThreads); returns the total.
-// Each thread scans a contiguous chunk, the chunk sums are scanned in shared
-// memory.
-__device__ int flex_block_scan(const int32_t* in, int32_t* out, int n) {
-  __shared__ int part[kFlexScanThreads];
-  const int t = threadIdx.x;
+// Exclusive scan of one int per thread (one CTA of kFlexScanThreads), by
+// shuffles: three barriers.
+__device__ __forceinline__ int flex_thread_scan(int v, int& total) {
+  __shared__ int part[kFlexScanThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int sum = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xFFFFFFFFu, sum, o);
+    if (lane >= o) sum += u;
+  }
   __syncthreads();  // a previous call's readers of part[] are done
+  if (lane == 31) part[warp] = sum;
+  __syncthreads();
+  if (warp == 0) {
+    int w = part[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xFFFFFFFFu, w, o);
+      if (lane >= o) w += u;
+    }
+    part[lane] = w;
+  }
+  __syncthreads();
+  total = part[kFlexScanThreads / 32 - 1];
+  return sum - v + (warp > 0 ? part[warp - 1] : 0);
+}
+
+// Exclusive scan of n ints, a contiguous chunk per thread; returns the total.
+__device__ int flex_block_scan(const int32_t* in, int32_t* out, int n) {
+  const int t = threadIdx.x;
   const int chunk = (n + kFlexScanThreads - 1) / kFlexScanThreads;
   const int lo = min(n, t * chunk), hi = min(n, lo + chunk);
-  int sum = 0;
+  int sum = 0, total;
   for (int i = lo; i < hi; ++i) sum += in[i];
-  part[t] = sum;
-  __syncthreads();
-  for (int o = 1; o < kFlexScanThreads; o <<= 1) {
-    const int v = t >= o ? part[t - o] : 0;
-    __syncthreads();
-    part[t] += v;
-    __syncthreads();
-  }
-  int run = part[t] - sum;
+  int run = flex_thread_scan(sum, total);
   for (int i = lo; i < hi; ++i) {
     const int v = in[i];
     out[i] = run;
     run += v;
   }
-  return part[kFlexScanThreads - 1];
+  return total;
 }
 
 __device__ __forceinline__ void flex_elem_cells(const FlexGrid& g, float4 eb, int& lx, int& ly, int& ux, int& uy) {
@@ -263,13 +277,23 @@ __device__ void flex_rebuild(const Dev& d, const FlexDev& f) {
   for (int e = e0 + t; e < e1; e += T) {
     int lx, ly, ux, uy, n = 0;
     flex_elem_cells(g, f.ebox[e], lx, ly, ux, uy);
-    f.ecell[e] = make_int2(lx, ly);
+    f.ecell[e] = make_int4(lx, ly, ux, uy);
     for (int ix = lx; ix <= ux; ++ix)
       for (int iy = ly; iy <= uy; ++iy)
         if (ix + iy * g.cnx < g.tc) ++n;
     f.ecount[e] = n;
   }
   __syncthreads();
+  for (int b = f.body0 + (t >> 5); b < f.body0 + f.n_fem; b += T >> 5) {  // the bodies' cell ranges, a warp each
+    int4 m = make_int4(0x7FFFFFFF, 0x7FFFFFFF, -1, -1);
+    for (int e = f.be_off[b] + (t & 31); e < f.be_off[b] + f.be_cnt[b]; e += 32) {
+      const int4 c = f.ecell[e];
+      m = make_int4(min(m.x, c.x), min(m.y, c.y), max(m.z, c.z), max(m.w, c.w));
+    }
+    m = make_int4(__reduce_min_sync(0xFFFFFFFFu, m.x), __reduce_min_sync(0xFFFFFFFFu, m.y),
+                  __reduce_max_sync(0xFFFFFFFFu, m.z), __reduce_max_sync(0xFFFFFFFFu, m.w));
+    if ((t & 31) == 0) f.bcell[b] = m;
+  }
   const int npairs = flex_block_scan(f.ecount + e0, f.ebase + e0, f.n_be);
   if (t == 0) {
     f.g->npairs = npairs;
@@ -330,7 +354,7 @@ __device__ void flex_rebuild(const Dev& d, const FlexDev& f) {
         const int e = f.sorted[i];
         const int2 n = f.be[e];
         f.srec[i] = make_int4(e, f.be_dom[e], n.x, n.y);
-        f.scell[i] = f.ecell[e];
+        f.scell[i] = make_int2(f.ecell[e].x, f.ecell[e].y);
       }
     }
   }
@@ -339,18 +363,64 @@ __device__ void flex_rebuild(const Dev& d, const FlexDev& f) {
 
 __device__ void flex_ties(const Dev& d, const FlexDev& f);
 
-// Per substep, before k_elements, one block: the hash clock and, when it
+// The work items of a segment are taken kFlexUnit at a time, kFlexLanes lanes
+// each: one warp.
+constexpr int kFlexUnit = 4;
+constexpr int kFlexLanes = 32 / kFlexUnit;
+
+// First launch of a substep.  Block k < n_fs: scene k's hash clock and, when it
 // fires, the rebuild (flex_rebuild); pair activation, the broad-phase domain
-// stamps, and the compacted list of work items that run.  force != 0: the
-// construction-time build (explicitloop.py:383-385) -- rebuild, no contact.
+// stamps, and the list of work items that run.  The other blocks: the element
+// step, which needs none of it.  force != 0: the construction-time build
+// (explicitloop.py:383-385) -- rebuild, no contact.
 // Dynamic shared memory: (n_dom + n_fem) boxes -- every domain's, then every
 // FEM body's.
+// Bound by the latency of block k's chain: boxes, clock | stamps | scan, list.
+// 36 disks of 512 triangles, warm, under ncu: 10.7 us, where this block's work
+// alone took 11.4 (a scan of twenty barriers, the boxes loaded after the clock)
+// and the element step another 7.1 in its own launch.
 __global__ void __launch_bounds__(kFlexScanThreads) k_flex_pre(Dev d, FlexDev f0, int force) {
   extern __shared__ float4 sbox[];
   __shared__ int s_rebuild;
-  const FlexDev f = flex_view(f0, blockIdx.x);  // one block per scene with FEM-FEM contact
+  __shared__ uint32_t s_stamped[kFlexMaxFem / 32];  // a bit per domain: in a broad-phase pair this substep
+  if ((int)blockIdx.x >= f0.n_fs) {  // a contiguous, equal share of the triangles: every SM gets one
+    const int nb = gridDim.x - f0.n_fs, per = (d.E + nb - 1) / nb, e0 = (blockIdx.x - f0.n_fs) * per;
+    for (int e = e0 + threadIdx.x; e < min(d.E, e0 + per); e += blockDim.x) {
+      const float dtc = element_step(d, e);
+      if (d.cfl_ord) cfl_reduce(d, e, dtc);
+    }
+    return;
+  }
+  const FlexDev f = flex_view(f0, blockIdx.x);
   const int s = f.scene;
   const bool step = !force && flex_stepping(d, s);
+  const int k = d.scene_counter[s];
+  const int slot = k & 1;
+  float4* body_box = sbox + f.n_dom;
+  // this thread's segments: the first of them is fetched before it is needed
+  const int chunk = (f.n_seg + kFlexScanThreads - 1) / kFlexScanThreads;
+  const int lo = min(f.n_seg, (int)threadIdx.x * chunk), hi = min(f.n_seg, lo + chunk);
+  struct Seg {
+    int4 sg;
+    int2 pb;
+    int tied;
+  };
+  auto fetch = [&](int q) {
+    const int4 sg = f.seg[q];
+    return Seg{sg, f.pair_body[sg.z], f.pair_tied[sg.z]};
+  };
+  Seg first{};
+  if (step && lo < hi) first = fetch(lo);
+  for (int g = threadIdx.x; g < f.n_dom; g += blockDim.x) {
+    const int body = f.dom_body[g];
+    float4 bb = body >= 0 ? ring_box(d, slot, body) : body <= -2 ? rigid_box(d.rig[-2 - body]) : f.dom_box[g];
+    if (!f.dom_obj[g]) bb.x = __int_as_float(0x7FC00000);  // not a broad-phase object: overlaps nothing
+    sbox[g] = bb;
+  }
+  for (int b = threadIdx.x; b < f.n_fem; b += blockDim.x) {
+    body_box[b] = ring_box(d, slot, f.body0 + b);
+    if (b % 32 == 0) s_stamped[b / 32] = 0u;
+  }
   if (threadIdx.x == 0) {
     int rb = force ? 1 : 0;
     // maybe_rebuild_fem_spatial_hash(self.dt), called while untied work items
@@ -366,57 +436,47 @@ __global__ void __launch_bounds__(kFlexScanThreads) k_flex_pre(Dev d, FlexDev f0
     }
     f.g->rebuild = rb;
     if (rb) f.g->estimate = fw::f2ord(1e30f);
-    if (!step) f.g->n_active = 0;
+    if (!step) f.g->n_units = 0;
     s_rebuild = rb;
   }
   __syncthreads();
   if (s_rebuild) flex_rebuild(d, f);
   if (!step) return;
-  const int k = d.scene_counter[s];
-  const int slot = k & 1;
-  float4* body_box = sbox + f.n_dom;
-  for (int g = threadIdx.x; g < f.n_dom; g += blockDim.x)
-    sbox[g] = f.dom_body[g] >= 0    ? ring_box(d, slot, f.dom_body[g])
-              : f.dom_body[g] <= -2 ? rigid_box(d.rig[-2 - f.dom_body[g]])
-                                    : f.dom_box[g];
-  for (int b = threadIdx.x; b < f.n_fem; b += blockDim.x) body_box[b] = ring_box(d, slot, f.body0 + b);
-  __syncthreads();
-  // _activate_or_fill_pairs: every pair when the loop has no BVH, else BVH overlap
-  for (int p = threadIdx.x; p < f.n_pairs; p += blockDim.x) {
-    const int2 pb = f.pair_body[p];
-    f.pair_active[p] = f.skip_bvh ? 1 : (flex_boxes_overlap(body_box[pb.x - f.body0], body_box[pb.y - f.body0], k) ? 1 : 0);
-  }
   // _scan_bvh_pairs_stamp_kernel: domain g (global index) is stamped when it
   // is in some broad-phase pair; the contact kernel reads the stamp at the
   // item's fem-local target index.  One warp per g.
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   for (int gi = warp; gi < f.n_fem; gi += nwarps) {
     bool st = false;
-    if (gi < f.n_dom && f.dom_obj[gi]) {
+    if (gi < f.n_dom) {
       const float4 a = sbox[gi];
       for (int h0 = 0; h0 < f.n_dom && !st; h0 += 32) {
         const int h = h0 + lane;
-        const bool hit = h < f.n_dom && h != gi && f.dom_obj[h] && flex_boxes_overlap(a, sbox[h], k);
+        const bool hit = h < f.n_dom && h != gi && flex_boxes_overlap(a, sbox[h], k);
         st = __any_sync(0xFFFFFFFFu, hit);
       }
     }
-    if (lane == 0) f.stamped[f.body0 + gi] = st ? 1 : 0;
+    if (lane == 0 && st) atomicOr(&s_stamped[gi / 32], 1u << gi % 32);
   }
   __syncthreads();
-  // the work items that run: the (pair, side) segments whose pair is active
-  // and whose target is stamped (or every one when the loop has no BVH),
-  // compacted so the contact kernel visits nothing else
-  for (int q = threadIdx.x; q < f.n_seg; q += blockDim.x) {
-    const int4 sg = f.seg[q];
-    const bool on = !f.pair_tied[sg.z] && f.pair_active[sg.z] && (f.skip_bvh || f.stamped[sg.w]);
-    f.seg_off[q] = on ? sg.y : 0;
+  // the work items that run, in groups of kFlexUnit: the (pair, side) segments
+  // whose pair is active (_activate_or_fill_pairs: the bodies' boxes overlap)
+  // and whose target is stamped -- or every one when the loop has no BVH
+  auto groups = [&](const Seg& a) {
+    const bool on = !a.tied && (f.skip_bvh || (flex_boxes_overlap(body_box[a.pb.x - f.body0], body_box[a.pb.y - f.body0], k) &&
+                                               (s_stamped[(a.sg.w - f.body0) / 32] >> (a.sg.w - f.body0) % 32 & 1u)));
+    return on ? (a.sg.y + kFlexUnit - 1) / kFlexUnit : 0;
+  };
+  int units = 0, total;
+  for (int q = lo; q < hi; ++q) units += groups(q == lo ? first : fetch(q));
+  int at = flex_thread_scan(units, total);
+  for (int q = lo; units > 0 && q < hi; ++q) {
+    const Seg a = q == lo ? first : fetch(q);
+    const int n = groups(a);
+    for (int i = 0; i < n; ++i)
+      f.unit[at++] = make_int4(a.sg.x + i * kFlexUnit, min(kFlexUnit, a.sg.y - i * kFlexUnit), a.sg.w, 0);
   }
-  __syncthreads();
-  const int total = flex_block_scan(f.seg_off, f.seg_off, f.n_seg);
-  if (threadIdx.x == 0) {
-    f.seg_off[f.n_seg] = total;
-    f.g->n_active = total;
-  }
+  if (threadIdx.x == 0) f.g->n_units = total;
   if (f.n_tied > 0) flex_ties(d, f);
 }
 
@@ -455,15 +515,30 @@ __device__ __forceinline__ float flex_detect(float2 p, float2 a, float2 b, float
   return 1e9f;
 }
 
-__device__ __forceinline__ void flex_push(const Dev& d, int* err, int node, int item, float2 force) {
-  const int slot = d.flex_slot[node];
-  const int j = atomicAdd(&d.flex_cnt[slot], 1);
+// True only where flex_detect(p, a, b) cannot give a penetration below 1e-4:
+// the foot of p lies outside the edge, or p further than that on its outer
+// side, both by far more than the rounding of either test.  Without the
+// division and the square root, which all but one or two candidates can do without.
+__device__ __forceinline__ bool flex_clear(float2 p, float2 a, float2 b) {
+  const float ex = b.x - a.x, ey = b.y - a.y, tx = p.x - a.x, ty = p.y - a.y;
+  const float ee = ex * ex + ey * ey;
+  const float ux = tx * ex, uy = ty * ey, along = ux + uy, am = 1e-3f * ee + 1e-5f * (fabsf(ux) + fabsf(uy));
+  const float wx = tx * ey, wy = ty * ex, out = wx - wy - 1e-5f * (fabsf(wx) + fabsf(wy));
+  return along < -am || along > ee + am || (out > 0.0f && out * out > 1.05e-8f * ee);
+}
+
+__device__ __forceinline__ void flex_put(const Dev& d, int* err, int slot, int j, int item, float2 force) {
   if (j < kFlexListCap) {
     d.flex_item[slot * kFlexListCap + j] = item;
     d.flex_force[slot * kFlexListCap + j] = force;
   } else {
     atomicOr(err, 1);
   }
+}
+
+__device__ __forceinline__ void flex_push(const Dev& d, int* err, int node, int item, float2 force) {
+  const int slot = d.flex_slot[node];
+  flex_put(d, err, slot, atomicAdd(&d.flex_cnt[slot], 1), item, force);
 }
 
 // Tied pairs (mixedcontact.py:1680-1690).  At the scene's first substep every
@@ -579,74 +654,142 @@ __device__ void flex_ties(const Dev& d, const FlexDev& f) {
 // where two bodies meet, so few items run; to keep the SMs busy each item
 // gets kFlexLanes lanes.  The query walks cells ix-major then iy, each cell's
 // elements in order, strict < keeping the first minimum.  When every element
-// sits in every cell of its box (no cell cap, no pair truncation: g.simple),
-// an element is new at cell (ix, iy) exactly when that is the first cell of
-// its box inside the query window, so no candidate list is needed: the
-// window's cells are cut into kFlexLanes contiguous runs of the walk, each
-// lane keeps the first minimum of its run, and the group takes the smallest
-// penetration, ties to the lower lane (earlier in the walk) -- the serial
-// result.  Otherwise, or past the reference's 512 unique candidates, the walk
-// keeps the candidate list as written.
-constexpr int kFlexLanes = 8;
-constexpr int kFlexContactThreads = 128;
+// sits in every cell of its box (no cell cap, no pair truncation: g.simple)
+// - an item whose window misses its target's cells altogether has no candidate;
+// - an element is a candidate exactly when its cell box meets the window, and
+//   the walk meets it first at the first cell of its box inside the window.
+// So no candidate list is needed: a lane takes a share of the candidates and
+// keeps the smallest penetration with its place in the walk, and the group takes
+// the smallest, ties to the earlier place -- the serial result.  The candidates
+// are found in one of two ways: through the target's own boundary edges
+// (contiguous; independent loads), or through the window's cells, in contiguous
+// runs of the walk.  Past the reference's 512 unique candidates, and where
+// g.simple does not hold, the walk keeps the candidate list as written.
+constexpr int kFlexContactThreads = 64;
+// Edges of the target per cell of the window up to which the edges are looked
+// through.  A step of two touching disks, edges / cells, us: 32 edges 14.3 /
+// 16.3, 64 15.7 / 19.6, 160 16.4 / 18.5, 320 18.2 / 19.2 and 480 19.7 / 18.9
+// (windows of about 9 to 16 cells); 36 disks of 64 edges, windows of 144 cells:
+// 22.4 / 46.8.
+constexpr int kFlexEdgesPerCell = 16;
 
 struct FlexBest {
   float pen, nx, ny, w0, w1;
   int e, n0, n1;
+  long long place;  // cell of the walk, then registration order
 };
+
+// The walk as written, with its candidate list.
+__device__ __noinline__ FlexBest flex_walk(const Dev& d, const FlexDev& f, const FlexGrid& g, float2 p, float qbuf, int target,
+                                           int lx, int ly, int ux, int uy) {
+  FlexBest b{1e9f, 0.f, 0.f, 0.f, 0.f, -1, 0, 0, 0};
+  int cand[kFlexMaxQuery];
+  int num = 0;
+  for (int ix = lx; ix <= ux; ++ix)
+    for (int iy = ly; iy <= uy; ++iy) {
+      const int cid = ix + iy * g.cnx;
+      if (cid < 0 || cid >= g.tc) continue;
+      for (int q = f.cell_start[cid]; q < f.cell_end[cid]; ++q) {
+        const int e = f.sorted[q];
+        if (e < 0 || f.be_dom[e] != target) continue;
+        bool dup = false;
+        for (int k = 0; k < num; ++k) dup |= cand[k] == e;
+        if (!dup && num < kFlexMaxQuery) cand[num++] = e;
+      }
+    }
+  for (int j = 0; j < num; ++j) {
+    const int e = cand[j];
+    const int2 n = f.be[e];
+    float nx, ny, w0, w1;
+    const float pen = flex_detect(p, d.x[n.x], d.x[n.y], qbuf, nx, ny, w0, w1);
+    if (pen < b.pen && pen < 1e-4f && fabsf(pen) < qbuf) b = FlexBest{pen, nx, ny, w0, w1, e, n.x, n.y, 0};
+  }
+  return b;
+}
 
 __device__ __forceinline__ void flex_item(const Dev& d, const FlexDev& f, const FlexGrid& g, int it, int target,
                                           int sub, unsigned gmask) {
-  const int nid = f.item_node[it];
-  const int be_off = f.be_off[target], be_cnt = f.be_cnt[target];
-  const float2 p = d.x[nid], vp = d.v[nid];
+  const int nid = f.item_node[it], cached = f.item_cache[it];
   const float pen_k = f.item_pen[it], fric = f.item_fric[it];
+  const int be_off = f.be_off[target], be_cnt = f.be_cnt[target];
+  const int4 tc = f.bcell[target];
+  const float2 p = d.x[nid], vp = d.v[nid];
+  const int s0 = d.flex_slot[nid];
   const float qbuf = wmax(wmax(1e-4f, wmax(g.gsx, g.gsy)), 0.016f);
-  float best = 1e9f, bnx = 0.f, bny = 0.f, bw0 = 0.f, bw1 = 0.f;
-  int bn0 = 0, bn1 = 0;
-  bool found = false;
-  const int cached = f.item_cache[it];
-  int cache_out = cached;
+  FlexBest b{1e9f, 0.f, 0.f, 0.f, 0.f, -1, 0, 0, 0x7FFFFFFFFFFFFFFFll};
   if (cached >= be_off && cached < be_off + be_cnt) {
     const int2 n = f.be[cached];
-    const float2 a = d.x[n.x], b = d.x[n.y];
+    const float2 a = d.x[n.x], c = d.x[n.y];
     float lx = 1e30f, ly = 1e30f, ux = -1e30f, uy = -1e30f;
     lx = wmin(lx, a.x); ly = wmin(ly, a.y); ux = wmax(ux, a.x); uy = wmax(uy, a.y);
-    lx = wmin(lx, b.x); ly = wmin(ly, b.y); ux = wmax(ux, b.x); uy = wmax(uy, b.y);
+    lx = wmin(lx, c.x); ly = wmin(ly, c.y); ux = wmax(ux, c.x); uy = wmax(uy, c.y);
     const float dx = ux - lx, dy = uy - ly;
     const float margin = wmax(1e-4f, 1e-2f * sqrtf(dx * dx + dy * dy));
     lx = lx - margin; ly = ly - margin; ux = ux + margin; uy = uy + margin;
     const bool outside = wmin(p.x - lx, p.y - ly) < 0.0f || wmin(ux - p.x, uy - p.y) < 0.0f;
     if (!outside) {
       float nx, ny, w0, w1;
-      const float pen = flex_detect(p, a, b, margin, nx, ny, w0, w1);
-      if (pen < 1e-4f && fabsf(pen) < margin) {
-        best = pen; bnx = nx; bny = ny; bw0 = w0; bw1 = w1; bn0 = n.x; bn1 = n.y; found = true;
-      }
+      const float pen = flex_detect(p, a, c, margin, nx, ny, w0, w1);
+      if (pen < 1e-4f && fabsf(pen) < margin) b = FlexBest{pen, nx, ny, w0, w1, cached, n.x, n.y, 0};
     }
   }
-  if (!found && g.tc > 0) {  // query_point_with_buffer, then every candidate in order
+  if (b.e < 0 && g.tc > 0) {  // query_point_with_buffer, then every candidate in order
     const int lx = flex_cell(p.x - qbuf - g.olx, g.gsx, g.cnx), ly = flex_cell(p.y - qbuf - g.oly, g.gsy, g.cny);
     const int ux = flex_cell(p.x + qbuf - g.olx, g.gsx, g.cnx), uy = flex_cell(p.y + qbuf - g.oly, g.gsy, g.cny);
     bool serial = !g.simple;
-    if (g.simple) {
+    if (g.simple && tc.x <= ux && tc.z >= lx && tc.y <= uy && tc.w >= ly) {
       const int h = uy - ly + 1, ncell = (ux - lx + 1) * h;
-      const int chunk = (ncell + kFlexLanes - 1) / kFlexLanes;
-      const int t1 = min(ncell, (sub + 1) * chunk);
-      FlexBest b{1e9f, 0.f, 0.f, 0.f, 0.f, -1, 0, 0};
       int num = 0;
-      for (int t = min(ncell, sub * chunk); t < t1; ++t) {
-        const int ix = lx + t / h, iy = ly + t % h;
-        const int2 r = f.crange[ix * g.cny + iy];
-        for (int q = r.x; q < r.y; ++q) {
-          const int4 rec = f.srec[q];  // element, domain, nodes
-          if (rec.y != target) continue;
-          const int2 ec = f.scell[q];
-          if (ix != (lx > ec.x ? lx : ec.x) || iy != (ly > ec.y ? ly : ec.y)) continue;  // seen earlier
-          ++num;
-          float nx, ny, w0, w1;
-          const float pen = flex_detect(p, d.x[rec.z], d.x[rec.w], qbuf, nx, ny, w0, w1);
-          if (pen < b.pen && pen < 1e-4f && fabsf(pen) < qbuf) b = FlexBest{pen, nx, ny, w0, w1, rec.x, rec.z, rec.w};
+      auto look = [&](int e, int n0, int n1, float2 a, float2 c, int ix, int iy) {
+        if (flex_clear(p, a, c)) return;
+        float nx, ny, w0, w1;
+        const float pen = flex_detect(p, a, c, qbuf, nx, ny, w0, w1);
+        const long long place = (long long)(ix * g.cny + iy) << 32 | e;
+        if (pen < 1e-4f && fabsf(pen) < qbuf && (pen < b.pen || (pen == b.pen && place < b.place)))
+          b = FlexBest{pen, nx, ny, w0, w1, e, n0, n1, place};
+      };
+      if (be_cnt <= kFlexEdgesPerCell * ncell) {
+        constexpr int U = 4;  // edges in flight per lane
+        for (int e0 = be_off + sub; e0 < be_off + be_cnt; e0 += U * kFlexLanes) {
+          int4 c[U];
+          int2 n[U];
+          float2 a[U], b2[U];
+#pragma unroll
+          for (int i = 0; i < U; ++i) {
+            const int e = e0 + i * kFlexLanes;
+            c[i] = make_int4(0x7FFFFFFF, 0, 0, 0);
+            if (e < be_off + be_cnt) {
+              c[i] = f.ecell[e];
+              n[i] = f.be[e];
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < U; ++i)
+            if (!(c[i].x > ux || c[i].z < lx || c[i].y > uy || c[i].w < ly)) {
+              a[i] = d.x[n[i].x];
+              b2[i] = d.x[n[i].y];
+            }
+#pragma unroll
+          for (int i = 0; i < U; ++i)
+            if (!(c[i].x > ux || c[i].z < lx || c[i].y > uy || c[i].w < ly)) {
+              ++num;
+              look(e0 + i * kFlexLanes, n[i].x, n[i].y, a[i], b2[i], max(lx, c[i].x), max(ly, c[i].y));
+            }
+        }
+      } else {
+        const int chunk = (ncell + kFlexLanes - 1) / kFlexLanes;
+        const int t1 = min(ncell, (sub + 1) * chunk);
+        for (int t = min(ncell, sub * chunk); t < t1; ++t) {
+          const int ix = lx + t / h, iy = ly + t % h;
+          const int2 r = f.crange[ix * g.cny + iy];
+          for (int q = r.x; q < r.y; ++q) {
+            const int4 rec = f.srec[q];  // element, domain, nodes
+            if (rec.y != target) continue;
+            const int2 ec = f.scell[q];
+            if (ix != (lx > ec.x ? lx : ec.x) || iy != (ly > ec.y ? ly : ec.y)) continue;  // seen earlier
+            ++num;
+            look(rec.x, rec.z, rec.w, d.x[rec.z], d.x[rec.w], ix, iy);
+          }
         }
       }
       for (int o = kFlexLanes / 2; o > 0; o >>= 1) num += __shfl_xor_sync(gmask, num, o);
@@ -654,67 +797,43 @@ __device__ __forceinline__ void flex_item(const Dev& d, const FlexDev& f, const 
         serial = true;  // the reference stops adding candidates at 512: walk as written
       } else {
         float wp = b.pen;
+        long long wk = b.place;
         int wl = sub;
-        for (int o = kFlexLanes / 2; o > 0; o >>= 1) {  // min penetration, ties to the lower lane
+        for (int o = kFlexLanes / 2; o > 0; o >>= 1) {  // min penetration, ties to the earlier place
           const float op = __shfl_xor_sync(gmask, wp, o);
+          const long long ok = __shfl_xor_sync(gmask, wk, o);
           const int ol = __shfl_xor_sync(gmask, wl, o);
-          if (op < wp || (op == wp && ol < wl)) {
+          if (op < wp || (op == wp && (ok < wk || (ok == wk && ol < wl)))) {
             wp = op;
+            wk = ok;
             wl = ol;
           }
         }
         const int src = (threadIdx.x & 31 & ~(kFlexLanes - 1)) + wl;
-        const int we = __shfl_sync(gmask, b.e, src);
-        const float pbest = __shfl_sync(gmask, b.pen, src), pnx = __shfl_sync(gmask, b.nx, src);
-        const float pny = __shfl_sync(gmask, b.ny, src), pw0 = __shfl_sync(gmask, b.w0, src);
-        const float pw1 = __shfl_sync(gmask, b.w1, src);
-        const int pn0 = __shfl_sync(gmask, b.n0, src), pn1 = __shfl_sync(gmask, b.n1, src);
-        if (we >= 0) {
-          best = pbest; bnx = pnx; bny = pny; bw0 = pw0; bw1 = pw1; bn0 = pn0; bn1 = pn1;
-          found = true;
-          cache_out = we;
-        }
+        b.e = __shfl_sync(gmask, b.e, src);
+        b.pen = wp;
+        b.nx = __shfl_sync(gmask, b.nx, src);
+        b.ny = __shfl_sync(gmask, b.ny, src);
+        b.w0 = __shfl_sync(gmask, b.w0, src);
+        b.w1 = __shfl_sync(gmask, b.w1, src);
+        b.n0 = __shfl_sync(gmask, b.n0, src);
+        b.n1 = __shfl_sync(gmask, b.n1, src);
       }
     }
-    if (serial) {  // every lane of the group walks the window (same result in each)
-      int cand[kFlexMaxQuery];
-      int num = 0;
-      for (int ix = lx; ix <= ux; ++ix)
-        for (int iy = ly; iy <= uy; ++iy) {
-          const int cid = ix + iy * g.cnx;
-          if (cid < 0 || cid >= g.tc) continue;
-          for (int q = f.cell_start[cid]; q < f.cell_end[cid]; ++q) {
-            const int e = f.sorted[q];
-            if (e < 0 || f.be_dom[e] != target) continue;
-            bool dup = false;
-            for (int k = 0; k < num; ++k) dup |= cand[k] == e;
-            if (!dup && num < kFlexMaxQuery) cand[num++] = e;
-          }
-        }
-      for (int j = 0; j < num; ++j) {
-        const int e = cand[j];
-        const int2 n = f.be[e];
-        float nx, ny, w0, w1;
-        const float pen = flex_detect(p, d.x[n.x], d.x[n.y], qbuf, nx, ny, w0, w1);
-        if (pen < best && pen < 1e-4f && fabsf(pen) < qbuf) {
-          best = pen; bnx = nx; bny = ny; bw0 = w0; bw1 = w1; bn0 = n.x; bn1 = n.y; found = true;
-          cache_out = e;
-        }
-      }
-    }
+    if (serial) b = flex_walk(d, f, g, p, qbuf, target, lx, ly, ux, uy);  // every lane of the group: the same result
   }
   if (sub != 0) return;
-  if (!found) cache_out = -1;
-  if (cache_out != cached) f.item_cache[it] = cache_out;
-  if (found && best < 0.0f) {
-    const float fx = -bnx * pen_k * best, fy = -bny * pen_k * best;
+  if (b.e != cached) f.item_cache[it] = b.e;
+  if (b.e >= 0 && b.pen < 0.0f) {
+    const int s1 = d.flex_slot[b.n0], s2 = d.flex_slot[b.n1];
+    const float fx = -b.nx * pen_k * b.pen, fy = -b.ny * pen_k * b.pen;
     float tx = fx, ty = fy;
     if (fric > 1e-9f) {
-      const float2 va = d.v[bn0], vb = d.v[bn1];
-      const float sx = va.x * bw0 + vb.x * bw1, sy = va.y * bw0 + vb.y * bw1;
+      const float2 va = d.v[b.n0], vb = d.v[b.n1];
+      const float sx = va.x * b.w0 + vb.x * b.w1, sy = va.y * b.w0 + vb.y * b.w1;
       const float rx = vp.x - sx, ry = vp.y - sy;
-      const float dn = rx * bnx + ry * bny;
-      const float gx = rx - dn * bnx, gy = ry - dn * bny;
+      const float dn = rx * b.nx + ry * b.ny;
+      const float gx = rx - dn * b.nx, gy = ry - dn * b.ny;
       const float tl = sqrtf(gx * gx + gy * gy);
       if (tl > 1e-9f) {
         const float ddx = -gx / tl, ddy = -gy / tl;
@@ -724,30 +843,37 @@ __device__ __forceinline__ void flex_item(const Dev& d, const FlexDev& f, const 
       }
     }
     const int key = f.n_items + it;  // after every tie entry of the node
-    flex_push(d, f.err, nid, key, make_float2(tx, ty));
-    flex_push(d, f.err, bn0, key, make_float2(-(tx * bw0), -(ty * bw0)));
-    flex_push(d, f.err, bn1, key, make_float2(-(tx * bw1), -(ty * bw1)));
+    // flex_push for the node and the edge's two, their list places taken together
+    const int j0 = atomicAdd(&d.flex_cnt[s0], 1), j1 = atomicAdd(&d.flex_cnt[s1], 1), j2 = atomicAdd(&d.flex_cnt[s2], 1);
+    flex_put(d, f.err, s0, j0, key, make_float2(tx, ty));
+    flex_put(d, f.err, s1, j1, key, make_float2(-(tx * b.w0), -(ty * b.w0)));
+    flex_put(d, f.err, s2, j2, key, make_float2(-(tx * b.w1), -(ty * b.w1)));
   }
 }
 
-// Each group of kFlexLanes lanes takes active work items in turn (grid
-// stride over the compacted list): the item's segment by binary search over
-// the segment offsets, then flex_item.
-__global__ void __launch_bounds__(kFlexContactThreads) k_flex_contact(Dev d, FlexDev f0) {
+// Second launch of a substep: a warp per group of work items (grid stride).
+// control != 0: one block does the scenes' step control meanwhile, which only
+// the node step waits for.
+// Bound by the latency of an item's chain of loads (node, cached edge, window,
+// candidates), times the groups a warp takes.  36 disks in contact: a substep
+// went from 49.2 to 22.3 us; four disks of 160 edges from 108 to 22, of 400
+// edges from 269 to 20.  Blocks of 64 threads: 22.3 us against 24.1 at 128, 23.6
+// at 32 (a block's registers are free again when its slower warp ends); groups
+// of 8 items run the disks of 400 edges in 23.3 us instead of 20.0.
+__global__ void __launch_bounds__(kFlexContactThreads) k_flex_contact(Dev d, FlexDev f0, int control) {
+  if (control && blockIdx.x == 0) {
+    if (blockIdx.y == 0) step_control(d);
+    return;
+  }
   const FlexDev f = flex_view(f0, blockIdx.y);  // blockIdx.y: the scene
-  const int sub = threadIdx.x % kFlexLanes;
-  const unsigned gmask = ((1u << kFlexLanes) - 1u) << ((threadIdx.x & 31) & ~(kFlexLanes - 1));
+  const int lane = threadIdx.x & 31, sub = lane % kFlexLanes;
+  const unsigned gmask = ((1u << kFlexLanes) - 1u) << (lane & ~(kFlexLanes - 1));
   const FlexGrid g = *f.g;
-  const int groups = gridDim.x * (blockDim.x / kFlexLanes);
-  for (int a = blockIdx.x * (blockDim.x / kFlexLanes) + threadIdx.x / kFlexLanes; a < g.n_active; a += groups) {
-    int lo = 0, hi = f.n_seg - 1;  // the last segment whose offset is <= a (the active one of a run)
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (f.seg_off[mid] <= a) lo = mid;
-      else hi = mid - 1;
-    }
-    const int4 sg = f.seg[lo];
-    flex_item(d, f, g, sg.x + (a - f.seg_off[lo]), sg.w, sub, gmask);
+  const int warps = (gridDim.x - control) * (blockDim.x / 32);
+  for (int u = (blockIdx.x - control) * (blockDim.x / 32) + (threadIdx.x >> 5); u < g.n_units; u += warps) {
+    const int4 w = f.unit[u];
+    const int j = lane / kFlexLanes;
+    if (j < w.y) flex_item(d, f, g, w.x + j, w.z, sub, gmask);
   }
 }
 

@@ -137,7 +137,6 @@ struct Dev {
 
 }  // namespace
 
-#include "fw_flex.cuh"
 
 namespace {
 
@@ -340,6 +339,12 @@ __device__ __forceinline__ void elements_pass(const Dev& d, int nb) {
   }
 }
 
+}  // namespace
+
+#include "fw_flex.cuh"
+
+namespace {
+
 __global__ void __launch_bounds__(kMaxBlock) k_elements(Dev d) { elements_pass(d, gridDim.x); }
 
 // Worlds with FEM-rigid contact: blocks [0, eb) run the element step, the
@@ -366,30 +371,67 @@ __global__ void __launch_bounds__(kMaxBlock) k_elements_rigid(Dev d, int eb) {
   }
 }
 
-// This substep's FEM-FEM contact forces on one node, in work-item order (the
-// reference adds them with atomic_add in launch order): the entries' item ids
-// are distinct, so each pass adds the entry with the next larger id.  The list
-// is emptied for the next substep.
-__device__ __forceinline__ void flex_add(const Dev& d, int slot, float2& f) {
-  const int n = min(d.flex_cnt[slot], kFlexListCap);
-  const int* items = d.flex_item + slot * kFlexListCap;
-  const float2* forces = d.flex_force + slot * kFlexListCap;
-  int last = -1;
-  for (int r = 0; r < n; ++r) {
-    int pick = 0, best = 0x7FFFFFFF;
-    for (int j = 0; j < n; ++j) {
-      const int w = items[j];
-      if (w > last && w < best) {
-        best = w;
-        pick = j;
-      }
-    }
-    const float2 c = forces[pick];
-    f.x += c.x;
-    f.y += c.y;
-    last = best;
+// This substep's FEM-FEM contact forces on one node: their number and the
+// first four, loaded with the node's own state.
+struct FlexList {
+  int slot = -1, n = 0;
+  int4 item;
+  float4 f01, f23;
+  __device__ __forceinline__ void load(const Dev& d, int i) {
+    slot = d.flex_slot[i];
+    if (slot < 0) return;
+    n = min(d.flex_cnt[slot], kFlexListCap);
+    if (n == 0) return;
+    item = *reinterpret_cast<const int4*>(d.flex_item + slot * kFlexListCap);
+    const float4* f = reinterpret_cast<const float4*>(d.flex_force + slot * kFlexListCap);
+    f01 = f[0];
+    f23 = f[1];
   }
-  d.flex_cnt[slot] = 0;
+};
+
+// Adds them in work-item order (the reference adds them with atomic_add in
+// launch order): the entries' item ids are distinct, so each pass adds the
+// entry with the next larger id.  The list is emptied for the next substep.
+__device__ __forceinline__ void flex_add(const Dev& d, const FlexList& l, float2& f) {
+  if (l.n == 0) return;
+  if (l.n <= 4) {
+    int4 w = l.item;
+    if (l.n < 4) w.w = 0x7FFFFFFF;
+    if (l.n < 3) w.z = 0x7FFFFFFF;
+    if (l.n < 2) w.y = 0x7FFFFFFF;
+    for (int r = 0; r < l.n; ++r) {
+      const int m = min(min(w.x, w.y), min(w.z, w.w));
+      const float2 c = w.x == m   ? make_float2(l.f01.x, l.f01.y)
+                       : w.y == m ? make_float2(l.f01.z, l.f01.w)
+                       : w.z == m ? make_float2(l.f23.x, l.f23.y)
+                                  : make_float2(l.f23.z, l.f23.w);
+      if (w.x == m) w.x = 0x7FFFFFFF;
+      if (w.y == m) w.y = 0x7FFFFFFF;
+      if (w.z == m) w.z = 0x7FFFFFFF;
+      if (w.w == m) w.w = 0x7FFFFFFF;
+      f.x += c.x;
+      f.y += c.y;
+    }
+  } else {
+    const int* items = d.flex_item + l.slot * kFlexListCap;
+    const float2* forces = d.flex_force + l.slot * kFlexListCap;
+    int last = -1;
+    for (int r = 0; r < l.n; ++r) {
+      int pick = 0, best = 0x7FFFFFFF;
+      for (int j = 0; j < l.n; ++j) {
+        const int w = items[j];
+        if (w > last && w < best) {
+          best = w;
+          pick = j;
+        }
+      }
+      const float2 c = forces[pick];
+      f.x += c.x;
+      f.y += c.y;
+      last = best;
+    }
+  }
+  d.flex_cnt[l.slot] = 0;
 }
 
 // The node's own state, its CSR range and its first kNodeCorners corner
@@ -411,6 +453,8 @@ __device__ __forceinline__ void node_step(const Dev& d, int i, bool valid) {
     mass = d.mass[i];
     bv0 = d.bcv[i];
   }
+  FlexList fl;
+  if (FLEX && valid && (w & fw::NODE_BOUNDARY)) fl.load(d, i);
   float2 cq[kNodeCorners];
 #pragma unroll
   for (int u = 0; u < kNodeCorners; ++u) cq[u] = k0 + u < k1 ? d.corner[k0 + u] : make_float2(0.f, 0.f);
@@ -426,12 +470,11 @@ __device__ __forceinline__ void node_step(const Dev& d, int i, bool valid) {
     bnd = (w & fw::NODE_BOUNDARY) != 0;
     if (bnd && mode == fw::MODE_STEP) {
       const int p0 = d.body_pair_off[b], pn = d.body_pair_cnt[b];
-      const int fs = FLEX ? d.flex_slot[i] : -1;
       const int bs = RIGID ? d.bslot[i] : 0;  // this node's slot in its body's boundary list
-      bool flex_done = !FLEX || fs < 0;
+      bool flex_done = !FLEX || fl.slot < 0;
       for (int k = 0; k < pn; ++k) {
         if (FLEX && !flex_done && d.pairs[p0 + k].kind != fw::PAIR_PLANE) {
-          flex_add(d, fs, f);  // FEM-FEM contact runs after the planes, before the height fields / voxels
+          flex_add(d, fl, f);  // FEM-FEM contact runs after the planes, before the height fields / voxels
           flex_done = true;
         }
         if (RIGID && d.pairs[p0 + k].kind == fw::PAIR_RIGID) {
@@ -455,7 +498,7 @@ __device__ __forceinline__ void node_step(const Dev& d, int i, bool valid) {
           f.y += cf.y;
         }
       }
-      if (FLEX && !flex_done) flex_add(d, fs, f);
+      if (FLEX && !flex_done) flex_add(d, fl, f);
     }
 #pragma unroll
     for (int u = 0; u < kNodeCorners; ++u)  // contiguous, ascending element
@@ -1466,23 +1509,25 @@ void set_grids(fw_ctx* c) {
 }
 
 // The FEM-FEM contact of one substep (force: the construction-time hash
-// build only): k_flex_pre (hash clock, the rebuild when it fires, activation,
-// the active work items), then the contact work items.
+// build only): k_flex_pre, then k_flex_contact.  Worlds without rigid bodies
+// have the element step in the first and the step control in the second.
 void flex_launch(fw_ctx* c, int force) {
   const FlexDev& f = c->fx;
-  k_flex_pre<<<f.n_fs, kFlexScanThreads, c->flex_pre_smem, c->stream>>>(c->d, f, force);
+  const int with_step = force || c->has_rigid ? 0 : 1;
+  const int eb = with_step ? std::max(1, std::min((c->E + 127) / 128, std::max(c->sms - f.n_fs, (c->E + 2047) / 2048))) : 0;
+  k_flex_pre<<<f.n_fs + eb, kFlexScanThreads, c->flex_pre_smem, c->stream>>>(c->d, f, force);
   c->launches += 1;
   if (!force) {
     const int64_t threads = (int64_t)f.n_items * kFlexLanes;
     const int64_t want = (threads + kFlexContactThreads - 1) / kFlexContactThreads;
     const int bx = (int)std::max<int64_t>(1, std::min<int64_t>(want, 8 * c->sms) / f.n_fs);
-    k_flex_contact<<<dim3(bx, f.n_fs), kFlexContactThreads, 0, c->stream>>>(c->d, f);
+    k_flex_contact<<<dim3(bx + with_step, f.n_fs), kFlexContactThreads, 0, c->stream>>>(c->d, f, with_step);
     c->launches += 1;
   }
 }
 
 // Kernel launches of one gather-path substep.
-int step_launches(const fw_ctx* c) { return 2 + (c->has_flex ? 2 : 0) + (c->has_rigid ? 1 : 0); }
+int step_launches(const fw_ctx* c) { return (c->has_flex ? (c->has_rigid ? 4 : 3) : 2) + (c->has_rigid ? 1 : 0); }
 
 int launch_step(fw_ctx* c) {
   if (c->has_flex) flex_launch(c, 0);
@@ -1499,14 +1544,13 @@ int launch_step(fw_ctx* c) {
     else
       k_rigid<<<(c->rd.n + kRigidThreads / 32 - 1) / (kRigidThreads / 32), kRigidThreads, 0, c->stream>>>(c->d, c->rd);
     c->launches += 1;
+  } else if (c->has_flex) {
+    k_nodes_flex<<<c->grid_n, c->block_n, 0, c->stream>>>(c->d);
   } else {
     k_elements<<<c->grid_e, c->block_e, 0, c->stream>>>(c->d);
-    if (c->has_flex)
-      k_nodes_flex<<<c->grid_n, c->block_n, 0, c->stream>>>(c->d);
-    else
-      k_nodes<<<c->grid_n, c->block_n, 0, c->stream>>>(c->d);
+    k_nodes<<<c->grid_n, c->block_n, 0, c->stream>>>(c->d);
   }
-  c->launches += 2;
+  c->launches += c->has_flex && !c->has_rigid ? 1 : 2;
   return check_kernel(c, "step");
 }
 
@@ -3777,6 +3821,7 @@ int build_flex(fw_ctx* c) {
   std::vector<int2> pair_body;
   std::vector<int32_t> pair_tied;
   std::vector<int4> segs;  // (first item, count, pair in its scene, target)
+  int n_units = 0;
   std::vector<FlexScene> scs;
   std::vector<int32_t> dom_obj, dom_body;
   std::vector<float4> dom_box;
@@ -3837,6 +3882,8 @@ int build_flex(fw_ctx* c) {
       }
     }
     fsd.n_seg = (int)segs.size() - fsd.seg_base;
+    fsd.unit_base = n_units;
+    for (int k = fsd.seg_base; k < (int)segs.size(); ++k) n_units += (segs[k].y + kFlexUnit - 1) / kFlexUnit;
     for (int k = fsd.be0; k < fsd.be0 + fsd.n_be; ++k)  // edge nodes receive the reactions
       for (int n : {c->h_be[k].x, c->h_be[k].y})
         if (slot[n] < 0) slot[n] = n_slots++;
@@ -3859,18 +3906,16 @@ int build_flex(fw_ctx* c) {
     dom_box.push_back(make_float4(0.f, 0.f, 0.f, 0.f));
   }
   std::vector<int32_t> minus1(std::max(n_items, 1), -1);
-  // each scene's seg_off has n_seg + 1 entries: seg_base + k
-  const size_t n_segoff = segs.size() + (size_t)n_fs;
   int rc;
   int32_t *inode = nullptr, *itgt = nullptr, *ipair = nullptr, *icache = nullptr, *bdom = nullptr, *boff = nullptr,
-          *bcnt = nullptr, *dobj = nullptr, *dbody = nullptr, *pact = nullptr, *stamp = nullptr, *ecount = nullptr,
+          *bcnt = nullptr, *dobj = nullptr, *dbody = nullptr, *ecount = nullptr,
           *ebase = nullptr, *ccount = nullptr, *cstart = nullptr, *cend = nullptr, *cursor = nullptr,
-          *sorted = nullptr, *dslot = nullptr, *dcnt = nullptr, *ditem = nullptr, *dsegoff = nullptr;
+          *sorted = nullptr, *dslot = nullptr, *dcnt = nullptr, *ditem = nullptr;
   float *ipen = nullptr, *ifric = nullptr;
   int32_t *ptied = nullptr, *telem = nullptr;
   float *tw0 = nullptr, *tw1 = nullptr, *tgap = nullptr;
-  int2 *pbody = nullptr, *dbe = nullptr, *crange = nullptr, *ecell = nullptr, *scell = nullptr;
-  int4 *srec = nullptr, *dseg = nullptr;
+  int2 *pbody = nullptr, *dbe = nullptr, *crange = nullptr, *scell = nullptr;
+  int4 *srec = nullptr, *dseg = nullptr, *ecell = nullptr, *bcell = nullptr, *dunit = nullptr;
   float4 *dbox = nullptr, *ebox = nullptr;
   float2* dforce = nullptr;
   FlexGrid* grid = nullptr;
@@ -3881,13 +3926,12 @@ int build_flex(fw_ctx* c) {
       (rc = upload(c, &pbody, pair_body)) || (rc = upload(c, &dbe, c->h_be)) || (rc = upload(c, &bdom, be_dom)) ||
       (rc = upload(c, &boff, be_off)) || (rc = upload(c, &bcnt, be_cnt)) || (rc = upload(c, &dobj, dom_obj)) ||
       (rc = upload(c, &dbody, dom_body)) || (rc = upload(c, &dbox, dom_box)) || (rc = upload(c, &dsc, scs)) ||
-      (rc = dalloc(c, &pact, std::max<size_t>(1, pair_body.size()))) || (rc = dalloc(c, &stamp, B)) ||
       (rc = dalloc(c, &grid, n_fs)) || (rc = dalloc(c, &ebox, n_be)) || (rc = dalloc(c, &ecount, n_be)) ||
       (rc = dalloc(c, &ebase, n_be)) || (rc = dalloc(c, &ccount, cells)) || (rc = dalloc(c, &cstart, cells)) ||
       (rc = dalloc(c, &cend, cells)) || (rc = dalloc(c, &cursor, cells)) || (rc = dalloc(c, &crange, cells)) ||
       (rc = dalloc(c, &sorted, (size_t)pair_base)) || (rc = dalloc(c, &srec, (size_t)pair_base)) ||
       (rc = dalloc(c, &scell, (size_t)pair_base)) || (rc = dalloc(c, &ecell, n_be)) ||
-      (rc = upload(c, &dseg, segs)) || (rc = dalloc(c, &dsegoff, n_segoff)) ||
+      (rc = upload(c, &dseg, segs)) || (rc = dalloc(c, &bcell, B)) || (rc = dalloc(c, &dunit, std::max(1, n_units))) ||
       (rc = upload(c, &dslot, slot)) || (rc = dalloc(c, &dcnt, std::max(1, n_slots))) ||
       (rc = dalloc(c, &ditem, std::max(1, n_slots) * kFlexListCap)) ||
       (rc = dalloc(c, &dforce, std::max(1, n_slots) * kFlexListCap)) || (rc = dalloc(c, &c->d_flex_clock, n_fs)) ||
@@ -3903,11 +3947,11 @@ int build_flex(fw_ctx* c) {
   FW_CUDA(c, cudaMemsetAsync(cend, 0, sizeof(int32_t) * cells, c->stream));
   f.item_node = inode; f.item_target = itgt; f.item_pair = ipair; f.item_pen = ipen; f.item_fric = ifric;
   f.item_cache = icache; f.pair_body = pbody; f.be = dbe; f.be_dom = bdom; f.be_off = boff; f.be_cnt = bcnt;
-  f.dom_obj = dobj; f.dom_body = dbody; f.dom_box = dbox; f.pair_active = pact; f.stamped = stamp; f.g = grid;
+  f.dom_obj = dobj; f.dom_body = dbody; f.dom_box = dbox; f.g = grid;
   f.ebox = ebox; f.ecount = ecount; f.ebase = ebase; f.cell_count = ccount; f.cell_start = cstart;
   f.cell_end = cend; f.cursor = cursor; f.sorted = sorted; f.crange = crange; f.ecell = ecell;
   f.srec = srec; f.scell = scell;
-  f.seg = dseg; f.seg_off = dsegoff;
+  f.seg = dseg; f.unit = dunit; f.bcell = bcell;
   f.sc = dsc; f.clock_dt = c->d_flex_clock; f.err = c->d_flags + fw_ctx::kFlagFlex;
   f.pair_tied = ptied; f.tie_elem = telem; f.tie_w0 = tw0; f.tie_w1 = tw1; f.tie_gap = tgap;
   c->flex_pre_smem = sizeof(float4) * (size_t)max_dom_fem;

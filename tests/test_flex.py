@@ -211,3 +211,33 @@ def test_gpu_tied_pairs_equal_oracle():
         assert np.array_equal(lp.femSpringManager.coords.numpy()[:n].astype(np.float64), xo), k
         assert np.array_equal(lp.femSpringManager.V.numpy()[:n].astype(np.float64), vo), k
 
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells,radius,steps", [(3, 0.025, 300), (16, 0.025, 300), (17, 0.025, 150), (80, 1.2, 150), (140, 0.009, 6)])
+def test_gpu_edge_search_equals_oracle(cells, radius, steps):
+    """Two touching disks over the ways of finding an item's edge: the target's
+    own edges (small disks), the window's cells (few cells, many edges: radius
+    1.2), and the walk past 512 candidates (a disk inside the query window)."""
+
+    def build():
+        c = [0.1, radius], [0.1 + 2 * radius * (1.0 - 2e-4), radius]
+        return [fw.GroundDomain(2, [0.0, 0.0], [0.0, 1.0])] + [
+            fw.FemDomain(scenes.ccw_disk(fw, cells, radius, at), fw.SolidProp(mat(E=1e5, nu=0.3, rho=1000.0)),
+                         [fw.Gravity([g, -9.8])], friction=0.2)
+            for at, mat, g in zip(c, (fw.Elastic, fw.HyperElastic), (9.8, -9.8))]
+
+    dt = 0.3 * oracle.OracleLoop(build(), useAdapativeDT=True).dt
+    lp = fw.ExplicitLoop(dt, build(), useAdapativeDT=False)
+    o = oracle.OracleLoop(build(), dt=dt, useAdapativeDT=False, threads=4)
+    touched = False
+    for k in range(3):
+        lp.advance_n(steps // 3)
+        o.advance(steps // 3)
+        xo, vo, _ = o.state()
+        assert np.array_equal(lp.femSpringManager.coords.numpy()[: o.N].astype(np.float64), xo), k
+        assert np.array_equal(lp.femSpringManager.V.numpy()[: o.N].astype(np.float64), vo), k
+        cache, _ = lp._native.read_flex_state(len(o.flex_cache()))
+        assert np.array_equal(cache, o.flex_cache()), k
+        touched |= bool((cache >= 0).any())
+    assert touched
