@@ -9,12 +9,13 @@
 //   flatworld/rigidmanager.py:832-964       _rigid_step_wp, _update_u_and_bbox_wp
 //   flatworld/explicitloop.py:533-552       the rigid update every N substeps
 //
-// Per substep, the node kernel evaluates each FEM-rigid work item of its node
-// (pair order, after FEM-FEM contact and before the height fields) and writes
-// the item's reaction (impulse, torque, rigid) to its slot; k_rigid then adds
-// the reactions to the rigid accumulators in work-item order -- the order in
-// which a serial run of the reference's atomic adds applies them -- and, on
-// the substeps the schedule names, runs the rigid velocity and position update.
+// Per substep, k_elements_rigid evaluates every FEM-rigid work item and writes
+// the item's reaction (impulse, torque, rigid) to its slot; the node step adds
+// the items' forces (pair order, after FEM-FEM contact and before the height
+// fields) while the rigid side adds the reactions to the rigid accumulators in
+// work-item order -- the order in which a serial run of the reference's atomic
+// adds applies them -- and, on the substeps the schedule names, runs the rigid
+// velocity and position update.
 #pragma once
 #include "fw_device.cuh"
 
@@ -276,10 +277,14 @@ constexpr float kRigidClearance = 0.01f;
 // another contact rigid's box sets bit 0 of *err: the reference would solve
 // that contact, this library does not.  So does a rigid whose state is no
 // longer finite.
+//
+// By one warp, a lane per rigid: the checks read every box before any of them
+// moves, and nothing else reads another rigid.
 __device__ __forceinline__ void rigid_update(Rigid* rig, int n, const float4* gbox, const int* gkind,
-                                             int n_ground, float dt, float damping, int* err) {
+                                             int n_ground, float dt, float damping, int* err, int lane) {
   const float cl = kRigidClearance;
-  for (int a = 0; a < n; ++a) {
+  bool bad = false;
+  for (int a = lane; a < n; a += 32) {
     const Rigid& g = rig[a];
     if (g.type == RIGID_ANALYTICAL) continue;  // not a rigid body
     for (int q = 0; q < n_ground; ++q) {
@@ -287,56 +292,53 @@ __device__ __forceinline__ void rigid_update(Rigid* rig, int n, const float4* gb
       // written as "not clear", so that a non-finite box is flagged too
       if (gkind[q] == 0) {
         const float sx = b.z < 0.0f ? g.ub[0] : g.lb[0], sy = b.w < 0.0f ? g.ub[1] : g.lb[1];
-        if (!((sx - b.x) * b.z + (sy - b.y) * b.w > cl)) *err |= 1;
-      } else if (!(g.lb[0] - cl > b.z || g.ub[0] + cl < b.x || g.lb[1] - cl > b.w || g.ub[1] + cl < b.y)) {
-        *err |= 1;
+        bad |= !((sx - b.x) * b.z + (sy - b.y) * b.w > cl);
+      } else {
+        bad |= !(g.lb[0] - cl > b.z || g.ub[0] + cl < b.x || g.lb[1] - cl > b.w || g.ub[1] + cl < b.y);
       }
     }
     for (int q = a + 1; q < n; ++q) {
       const Rigid& h = rig[q];
-      if (h.type != RIGID_ANALYTICAL && g.in_contact && h.in_contact &&
-          !(g.lb[0] - cl > h.ub[0] || g.ub[0] + cl < h.lb[0] || g.lb[1] - cl > h.ub[1] || g.ub[1] + cl < h.lb[1]))
-        *err |= 1;
+      bad |= h.type != RIGID_ANALYTICAL && g.in_contact && h.in_contact &&
+             !(g.lb[0] - cl > h.ub[0] || g.ub[0] + cl < h.lb[0] || g.lb[1] - cl > h.ub[1] || g.ub[1] + cl < h.lb[1]);
     }
-    if (!(fabsf(g.c[0]) < 1e30f && fabsf(g.c[1]) < 1e30f && fabsf(g.quat) < 1e30f)) *err |= 1;
+    bad |= !(fabsf(g.c[0]) < 1e30f && fabsf(g.c[1]) < 1e30f && fabsf(g.quat) < 1e30f);
   }
-  for (int a = 0; a < n; ++a) {  // _rigid_step_wp
-    Rigid& g = rig[a];
+  if (bad) atomicOr(err, 1);
+  __syncwarp();
+  for (int a = lane; a < n; a += 32) {
+    Rigid g = rig[a];
     rigid_rot(g);
-    if (g.type == RIGID_ANALYTICAL) continue;  // the impulse pass covers the rigid bodies only
-    if (g.bc & RBC_A) {
-      g.acc[0] = 0.0f;
-      g.acc[1] = 0.0f;
-    } else {
-      if (g.bc & RBC_GRAVITY) {
-        g.acc[0] = g.acc[0] + g.mass * g.bcG[0] * dt;
-        g.acc[1] = g.acc[1] + g.mass * g.bcG[1] * dt;
+    if (g.type != RIGID_ANALYTICAL) {  // _rigid_step_wp; the impulse pass covers the rigid bodies only
+      if (g.bc & RBC_A) {
+        g.acc[0] = 0.0f;
+        g.acc[1] = 0.0f;
+      } else {
+        if (g.bc & RBC_GRAVITY) {
+          g.acc[0] = g.acc[0] + g.mass * g.bcG[0] * dt;
+          g.acc[1] = g.acc[1] + g.mass * g.bcG[1] * dt;
+        }
+        if (g.bc & RBC_FORCE) {
+          g.acc[0] = g.acc[0] + g.bcT[0] * dt;
+          g.acc[1] = g.acc[1] + g.bcT[1] * dt;
+        }
       }
-      if (g.bc & RBC_FORCE) {
-        g.acc[0] = g.acc[0] + g.bcT[0] * dt;
-        g.acc[1] = g.acc[1] + g.bcT[1] * dt;
-      }
+      if (g.bc & RBC_ROTA) g.accw = 0.0f;
+      else if (g.bc & RBC_TORQUE) g.accw = g.accw + g.bcR * dt;
+      g.V[0] = g.V[0] + g.acc[0] / g.mass;
+      g.V[1] = g.V[1] + g.acc[1] / g.mass;
+      g.W = g.W + g.accw / (g.inertia + 1e-6f);
+      const float damp = rmax(0.0f, 1.0f - damping * dt);
+      g.V[0] = g.V[0] * damp;
+      g.V[1] = g.V[1] * damp;
+      g.W = g.W * damp;
     }
-    if (g.bc & RBC_ROTA) g.accw = 0.0f;
-    else if (g.bc & RBC_TORQUE) g.accw = g.accw + g.bcR * dt;
-    g.V[0] = g.V[0] + g.acc[0] / g.mass;
-    g.V[1] = g.V[1] + g.acc[1] / g.mass;
-    g.W = g.W + g.accw / (g.inertia + 1e-6f);
-    const float damp = rmax(0.0f, 1.0f - damping * dt);
-    g.V[0] = g.V[0] * damp;
-    g.V[1] = g.V[1] * damp;
-    g.W = g.W * damp;
-  }
-  for (int a = 0; a < n; ++a) {
-    Rigid& g = rig[a];
     if (g.bc & RBC_A) {
       g.V[0] = g.V[0] + g.bcT[0] * dt;
       g.V[1] = g.V[1] + g.bcT[1] * dt;
     }
     if (g.bc & RBC_ROTA) g.W = g.W + g.bcR * dt;
-  }
-  for (int a = 0; a < n; ++a) {  // _update_u_and_bbox_wp
-    Rigid& g = rig[a];
+    // _update_u_and_bbox_wp
     if (g.bc & RBC_V) {
       g.V[0] = g.bcT[0];
       g.V[1] = g.bcT[1];
@@ -357,13 +359,12 @@ __device__ __forceinline__ void rigid_update(Rigid* rig, int n, const float4* gb
     g.quat = g.quat + g.W * dt;
     if (g.quat > 3.141592653589793f) g.quat = g.quat - 2.0f * 3.141592653589793f;
     else if (g.quat < -3.141592653589793f) g.quat = g.quat + 2.0f * 3.141592653589793f;
+    g.acc[0] = 0.0f;
+    g.acc[1] = 0.0f;
+    g.accw = 0.0f;
+    rigid_aabb(g);
+    rig[a] = g;
   }
-  for (int a = 0; a < n; ++a) {
-    rig[a].acc[0] = 0.0f;
-    rig[a].acc[1] = 0.0f;
-    rig[a].accw = 0.0f;
-  }
-  for (int a = 0; a < n; ++a) rigid_aabb(rig[a]);
 }
 
 }  // namespace fw

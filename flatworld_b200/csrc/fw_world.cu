@@ -319,8 +319,8 @@ __device__ __forceinline__ void cfl_reduce(const Dev& d, int e, float dtc) {
   if ((int)(threadIdx.x & 31) == __ffs(grp) - 1 && m < 0x7f800000) atomicMin(d.cfl_ord + s, m);
 }
 
-// The element step over blocks [0, nb) of the grid.
-__device__ __forceinline__ void elements_pass(const Dev& d, int nb) {
+__global__ void __launch_bounds__(kMaxBlock) k_elements(Dev d) {
+  const int nb = gridDim.x;
   if (blockIdx.x == 0) step_control(d);
   if (d.use_chunks) {
     for (int c = blockIdx.x; c < d.n_e_chunks; c += nb) {
@@ -345,22 +345,29 @@ __device__ __forceinline__ void elements_pass(const Dev& d, int nb) {
 
 namespace {
 
-__global__ void __launch_bounds__(kMaxBlock) k_elements(Dev d) { elements_pass(d, gridDim.x); }
-
-// Worlds with FEM-rigid contact: blocks [0, eb) run the element step, the
-// others evaluate every FEM-rigid work item -- one thread per item instead of
-// one thread per boundary node walking all its rigid pairs -- from the
-// substep's start state, whatever the gate and the scene's mode (the node
-// step uses an item only when its scene steps and its pair is gated on).
+// Worlds with FEM-rigid contact: block 0 does the step control, blocks [1, eb]
+// run the element step, the others evaluate every FEM-rigid work item -- one
+// thread per item instead of one thread per boundary node walking all its rigid
+// pairs -- from the substep's start state, whatever the gate and the scene's
+// mode (the node step and the rigid sums use an item only when its scene steps
+// and its pair is gated on).
 // rigid_item adds its force to a -0 start, which leaves it exactly as it
 // would be added to the node's sum.
 __global__ void __launch_bounds__(kMaxBlock) k_elements_rigid(Dev d, int eb) {
-  if ((int)blockIdx.x < eb) {
-    elements_pass(d, eb);
+  if (blockIdx.x == 0) {
+    step_control(d);
     return;
   }
-  const int stride = (gridDim.x - eb) * blockDim.x;
-  for (int it = (blockIdx.x - eb) * blockDim.x + threadIdx.x; it < d.n_ritems; it += stride) {
+  const int b = blockIdx.x - 1;
+  if (b < eb) {
+    for (int e = b * blockDim.x + threadIdx.x; e < d.E; e += eb * blockDim.x) {
+      const float dtc = element_step(d, e);
+      if (d.cfl_ord) cfl_reduce(d, e, dtc);
+    }
+    return;
+  }
+  const int stride = (gridDim.x - 1 - eb) * blockDim.x;
+  for (int it = (b - eb) * blockDim.x + threadIdx.x; it < d.n_ritems; it += stride) {
     const int2 w = d.rwork[it];
     const Pair& pr = d.pairs[w.x];
     const float dt = d.uniform_dt ? d.dt_uniform : d.scene_dt[d.body_scene[pr.body]];
@@ -472,28 +479,44 @@ __device__ __forceinline__ void node_step(const Dev& d, int i, bool valid) {
       const int p0 = d.body_pair_off[b], pn = d.body_pair_cnt[b];
       const int bs = RIGID ? d.bslot[i] : 0;  // this node's slot in its body's boundary list
       bool flex_done = !FLEX || fl.slot < 0;
-      for (int k = 0; k < pn; ++k) {
-        if (FLEX && !flex_done && d.pairs[p0 + k].kind != fw::PAIR_PLANE) {
-          flex_add(d, fl, f);  // FEM-FEM contact runs after the planes, before the height fields / voxels
-          flex_done = true;
+      // U pairs at a time.  Rigid pairs: the items were evaluated by
+      // k_elements_rigid from this same state, and are fetched together (one
+      // after the other, the 13 pairs of a slab under 12 rigids were a chain of
+      // 39 loads).
+      constexpr int U = RIGID ? 4 : 1;
+      for (int k0 = 0; k0 < pn; k0 += U) {
+        int kind[U], on[U], slot[U];
+        float2 rf[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          on[u] = 0;
+          if (k0 + u >= pn) continue;
+          const Pair& pr = d.pairs[p0 + k0 + u];
+          on[u] = d.pair_active[p0 + k0 + u];
+          kind[u] = pr.kind;
+          slot[u] = pr.n0 + bs;
         }
-        if (RIGID && d.pairs[p0 + k].kind == fw::PAIR_RIGID) {
-          // the item was evaluated by k_elements_rigid from this same state
-          const int slot = d.pairs[p0 + k].n0 + bs;
-          if (d.pair_active[p0 + k]) {
-            if (__float_as_int(d.ritem[slot].w) >= 0) {
-              const float2 rf = d.rforce[slot];
-              f.x += rf.x;
-              f.y += rf.y;
+        if (RIGID) {
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (k0 + u < pn && kind[u] == fw::PAIR_RIGID && on[u]) {
+              on[u] = __float_as_int(d.ritem[slot[u]].w) >= 0;
+              rf[u] = d.rforce[slot[u]];
             }
-          } else {
-            d.ritem[slot] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-          }
-          continue;
         }
-        if (!d.pair_active[p0 + k]) continue;
-        float2 cf;
-        if (fw::contact_force(d.pairs[p0 + k], d.heights, d.occ, d.vox, x, v, dt, cf)) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (k0 + u >= pn) continue;
+          if (FLEX && !flex_done && kind[u] != fw::PAIR_PLANE) {
+            flex_add(d, fl, f);  // FEM-FEM contact runs after the planes, before the height fields / voxels
+            flex_done = true;
+          }
+          if (!on[u]) continue;
+          float2 cf;
+          if (RIGID && kind[u] == fw::PAIR_RIGID)
+            cf = rf[u];
+          else if (!fw::contact_force(d.pairs[p0 + k0 + u], d.heights, d.occ, d.vox, x, v, dt, cf))
+            continue;
           f.x += cf.x;
           f.y += cf.y;
         }
@@ -569,23 +592,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_nodes_flex(Dev d) {
   node_step<true, false>(d, i, i < d.N);
 }
 
-// k_nodes of worlds with FEM-rigid contact (FLEX: FEM-FEM contact as well).
-template <bool FLEX>
-__global__ void __launch_bounds__(kMaxBlock) k_nodes_rigid(Dev d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  node_step<FLEX, true>(d, i, i < d.N);
-}
-
 // The rigid side of a substep: one warp per rigid of a stepping scene adds
 // its work items' reactions to its accumulators in work-item order (its
-// pairs in pair order, each pair's items in boundary-node order: lanes load
-// 128 records at a time, and every lane adds the hits in ascending lane order
-// through shuffles, so the sum is a serial run of the reference's atomic
-// adds).  Then each stepping scene's substep is counted and, on the substeps
-// of its schedule, its rigid update runs (fw_rigid.cuh): after a barrier, one
-// thread per scene, when all rigids fit in one block; otherwise by the warp
-// that finishes the scene's last rigid (a per-scene arrival count after a
-// fence).  The update reads only finished accumulators either way.
+// pairs in pair order, each gated pair's items in boundary-node order: lanes
+// load 256 records at a time, and every lane adds the hits in ascending lane
+// order through shuffles, so the sum is a serial run of the reference's atomic
+// adds).  The warp that finishes a scene's last rigid (a per-scene arrival count
+// after a fence) counts the substep and, on the substeps of its schedule, runs
+// the rigid update (fw_rigid.cuh), a lane per rigid.
 struct RigidDev {
   Rigid* rig;
   int n;
@@ -595,7 +609,7 @@ struct RigidDev {
   float4* item;
   int n_items;
   int* rp_off;   // per rigid: its pairs' item ranges rp_rng[rp_off[g] .. rp_off[g + 1])
-  int2* rp_rng;  // (first item, item count), pair order
+  int4* rp_rng;  // (first item, item count, pair), pair order
   fw::RigidScene* rs;  // the scenes with rigids
   int n_rs;
   int* done;           // per scene with rigids: warps finished this substep
@@ -604,70 +618,78 @@ struct RigidDev {
   int* err;
 };
 
-constexpr int kRigidThreads = 256;   // grid launch: 8 rigids per block
-constexpr int kRigidOneBlock = 1024;  // up to 32 rigids: one block, scenes updated after a barrier
-
-// The counter and, when due, the rigid update of scene-with-rigids k.
-__device__ __forceinline__ void rigid_scene_update(const RigidDev& r, int k) {
-  const fw::RigidScene rs = r.rs[k];
-  const fw::RigidClock ck = r.clock[rs.scene];
-  const int cnt = r.count[rs.scene] + 1;
-  r.count[rs.scene] = cnt;
-  if (ck.every < 1 || cnt % ck.every != 0) return;
-  fw::rigid_update(r.rig + rs.r0, rs.rn, r.gbox + rs.g0, r.gkind + rs.g0, rs.gn, ck.dt, ck.damping, r.err);
-}
-
-__global__ void __launch_bounds__(kRigidOneBlock) k_rigid(Dev d, RigidDev r) {
+// Warp g of the rigid side.
+__device__ __forceinline__ void rigid_step(const Dev& d, const RigidDev& r, int g) {
   const unsigned full = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31;
   const float4 none = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-  const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const bool live = g < r.n && d.scene_mode[r.rig[min(g, r.n - 1)].scene] == fw::MODE_STEP;
-  if (live) {
-    Rigid& rg = r.rig[g];
-    float ax = rg.acc[0], ay = rg.acc[1], aw = rg.accw;
-    for (int q = r.rp_off[g]; q < r.rp_off[g + 1]; ++q) {
-      const int2 rng = r.rp_rng[q];
-      for (int base = 0; base < rng.y; base += 128) {
-        float4 rec[4];
+  if (g >= r.n) return;
+  Rigid& rg = r.rig[g];
+  const int q0 = r.rp_off[g], q1 = r.rp_off[g + 1], k = rg.rs;
+  if (d.scene_mode[rg.scene] != fw::MODE_STEP) return;
+  float ax = rg.acc[0], ay = rg.acc[1], aw = rg.accw;
+  for (int q = q0; q < q1; ++q) {
+    const int4 rng = r.rp_rng[q];
+    if (!d.pair_active[rng.z]) continue;
+    for (int base = 0; base < rng.y; base += 256) {
+      float4 rec[8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int it = base + 32 * u + lane;
-          rec[u] = it < rng.y ? r.item[rng.x + it] : none;
-        }
+      for (int u = 0; u < 8; ++u) {
+        const int it = base + 32 * u + lane;
+        rec[u] = it < rng.y ? r.item[rng.x + it] : none;
+      }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          unsigned m = __ballot_sync(full, __float_as_int(rec[u].w) >= 0);
-          while (m) {
-            const int l = __ffs(m) - 1;
-            m &= m - 1;
-            ax = ax + __shfl_sync(full, rec[u].x, l);
-            ay = ay + __shfl_sync(full, rec[u].y, l);
-            aw = aw + __shfl_sync(full, rec[u].z, l);
-          }
+      for (int u = 0; u < 8; ++u) {
+        unsigned m = __ballot_sync(full, __float_as_int(rec[u].w) >= 0);
+        while (m) {
+          const int l = __ffs(m) - 1;
+          m &= m - 1;
+          ax = ax + __shfl_sync(full, rec[u].x, l);
+          ay = ay + __shfl_sync(full, rec[u].y, l);
+          aw = aw + __shfl_sync(full, rec[u].z, l);
         }
       }
     }
-    if (lane == 0) {
-      rg.acc[0] = ax;
-      rg.acc[1] = ay;
-      rg.accw = aw;
-    }
   }
-  if (gridDim.x == 1) {  // every rigid in this block: a barrier, then one thread per scene
-    __syncthreads();
-    for (int k = threadIdx.x; k < r.n_rs; k += blockDim.x)
-      if (d.scene_mode[r.rs[k].scene] == fw::MODE_STEP) rigid_scene_update(r, k);
+  const fw::RigidScene rs = r.rs[k];
+  const fw::RigidClock ck = r.clock[rs.scene];
+  int last = 0;
+  if (lane == 0) {
+    rg.acc[0] = ax;
+    rg.acc[1] = ay;
+    rg.accw = aw;
+    __threadfence();
+    last = atomicAdd(r.done + k, 1) + 1 == rs.rn;
+    __threadfence();
+  }
+  if (!__shfl_sync(full, last, 0)) return;
+  __threadfence();  // every lane reads the other warps' sums
+  const int cnt = __ldcg(r.count + rs.scene) + 1;
+  __syncwarp();
+  if (lane == 0) {
+    r.done[k] = 0;
+    r.count[rs.scene] = cnt;
+  }
+  if (ck.every < 1 || cnt % ck.every != 0) return;
+  fw::rigid_update(r.rig + rs.r0, rs.rn, r.gbox + rs.g0, r.gkind + rs.g0, rs.gn, ck.dt, ck.damping, r.err, lane);
+}
+
+// k_nodes of worlds with FEM-rigid contact (FLEX: FEM-FEM contact as well).
+// Blocks [0, rb) are the rigid side, a warp per rigid: the node step reads
+// nothing that it writes.
+// Bound by the latency of either side's chain.  A slab of 8192 triangles under
+// 12 rigids: 20.3 us a substep with the rigid side in a launch of its own (one
+// thread updating the rigids one after the other through global memory) and the
+// node step walking its pairs one by one, 10.2 us now; 640 triangles under one
+// rigid 11.1 and 7.5.
+template <bool FLEX>
+__global__ void __launch_bounds__(kMaxBlock) k_nodes_rigid(Dev d, RigidDev r, int rb) {
+  if ((int)blockIdx.x < rb) {
+    rigid_step(d, r, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
     return;
   }
-  // grid: the warp that finishes a scene's last rigid runs that scene's update
-  if (!live || lane != 0) return;
-  __threadfence();
-  const int k = r.rig[g].rs;
-  if (atomicAdd(r.done + k, 1) + 1 != r.rs[k].rn) return;
-  __threadfence();
-  r.done[k] = 0;
-  rigid_scene_update(r, k);
+  const int i = (blockIdx.x - rb) * blockDim.x + threadIdx.x;
+  node_step<FLEX, true>(d, i, i < d.N);
 }
 
 // Rotation cache and boxes of the rigids at construction
@@ -1527,23 +1549,19 @@ void flex_launch(fw_ctx* c, int force) {
 }
 
 // Kernel launches of one gather-path substep.
-int step_launches(const fw_ctx* c) { return (c->has_flex ? (c->has_rigid ? 4 : 3) : 2) + (c->has_rigid ? 1 : 0); }
+int step_launches(const fw_ctx* c) { return c->has_flex ? (c->has_rigid ? 4 : 3) : 2; }
 
 int launch_step(fw_ctx* c) {
   if (c->has_flex) flex_launch(c, 0);
   if (c->has_rigid) {
     // the element step plus one thread per FEM-rigid work item
     const int rb = std::max(1, std::min((c->d.n_ritems + c->block_e - 1) / c->block_e, c->sms * 8));
-    k_elements_rigid<<<c->grid_e + rb, c->block_e, 0, c->stream>>>(c->d, c->grid_e);
+    k_elements_rigid<<<1 + c->grid_e + rb, c->block_e, 0, c->stream>>>(c->d, c->grid_e);
+    const int wb = c->block_n / 32, gb = (c->rd.n + wb - 1) / wb;  // blocks of the rigid side
     if (c->has_flex)
-      k_nodes_rigid<true><<<c->grid_n, c->block_n, 0, c->stream>>>(c->d);
+      k_nodes_rigid<true><<<c->grid_n + gb, c->block_n, 0, c->stream>>>(c->d, c->rd, gb);
     else
-      k_nodes_rigid<false><<<c->grid_n, c->block_n, 0, c->stream>>>(c->d);
-    if (c->rd.n <= kRigidOneBlock / 32)
-      k_rigid<<<1, 32 * c->rd.n, 0, c->stream>>>(c->d, c->rd);
-    else
-      k_rigid<<<(c->rd.n + kRigidThreads / 32 - 1) / (kRigidThreads / 32), kRigidThreads, 0, c->stream>>>(c->d, c->rd);
-    c->launches += 1;
+      k_nodes_rigid<false><<<c->grid_n + gb, c->block_n, 0, c->stream>>>(c->d, c->rd, gb);
   } else if (c->has_flex) {
     k_nodes_flex<<<c->grid_n, c->block_n, 0, c->stream>>>(c->d);
   } else {
@@ -4176,10 +4194,10 @@ int fw_finalize(fw_ctx* c) {
     std::vector<int32_t> rp_off(nr + 1, 0);
     for (const Pair& p : rpairs) rp_off[p.table + 1]++;
     for (int g = 0; g < nr; ++g) rp_off[g + 1] += rp_off[g];
-    std::vector<int2> rp_rng(std::max(1, rp_off[nr]));
+    std::vector<int4> rp_rng(std::max(1, rp_off[nr]));
     {
       std::vector<int32_t> fill(rp_off.begin(), rp_off.end() - 1);
-      for (const Pair& p : rpairs) rp_rng[fill[p.table]++] = make_int2(p.n0, c->h_bncnt[p.body]);
+      for (const Pair& p : rpairs) rp_rng[fill[p.table]++] = make_int4(p.n0, c->h_bncnt[p.body], c->h_bncnt[p.body] ? rwork[p.n0].x : 0, 0);
     }
     // the scenes with rigids: their rigids and grounds, each a contiguous range
     std::vector<fw::RigidScene> rs;

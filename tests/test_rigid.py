@@ -380,3 +380,26 @@ def test_gpu_spring_rigid_equals_oracle():
         _compare(lp, o, o.N, f)
 
 
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 4, 5, 9, 33])
+def test_gpu_rows_of_rigids_equal_oracle(n):
+    """n rigids over one slab: one to nine blocks of the rigid side, fewer and
+    more rigids than a warp has lanes, pair loops of 2 to 34 pairs, and items in
+    more than one round of loads; every other rigid is too high to be gated on."""
+
+    def build():
+        conn, coords = fw.structured_rectangle(8 * n, 4, 0.08 * n, 0.1, origin=(0.0, 0.0))
+        slab = fw.FemDomain(fw.Mesh(2, conn, coords), fw.SolidProp(fw.HyperElastic(E=1e5, nu=0.3, rho=500.0)),
+                            [fw.Gravity([0.0, -9.8])])
+        rigids = [fw.RigidBodyDomain(fw.BallRigid(2, [0.04 + 0.08 * k, 0.1245 + 0.2 * (k % 2)], 0.025, 0.5),
+                                     [fw.EnforceVel([0], [0.01, -0.1 * (k % 2)])], friction=0.2) for k in range(n)]
+        return [fw.GroundDomain(2, [0.0, 0.0], [0.0, 1.0]), slab] + rigids
+
+    lp = fw.ExplicitLoop(0.0, build())
+    o = oracle.OracleLoop(build())
+    for k in (1, 7, 40, 200):
+        lp.advance_n(k)
+        o.advance(k)
+        _compare(lp, o, o.N, k)
