@@ -75,6 +75,7 @@
 namespace {
 
 constexpr int kCluMaxCtas = 16;
+constexpr int kCluOneThreads = 640;  // grid form: most threads with a thread per triangle (clu_threads)
 constexpr int kCluMaxBodies = 8;   // per scene
 constexpr int kCluMaxPairs = 32;   // per scene
 constexpr int kCluMaxThreads = 1024;
@@ -1104,7 +1105,7 @@ using CluKernel = void (*)(const Dev, const CluLaunch, const float2*, float2*, c
 inline CluKernel clu_kernel(int threads, int one, int grid, int tri_l2 = 0) {
   if (grid) {
     if (tri_l2) return k_cluster<1024, false, true, true>;
-    if (one) return threads <= 512 ? k_cluster<512, true, true> : k_cluster<1024, true, true>;
+    if (one) return threads <= 512 ? k_cluster<512, true, true> : k_cluster<kCluOneThreads, true, true>;
     return threads <= 640 ? k_cluster<640, false, true> : k_cluster<1024, false, true>;
   }
   if (one) return threads <= 512 ? k_cluster<512, true, false> : k_cluster<1024, true, false>;

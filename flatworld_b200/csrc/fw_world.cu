@@ -2143,6 +2143,11 @@ size_t clu_smem(CluLaunch r) { return clu_layout(r); }
 // Threads of a CTA, control warps included: a control warp for the boxes and
 // one per 64 boundary nodes for their contact forces, at most 4; and a thread
 // per triangle where that fits a CTA (r.one), else an equal share of them.
+// One scene on the whole GPU: two triangles per thread as soon as a thread each
+// would leave it less than the 96 registers the substep needs (640 threads).
+// 64 substeps of 36,000 to 58,000 nodes, one / two per thread: 2.95 / 2.73,
+// 3.13 / 2.88, 3.16 / 2.90, 3.21 / 2.98, 3.30 / 3.08 us per substep; of 32,000
+// nodes (576 threads) 2.27 / 2.69.
 // Where the scenes fill the GPU (`shared`), two triangles per thread: 384
 // bodies of 60 to 400 nodes ran 5.06 / 4.08 / 4.53 / 4.83 us per substep at
 // 1 / 2 / 3 / 4, 256 of 100 to 20000 nodes 33.5 / 33.4 / 33.3 / 36.3.
@@ -2150,7 +2155,7 @@ int clu_threads(CluLaunch& r, bool shared) {
   r.ctl = r.np ? std::min(4, 1 + (r.nbnd + 63) / 64) : 1;
   const int most = kCluMaxThreads - 32 * r.ctl, work = std::max(1, std::max(r.ne, r.no));
   int rounds = (work + most - 1) / most;
-  if (shared && r.ne >= 128) rounds = std::max(rounds, 2);
+  if ((shared && r.ne >= 128) || (r.grid && work + 32 * r.ctl > kCluOneThreads)) rounds = std::max(rounds, 2);
   r.one = rounds == 1 ? 1 : 0;
   return (((work + rounds - 1) / rounds + 31) / 32 + r.ctl) * 32;
 }

@@ -51,6 +51,8 @@ SINGLE = {
     "one patch": lambda: _rectangle(3, 2, MATS["elastic"], _plane()),
     "two patches": lambda: _rectangle(15, 8, MATS["neohookean"], _plane()),
     "a thread per triangle, J2": lambda: _rectangle(60, 31, MATS["mises"], _plane()),
+    "a thread per triangle, 640 threads": lambda: _rectangle(200, 160, MATS["neohookean"], _plane(), cell=0.005),
+    "two triangles per thread": lambda: _rectangle(200, 200, MATS["mises"], _plane(), cell=0.005),
     "several triangles per thread": lambda: _rectangle(260, 251, MATS["neohookean"], _plane(), cell=0.004),
     "records in L2": lambda: _rectangle(640, 500, MATS["neohookean"], _plane(-0.0005), cell=0.002),
     "records in L2, J2": lambda: _rectangle(520, 440, MATS["mises"], _plane(-0.0005), cell=0.002),
