@@ -139,7 +139,10 @@ class BatchedLoop:
         fewer substeps are frozen while the others finish."""
         runs = [substep_schedule(frame_dt, lay.stableTime, lay.default_dt, lay.useAdapative)
                 for lay in self.layouts]
-        if (self.path == "stream" and max(len(r) for r in runs) <= _native.FW_MAX_RUNS
+        # one short run that all scenes share is left to the step calls, which
+        # choose between the on-chip and the stream kernels by its length
+        short = all(r == runs[0] for r in runs) and sum(n for n, _ in runs[0]) < 8
+        if (self.path == "stream" and max(len(r) for r in runs) <= _native.FW_MAX_RUNS and not short
                 and self._native.get_option(_native.FW_OPT_CLUSTER) == 1):
             return self._advance_runs(runs)
         pos = [0] * self.S      # index into each scene's run list

@@ -45,9 +45,21 @@ namespace {
 constexpr int kBlock = 256;     // default block size of the gather kernels
 constexpr int kMaxBlock = 512;  // launch bound (block sizes are a runtime option)
 constexpr int kGraphSteps = 32;
-constexpr int kCluServedNodes = 256;  // nodes of a served scene's cluster patch: latency before throughput
+// Nodes of a served scene's cluster patch: latency before throughput, up to a
+// point.  128 / 256 / 512: 48 requests of 100 to 4000 nodes 3.44 / 3.13 / 2.92 ms,
+// 8 such 1.33 / 1.42 / 1.72, 16 of 100 to 1000 nodes 1.49 / 1.69 / 1.76.
+constexpr int kCluServedNodes = 256;
 constexpr size_t kCluSharedBytes = 232448 - 64;  // of a CTA on sm_100
-constexpr int kCluMinSteps = 3;  // substeps of a call from which a stream world's scenes are stepped on chip
+
+// Substeps of a call from which a stream world's scenes are stepped on chip: a
+// patch is loaded and written once per call, which costs as much as that many
+// substeps gain, and gain less the more patches share an SM.  One call of ragged
+// bodies, on chip / stream kernels, us: 109,000 triangles 3 substeps 43 / 53;
+// 517,000 4: 99 / 94, 5: 110 / 113; 959,000 5: 175 / 177; 1,732,000 6: 340 / 332,
+// 8: 399 / 437; 3,674,000 6: 678 / 622, 8: 801 / 824.
+int clu_min_steps(int sms, int64_t triangles) {
+  return triangles <= (int64_t)sms * 1500 ? 3 : triangles <= (int64_t)sms * 6500 ? 5 : 8;
+}
 
 struct Dev {
   float2* x;
@@ -1337,6 +1349,7 @@ struct fw_ctx {
   unsigned char* d_cblob = nullptr;
   CluScene* d_cscene = nullptr;  // the scenes of a call, in launch order
   bool clu_size_ok[kCluMaxCtas + 1] = {};  // cluster sizes the device can hold
+  bool arena_clu = true;                   // the arena's lists leave out the scenes that are stepped on chip
   size_t clu_cap = 0;
   int32_t* d_plist = nullptr;     // the active scenes' patches (CTA -> patch)
   int32_t* d_budget = nullptr;    // fw_step_served_budget: per-scene substep budgets
@@ -1696,9 +1709,7 @@ StreamKernel stream_kernel(int nodes, int minb, int bulk) {
 // (starting buffer, dt mode, dt, count).
 int stream_steps(fw_ctx* c, int n) {
   c->host_counter += n;
-  // a patch is loaded once per call: one or two substeps cost a batch less on
-  // the stream kernels (256 ragged bodies, one substep: 88 / 190 us)
-  const bool clu = !c->clu.empty() && n >= kCluMinSteps;
+  const bool clu = !c->clu.empty() && n >= clu_min_steps(c->sms, c->E);
   StreamDev sd = c->sd;
   if (!clu) sd.list = nullptr;
   if (clu) {
@@ -3078,12 +3089,20 @@ int arena_cluster_steps(fw_ctx* c, int n) {
 // n substeps of a stream arena: k_control + k_stream over the active scenes'
 // patches each, then (n odd) the carry back into the first buffers.
 int arena_stream_steps(fw_ctx* c, int n) {
+  int64_t tris = 0;
+  for (size_t s = 0; n < 8 && s < c->ascenes.size(); ++s)
+    if (c->ascenes[s].live && c->cur_active[s]) tris += c->ascenes[s].ne;
+  const bool clu = c->clu_opt && c->d_cpatch && n >= clu_min_steps(c->sms, tris);
+  if (clu != c->arena_clu) {  // the lists hold what is not stepped on chip
+    c->arena_clu = clu;
+    c->chunks_dirty = true;
+  }
   if (c->chunks_dirty) {
     c->h_plist.clear();
     c->h_slist.clear();
     for (size_t s2 = 0; s2 < c->ascenes.size(); ++s2) {
       const fw_ctx::ArenaScene& a = c->ascenes[s2];
-      if (!a.live || !c->cur_active[s2] || (c->clu_opt && a.clu.ctas)) continue;
+      if (!a.live || !c->cur_active[s2] || (clu && a.clu.ctas)) continue;
       c->h_slist.push_back((int32_t)s2);
       for (int64_t k = 0; k < a.npp; ++k) c->h_plist.push_back((int32_t)(a.pp0 + k));
     }
@@ -3100,7 +3119,7 @@ int arena_stream_steps(fw_ctx* c, int n) {
   }
   c->host_counter += n;
   if (n <= 0) return FW_OK;
-  if (c->clu_opt && c->d_cpatch)
+  if (clu)
     if (int rc = arena_cluster_steps(c, n)) return rc;
   if (c->st_list_n == 0) return FW_OK;
   float2 *xa = c->d.x, *xb = c->d.x_alt;

@@ -150,6 +150,20 @@ def test_batch_bitwise(sizes, covered):
     _same(a, b)
 
 
+@pytest.mark.parametrize("bodies", [4, 34])
+def test_short_calls_equal_the_stream_kernels(bodies):
+    """Calls on both sides of the length from which a batch is stepped on chip, below and above 1500 triangles per SM."""
+    a = BatchedLoop(_batch([(60, 58)] * bodies), dt=5e-5, useAdapativeDT=False)
+    b = BatchedLoop(_batch([(60, 58)] * bodies), dt=5e-5, useAdapativeDT=False, stream_patch=64)
+    for lp in (a, b):
+        lp._packed = lp.packed
+        for n in (1, 2, 3, 4, 5, 1, 8, 2):
+            lp.advance(n)
+        lp.advanceWithTime(2e-4)
+        lp.advanceWithTime(1e-3)
+    _same(a, b)
+
+
 def test_wait_runs_out_and_the_context_recovers():
     lp = fw.ExplicitLoop(0.0, SINGLE["two patches"]())
     lp.advance_n(20)
