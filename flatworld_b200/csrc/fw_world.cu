@@ -61,6 +61,17 @@ int clu_min_steps(int sms, int64_t triangles) {
   return triangles <= (int64_t)sms * 1500 ? 3 : triangles <= (int64_t)sms * 6500 ? 5 : 8;
 }
 
+// The same for a single scene, whose shorter calls run on the gather kernels:
+// one substep is two plain launches, 5 to 10 us less than a cooperative one and
+// the patches' loads; more of them, as a graph, only where a mesh is so large
+// that the loads take as long as the gather kernels' substeps.  A call and its
+// synchronisation, on chip / gather, us: up to 131072 triangles 1 substep 31 /
+// 25, 2: 31 / 33; 537600 2: 49 / 43, 3: 55 / 62; 655360 2: 54 / 51, 3: 64 / 65,
+// 4: 73 / 87; 798000 3: 79 / 75, 4: 88 / 92.
+int grid_min_steps(int sms, int64_t triangles) {
+  return triangles <= (int64_t)sms * 2500 ? 2 : triangles <= (int64_t)sms * 4000 ? 3 : 4;
+}
+
 struct Dev {
   float2* x;
   float2* x_alt;       // stream path: the other position buffer (swapped every substep)
@@ -1662,7 +1673,8 @@ int run_steps(fw_ctx* c, int n) {
   int rc = FW_OK;
   if (c->arena && c->a_stream) return arena_stream_steps(c, n);
   if (c->arena && (rc = rebuild_chunks(c))) return rc;
-  if (c->path == FW_PATH_RESIDENT && c->d.uniform_dt) return launch_resident(c, n);
+  if (c->path == FW_PATH_RESIDENT && c->d.uniform_dt && (c->clu.empty() || n >= grid_min_steps(c->sms, c->E)))
+    return launch_resident(c, n);
   if (c->path == FW_PATH_STREAM) return stream_steps(c, n);
   c->host_counter += n;
   if (n >= kGraphSteps) {
@@ -5305,8 +5317,9 @@ int fw_set_active(fw_ctx* c, const int32_t* active) {
 
 int fw_synchronize(fw_ctx* c) {
   if (!c) return FW_ERR_ARG;
+  if (c->finalized && raises_flags(c)) return check_device_error(c);  // which waits: one trip
   FW_CUDA(c, cudaStreamSynchronize(c->stream));
-  return c->finalized ? check_device_error(c) : FW_OK;
+  return FW_OK;
 }
 
 int fw_read_nodes(fw_ctx* c, int32_t field, int32_t first, int32_t count, float* dst, int32_t on_device) {

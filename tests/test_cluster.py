@@ -150,6 +150,17 @@ def test_batch_bitwise(sizes, covered):
     _same(a, b)
 
 
+@pytest.mark.parametrize("n", [20, 530])
+def test_short_calls_of_one_scene_equal_the_gather_kernels(n):
+    """Calls on both sides of the length from which a scene is stepped on chip, small and above 2500 triangles per SM."""
+    a, b = (fw.ExplicitLoop(0.0, _rectangle(n, 380, MATS["neohookean"], _plane(-0.0005), cell=0.002), path=p)
+            for p in ("auto", "gather"))
+    for lp in (a, b):
+        for k in (1, 2, 3, 1, 4, 5, 2, 1, 9, 3):
+            lp.advance_n(k)
+    _same(a, b)
+
+
 @pytest.mark.parametrize("bodies", [4, 34])
 def test_short_calls_equal_the_stream_kernels(bodies):
     """Calls on both sides of the length from which a batch is stepped on chip, below and above 1500 triangles per SM."""
