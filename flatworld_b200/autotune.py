@@ -71,9 +71,18 @@ STREAM_MINB = {64: (32, 24, 20, 16), 128: (16, 12, 10, 8)}  # register budgets b
 def tune_stream(loop, steps=16, use_cache=True):
     """Pick the stream step's register budget (CTAs per SM) and record staging
     (bulk copy or per-thread loads) for ``loop`` (a BatchedLoop on the stream
-    path), timed on the loop's own world from a snapshot, as tune_batched."""
+    path), timed on the loop's own world from a snapshot, as tune_batched.
+
+    A loop whose scenes are all stepped on chip keeps that: setting a shape of
+    the stream kernels would give it up (2048 ragged bodies, 100 substeps in a
+    call: 290 us per substep on chip, 418 on the best stream shape)."""
     import torch
 
+    from . import _native
+
+    if loop._native.get_option(_native.FW_OPT_CLUSTER) == 1:
+        return {"path": "stream", "patch": loop.stream_patch, "minb": loop.stream_minb, "bulk": bool(loop.stream_bulk),
+                "on_chip": True, "candidates": []}
     key = (f"stream|{_gpu_name(loop._native.device)}|N={loop.n_nodes}|E={loop.n_elems}|S={loop.S}"
            f"|patch={loop.stream_patch}")
     if use_cache:

@@ -175,6 +175,17 @@ def test_short_calls_equal_the_stream_kernels(bodies):
     _same(a, b)
 
 
+@pytest.mark.parametrize("patch,on_chip", [(0, 1), (64, 0)])
+def test_tuning_keeps_the_on_chip_step(patch, on_chip, tmp_path, monkeypatch):
+    from flatworld_b200 import autotune
+
+    monkeypatch.setenv("FLATWORLD_B200_CACHE", str(tmp_path))
+    lp = BatchedLoop(_batch([(20, 9), (7, 30)]), dt=5e-5, useAdapativeDT=False, stream_patch=patch)
+    best = autotune.tune_batched(lp, steps=4)
+    assert best["path"] == "stream" and best["minb"] > 0 and bool(best.get("on_chip")) == bool(on_chip)
+    assert lp._native.get_option(_native.FW_OPT_CLUSTER) == on_chip
+
+
 def test_wait_runs_out_and_the_context_recovers():
     lp = fw.ExplicitLoop(0.0, SINGLE["two patches"]())
     lp.advance_n(20)
