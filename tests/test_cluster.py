@@ -242,6 +242,42 @@ def test_voxel_contact_matches_the_oracle(nx, ny, kind):
         assert np.array_equal(lp.femSpringManager.V.numpy()[:n].astype(np.float64), v)
 
 
+def _long_terrain_scene(nx, ny, at):
+    """A block lying in a long solid grid with its middle at cell ``at`` of the long side."""
+    along = nx > ny
+    cell = (0.001, 0.02) if along else (0.02, 0.001)
+    vox = fw.VoxelGridDomain(2, nx, ny, np.float32([0.0, 0.0]), np.float32([nx * cell[0], ny * cell[1]]),
+                             occupancy_np=np.ones((nx, ny), np.int32))
+    origin = (at * 0.001 - 0.05, ny * 0.02 - 0.01) if along else (nx * 0.02 - 0.01, at * 0.001 - 0.05)
+    conn, coords = fw.structured_rectangle(10, 10, 0.1, 0.1, origin=origin, jitter=0.1, seed=3)
+    return [vox, fw.FemDomain(fw.Mesh(2, conn, coords), fw.SolidProp(MATS["elastic"]), [fw.Gravity([0.0, -9.8])])]
+
+
+@pytest.mark.parametrize("nx,ny", [(65535, 4), (65536, 4), (70000, 4), (4, 65535), (2, 70000)])
+@pytest.mark.parametrize("at", [65400, 65535])
+def test_voxel_contact_on_long_grids(nx, ny, at):
+    """Sides on both sides of the cell table's 16 bits; nodes on both sides of cell 65535."""
+    import oracle
+
+    def build():
+        return _long_terrain_scene(nx, ny, at)
+
+    o = oracle.OracleLoop(build(), 0.0, useAdapativeDT=True, threads=4)
+    loops = [fw.ExplicitLoop(0.0, build(), path=p) for p in ("auto", "gather")]
+    loops.append(fw.ExplicitLoop(0.0, build(), front_warps=6))
+    batch = BatchedLoop([build(), build()], dt=loops[0].dt, useAdapativeDT=False, stream_patch=64)
+    o.advance(10)
+    x, v, _ = o.state()
+    assert np.abs(v).max() > 2 * 9.8 * 10 * loops[0].dt  # pushed out: faster than a free fall
+    for lp in loops:
+        lp.advance_n(10)
+        n = lp._packed.N
+        assert np.array_equal(lp.femSpringManager.coords.numpy()[:n].astype(np.float64), x)
+        assert np.array_equal(lp.femSpringManager.V.numpy()[:n].astype(np.float64), v)
+    batch.advance(10)
+    assert np.array_equal(batch.coords(1).astype(np.float64), x)
+
+
 @pytest.mark.parametrize("n,ground", [(3, "plane"), (16, "plane"), (41, "bump"), (70, "bump"), (150, "plane")])
 def test_reverse_pass_matches_the_gather_reverse(n, ground):
     """One patch, several, and meshes whose patches hold more than 512 triangles; contact on."""
