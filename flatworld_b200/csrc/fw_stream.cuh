@@ -56,8 +56,8 @@ struct StreamPatch {
 // Static data of one patch triangle, in patch order (32 B: what the triangle
 // step reads, in one record).  Its Lame constants come from its body's entry
 // of Dev::body_lm -- a body's triangles share one material -- unless
-// StreamDev::lm holds them per triangle (after a per-element Young's modulus
-// change); its global index, needed by J2 triangles only, is StreamDev::eid
+// StreamDev::lm holds them per triangle (a body whose triangles have different
+// moduli, at construction or after a per-element Young's modulus change); its global index, needed by J2 triangles only, is StreamDev::eid
 // at the same position.
 struct __align__(16) StreamElem {
   float area;  // emat[e].area
@@ -86,7 +86,7 @@ struct StreamDev {
   StreamNode* node;  // built from nodes by k_stream_nodes
   int* err;          // != 0: a staged copy did not complete in time
   const int32_t* list;  // arena worlds: CTA i runs patch list[i] (the active scenes' patches); else patch i
-  float2* lm;           // per patch triangle (lam, mu) once a triangle's Young's modulus was set; else null
+  float2* lm;           // per patch triangle (lam, mu) where a body's triangles may differ; else null
 };
 
 __global__ void k_stream_nodes(Dev d, const int32_t* nodes, StreamNode* out, int n) {

@@ -1356,6 +1356,7 @@ struct fw_ctx {
   // scene's node range and corner lists its 3 x triangle range
   bool a_stream = false;
   FreeList fl_patch, fl_halo, fl_ptri, fl_csrp, fl_cpatch, fl_cblob;
+  int64_t st_ptri_cap = 0;  // patch triangles the arena holds
   CluPatch* d_cpatch = nullptr;
   unsigned char* d_cblob = nullptr;
   CluScene* d_cscene = nullptr;  // the scenes of a call, in launch order
@@ -1779,6 +1780,17 @@ int stream_steps(fw_ctx* c, int n) {
 void rcb(const std::vector<float2>& x, std::vector<int>& idx, int lo, int hi, int p0, int np,
          std::vector<int>& part);
 
+// Triangles of one body with different moduli (FemDomain.elementYoung): the
+// stream records then keep Lame constants per triangle, not per body.
+bool mixed_moduli(const fw_ctx* c) {
+  for (size_t b = 0; b < c->h_noff.size(); ++b) {
+    const int e0 = c->h_eoff[b];
+    for (int e = e0 + 1; e < e0 + c->h_ecnt[b]; ++e)
+      if (c->h_E[e] != c->h_E[e0] || c->h_nu[e] != c->h_nu[e0]) return true;
+  }
+  return false;
+}
+
 // (Re)build the patch-ordered records of the stream path from the element and
 // node arrays (after finalize, and after a Young's modulus changes).
 int stream_records(fw_ctx* c) {
@@ -1957,6 +1969,7 @@ int build_stream(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<i
   c->sd = StreamDev{dp, dn, dh, de, dc, dcp, dcs, no_max, nh_max, ne_max, dse, dsn, c->d_flags + fw_ctx::kFlagStream};
   c->st_ne = (int)re.size();
   c->st_no = (int)rn.size();
+  if (mixed_moduli(c) && (r = dalloc(c, &c->sd.lm, (size_t)std::max(1, c->st_ne)))) return r;
   if ((r = stream_records(c))) return r;
   c->st_P = P;
   c->st_smem = sizeof(float2) * (size_t)(no_max + nh_max) + sizeof(float2) * 3 * (size_t)ne_max;
@@ -2518,6 +2531,7 @@ int cluster_per_tri(fw_ctx* c) {
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
   for (fw_ctx::CluGroup& g : c->clu) {
     if (g.r.per_tri) continue;
+    drop_graphs(c);  // they hold the carve-up
     g.r.per_tri = 1;
     g.smem = clu_layout(g.r);
     if (g.smem + kCluStatic > (size_t)optin || !clu_fits(g.r, g.threads, g.smem)) return cluster_off(c);
@@ -3179,6 +3193,7 @@ struct fw_pack {
   int64_t Ps = 0, Hs = 0, Ts = 0, CPs = 0;  // stream records (patch_nodes > 0)
   int patch_nodes = 0;
   int no_max = 0, nh_max = 0, ne_max = 0;
+  bool mixed = false;  // a body's triangles have different moduli
   CluLaunch clu{};  // cluster size and maxima of its cluster patches (ctas 0: none)
   float damp = 0.f;
   unsigned char* block = nullptr;
@@ -3327,6 +3342,7 @@ int build_pack(fw_ctx* c, int patch_nodes, bool pinned, fw_pack** out) {
   }
   fw_pack* pk = new fw_pack();
   pk->clu = clu;
+  pk->mixed = mixed_moduli(c);
   pk->Ns = Ns; pk->Es = Es; pk->Bs = Bs; pk->Np = (int64_t)pairs.size();
   pk->Nh = (int64_t)c->h_heights.size(); pk->No = (int64_t)c->h_occ.size();
   pk->damp = c->h_damp.empty() ? 0.f : c->h_damp[0];
@@ -4628,6 +4644,7 @@ int fw_arena_init(fw_ctx* c, int64_t max_nodes, int64_t max_elems, int32_t max_b
     c->fl_patch.init(Pcap);
     c->fl_halo.init(Hcap);
     c->fl_ptri.init(Tcap);
+    c->st_ptri_cap = Tcap;
     c->fl_csrp.init(CPcap);
     if (c->clu_opt) {
       const int64_t Qcap = N / kCluServedNodes * 2 + 16 * (int64_t)S, Bcap = 24 * N + 32 * E + 256 * Qcap;
@@ -4673,6 +4690,19 @@ int fw_arena_commit_pack(fw_ctx* c, const fw_pack* pk, int32_t* scene_out) {
     return fail(c, FW_ERR_ARG, "fw_arena_commit_pack: the pack is cut into %d-node patches, the arena steps %d-node "
                                "patches", pk->patch_nodes, c->st_nodes);
   if (c->free_scene_ids.empty()) return fail(c, FW_ERR_OOM, "arena: no free scene slot");
+  if (c->a_stream && pk->mixed && !c->sd.lm) {
+    // the first such scene: Lame constants per triangle from here on, for the resident scenes as well
+    float2* lm = nullptr;
+    if (int rl = dalloc(c, &lm, (size_t)c->st_ptri_cap)) return rl;
+    c->sd.lm = lm;
+    for (const fw_ctx::ArenaScene& o : c->ascenes)
+      if (o.live && o.nt > 0) {
+        k_stream_elems<<<(int)((o.nt + kBlock - 1) / kBlock), kBlock, 0, c->stream>>>(
+            c->d, c->sd.eid + o.t0, c->sd.conn + o.t0, c->sd.elem + o.t0, lm + o.t0, (int)o.nt);
+        c->launches += 1;
+      }
+    if (int rk = check_kernel(c, "arena records")) return rk;
+  }
   fw_ctx::ArenaScene a;
   a.nn = pk->Ns; a.ne = pk->Es; a.nb = pk->Bs; a.np = pk->Np; a.nh = pk->Nh; a.no = pk->No;
   if (c->a_stream) { a.npp = pk->Ps; a.nhh = pk->Hs; a.nt = pk->Ts; a.ncp = pk->CPs; }
@@ -4789,7 +4819,7 @@ int fw_arena_commit_pack(fw_ctx* c, const fw_pack* pk, int32_t* scene_out) {
   if (c->a_stream) {
     if (a.nt > 0)
       k_stream_elems<<<(int)((a.nt + kBlock - 1) / kBlock), kBlock, 0, c->stream>>>(
-          d, c->sd.eid + a.t0, c->sd.conn + a.t0, c->sd.elem + a.t0, nullptr, (int)a.nt);
+          d, c->sd.eid + a.t0, c->sd.conn + a.t0, c->sd.elem + a.t0, c->sd.lm ? c->sd.lm + a.t0 : nullptr, (int)a.nt);
     k_stream_nodes<<<(int)((a.nn + kBlock - 1) / kBlock), kBlock, 0, c->stream>>>(d, c->sd.nodes + n0,
                                                                                   c->sd.node + n0, (int)a.nn);
     c->launches += 2;

@@ -114,6 +114,61 @@ def test_moduli_per_triangle_and_set_later():
     _same(u, v)
 
 
+def _graded(nx, ny):
+    """A body whose triangles each have their own Young's modulus."""
+    doms = _rectangle(nx, ny, MATS["neohookean"], _plane(), cell=0.01)
+    doms[1].elementYoung = np.linspace(2e4, 8e4, doms[1].nelements).astype(np.float32)
+    return doms
+
+
+@pytest.mark.parametrize("sizes,covered", [([(9, 9), (30, 20), (60, 40)], 1), ([(9, 9), (200, 160), (30, 20)], 2)],
+                         ids=["on chip", "one too large"])
+def test_moduli_per_triangle_in_batches(sizes, covered):
+    """The same bits however the substeps are cut into calls: the on-chip, the stream and the gather kernels."""
+    def build(**kw):
+        return BatchedLoop([_graded(*size) for size in sizes] + _batch([(12, 7)]), dt=5e-5, useAdapativeDT=False, **kw)
+
+    a, b, c, d = build(), build(), build(stream_patch=64), build(path="gather")
+    assert a._native.get_option(_native.FW_OPT_CLUSTER) == covered
+    for lp in (a, b, c, d):
+        lp._packed = lp.packed
+    for _ in range(24):
+        b.advance(1)
+    for lp in (a, c, d):
+        lp.advance(24)
+    for lp in (b, c, d):
+        _same(a, lp)
+    for lp in (a, c, d):  # and changed later, with the batch's graphs made
+        lp.advance(24)
+        lp._native.set_element_young(np.linspace(8e4, 2e4, lp.packed.E).astype(np.float32))
+        lp.advance(24)
+    for lp in (c, d):
+        _same(a, lp)
+
+
+def test_moduli_per_triangle_in_arenas():
+    from flatworld_b200.serve import Arena
+
+    ar = Arena(60_000, 120_000, 16, 16, 64, 1 << 16, 1 << 16)
+    build = [lambda: _batch([(12, 7)])[0], lambda: _graded(30, 20), lambda: _graded(200, 160), lambda: _graded(9, 9)]
+    dt = np.float32(5e-5)
+    ran, sc = [], []
+    for b in build:  # the first scene is resident before one with several moduli comes
+        sc.append(ar.insert(b()))
+        ran.append(0)
+        for n in (1, 1, 1, 9, 2):
+            ar.native.step_served_n(np.where(np.isin(np.arange(ar.S), sc), dt, np.float32(0.0)), n)
+            ran = [r + n for r in ran]
+    ar.native.synchronize()
+    for s, b, n in zip(sc, build, ran):
+        lp = fw.ExplicitLoop(5e-5, b(), useAdapativeDT=False, path="gather")
+        lp.advance_n(n - 1)  # the first substep of a committed scene is its construction step
+        nn = lp._packed.N
+        assert np.array_equal(ar.coords(s), lp.femSpringManager.coords.numpy()[:nn])
+        assert np.array_equal(ar.velocities(s), lp.femSpringManager.V.numpy()[:nn])
+    ar.close()
+
+
 def _batch(sizes):
     out = []
     for k, (nx, ny) in enumerate(sizes):
