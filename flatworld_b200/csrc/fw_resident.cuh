@@ -523,8 +523,9 @@ k_resident(Dev d, Res r, int step0, int nsteps, float dt, float damp, uint32_t e
           const int leader = __ffs(mb) - 1;
           const int bl = __shfl_sync(full, body, leader);
           const bool uniform = __all_sync(full, !bnd || body == bl);
-          float lx = bnd ? x.x : 1e30f, ly = bnd ? x.y : 1e30f;
-          float hx = bnd ? x.x : -1e30f, hy = bnd ? x.y : -1e30f;
+          const bool okx = bnd && x.x == x.x, oky = bnd && x.y == x.y;  // NaN widens no box
+          float lx = okx ? x.x : 1e30f, ly = oky ? x.y : 1e30f;
+          float hx = okx ? x.x : -1e30f, hy = oky ? x.y : -1e30f;
           if (uniform) {
             for (int o = 16; o > 0; o >>= 1) {
               lx = fminf(lx, __shfl_xor_sync(full, lx, o));

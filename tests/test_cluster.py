@@ -241,6 +241,25 @@ def test_tuning_keeps_the_on_chip_step(patch, on_chip, tmp_path, monkeypatch):
     assert lp._native.get_option(_native.FW_OPT_CLUSTER) == on_chip
 
 
+@pytest.mark.parametrize("build,bad", [
+    (lambda: _rectangle(20, 100, MATS["neohookean"], _plane(0.005)), range(32, 64)),
+    (lambda: scenes.multi_block_scene(fw, 2), [121]),
+], ids=["a warp of boundary nodes", "a warp of two bodies"])
+def test_nan_nodes_leave_the_contact_of_the_others(build, bad):
+    """Nodes that are NaN widen no box: the others' gates are the same on every path."""
+    loops = [fw.ExplicitLoop(2e-5, build(), useAdapativeDT=False, path=p) for p in ("auto", "gather")]
+    loops.append(fw.ExplicitLoop(2e-5, build(), useAdapativeDT=False, front_warps=6))
+    loops += [BatchedLoop([build()], dt=2e-5, useAdapativeDT=False, **kw) for kw in ({}, {"stream_patch": 64})]
+    for lp in loops:
+        lp._packed = lp.packed if isinstance(lp, BatchedLoop) else lp._packed
+        x = lp._native.read_nodes(_native.FW_FIELD_X, 0, lp._packed.N)
+        x[list(bad)] = np.nan
+        lp._native.write_nodes(_native.FW_FIELD_X, 0, x)
+        (lp.advance if isinstance(lp, BatchedLoop) else lp.advance_n)(8)
+    for lp in loops[1:]:
+        _same(loops[0], lp)
+
+
 def test_wait_runs_out_and_the_context_recovers():
     lp = fw.ExplicitLoop(0.0, SINGLE["two patches"]())
     lp.advance_n(20)
