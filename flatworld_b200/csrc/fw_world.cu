@@ -27,6 +27,8 @@
 #include <mutex>
 #include <cstdio>
 #include <cstring>
+#include <exception>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -2013,20 +2015,50 @@ void rcb(const std::vector<float2>& x, std::vector<int>& idx, int lo, int hi, in
 
 // ------------------------------------------------------------------ cluster-resident scenes
 
-// f(k) for k in [0, n) on up to `threads` host threads (this one among them).
+// f(k) for k in [0, n) on up to `threads` host threads (this one among them; on
+// fewer where no more can be made).  What f throws is thrown here, once all
+// threads have ended.
 template <class F>
 void parallel_for(int n, int threads, F f) {
   std::atomic<int> next{0};
+  std::exception_ptr thrown;
+  std::mutex lock;
   auto work = [&] {
-    for (int k; (k = next.fetch_add(1)) < n;) f(k);
+    try {
+      for (int k; (k = next.fetch_add(1)) < n;) f(k);
+    } catch (...) {
+      std::lock_guard<std::mutex> hold(lock);
+      if (!thrown) thrown = std::current_exception();
+      next = n;
+    }
   };
   std::vector<std::thread> pool;
-  for (int k = 1; k < std::min(n, threads); ++k) pool.emplace_back(work);
+  try {
+    for (int k = 1; k < std::min(n, threads); ++k) pool.emplace_back(work);
+  } catch (const std::exception&) {  // the threads there are take the rest
+  }
   work();
   for (std::thread& th : pool) th.join();
+  if (thrown) std::rethrow_exception(thrown);
 }
 
-int host_threads() { return (int)std::min(16u, std::max(1u, std::thread::hardware_concurrency())); }
+// Threads for host work on so many nodes: a few thousand nodes are cut faster
+// than a thread starts.
+int host_threads(int64_t nodes) {
+  return (int)std::min<int64_t>({16, std::max(1u, std::thread::hardware_concurrency()), 1 + nodes / 4096});
+}
+
+// A C entry's work, with what the C++ library throws as an error code.
+template <class F>
+int guarded(fw_ctx* c, F f) {
+  try {
+    return f();
+  } catch (const std::bad_alloc&) {
+    return fail(c, FW_ERR_OOM, "out of host memory");
+  } catch (const std::exception& e) {
+    return fail(c, FW_ERR_STATE, "%s", e.what());
+  }
+}
 
 // One scene's patches for `ctas` CTAs into out / blob (ids relative to the
 // scene; byte offsets relative to blob).  Returns false when the scene does not
@@ -2345,7 +2377,7 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
     std::vector<unsigned char> blob;
   };
   std::vector<Cut> cuts(S);
-  parallel_for(S, host_threads(), [&](int s) {
+  parallel_for(S, host_threads(c->N), [&](int s) {
     if (!ok[s]) return;
     const int most = single ? sms : kCluMaxCtas;
     int ctas = single ? std::min(sms, (nn[s] + want_nodes - 1) / want_nodes) : 1;
@@ -2358,7 +2390,7 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
       Cut& k = cuts[s];
       k.patches.clear();
       k.blob.clear();
-      if (!make_cluster_patches(c, scenes[s], nn[s], off, slot, x0, word, ctas, part, S == 1 ? host_threads() : 1, k.patches,
+      if (!make_cluster_patches(c, scenes[s], nn[s], off, slot, x0, word, ctas, part, S == 1 ? host_threads(nn[s]) : 1, k.patches,
                                 k.blob))
         continue;
       CluLaunch r{};
@@ -3290,8 +3322,8 @@ int build_pack(fw_ctx* c, int patch_nodes, bool pinned, fw_pack** out) {
   CluLaunch clu{};
   std::vector<CluPatch> cpatch;
   std::vector<unsigned char> cblob;
-  auto cut = [&] {
-    if (!patch_nodes || Bs > kCluMaxBodies || pairs.size() > (size_t)kCluMaxPairs) return;
+  auto cut_clusters = [&] {
+    if (Bs > kCluMaxBodies || pairs.size() > (size_t)kCluMaxPairs) return;
     bool per_tri = Bs > 1;
     int64_t at = 0;
     for (int b = 0; b < Bs; ++b) {  // bodies one after the other
@@ -3325,21 +3357,35 @@ int build_pack(fw_ctx* c, int patch_nodes, bool pinned, fw_pack** out) {
     cpatch.clear();
     cblob.clear();
   };
-  std::thread cutter(cut);
-  struct Join {
-    std::thread& t;
-    ~Join() { t.join(); }
+  auto cut = [&] {  // without them the stream kernels step the scene
+    try {
+      cut_clusters();
+    } catch (const std::exception&) {
+      clu = CluLaunch{};
+      cpatch.clear();
+      cblob.clear();
+    }
   };
   // stream records
   PatchSet ps;
   if (patch_nodes) {
-    Join wait{cutter};
+    struct Join {
+      std::thread t;
+      ~Join() { if (t.joinable()) t.join(); }
+    } cutter;
+    bool beside = host_threads(4 * Ns) > 1;
+    if (beside) {
+      try {
+        cutter.t = std::thread(cut);
+      } catch (const std::exception&) {  // no thread to be had
+        beside = false;
+      }
+    }
+    if (!beside) cut();
     std::string why;
     std::vector<int32_t> bscene(Bs, 0);
     if (make_patches((int)Ns, (int)Es, conn.data(), off, slot, x0, c->h_noff, c->h_ncnt, bscene, patch_nodes, ps, why))
       return fail(c, FW_ERR_ARG, "%s", why.c_str());
-  } else {
-    cutter.join();
   }
   fw_pack* pk = new fw_pack();
   pk->clu = clu;
@@ -4042,8 +4088,7 @@ int build_flex(fw_ctx* c) {
   return FW_OK;
 }
 
-int fw_finalize(fw_ctx* c) {
-  if (!c) return FW_ERR_ARG;
+static int finalize(fw_ctx* c) {
   if (c->device < 0) return fail(c, FW_ERR_STATE, "fw_finalize on a staging context (fw_create_stage)");
   if (c->finalized) return fail(c, FW_ERR_STATE, "fw_finalize called twice");
   if (c->N <= 0 || c->E <= 0 || c->B <= 0 || c->S <= 0)
@@ -4347,6 +4392,11 @@ static int shared_optin(fw_ctx* c) {
   int optin = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
   return optin;
+}
+
+int fw_finalize(fw_ctx* c) {
+  if (!c) return FW_ERR_ARG;
+  return guarded(c, [&] { return finalize(c); });
 }
 
 int fw_set_option(fw_ctx* c, int32_t option, int32_t value) {
@@ -4672,7 +4722,7 @@ int fw_arena_pack(fw_ctx* stage, int32_t patch_nodes, int32_t flags, fw_pack** o
   *out = nullptr;
   if (stage->finalized && !stage->arena)
     return fail(stage, FW_ERR_STATE, "fw_arena_pack: stage on a context that is not finalized, or on an arena");
-  return build_pack(stage, patch_nodes, (flags & FW_PACK_PINNED) != 0, out);
+  return guarded(stage, [&] { return build_pack(stage, patch_nodes, (flags & FW_PACK_PINNED) != 0, out); });
 }
 
 int fw_pack_info(const fw_pack* pk, int64_t* info) {
@@ -4843,7 +4893,7 @@ int fw_arena_commit(fw_ctx* c, int32_t* scene_out) {
   if (!c || !scene_out) return FW_ERR_ARG;
   if (!c->arena) return fail(c, FW_ERR_STATE, "fw_arena_commit without fw_arena_init");
   fw_pack* pk = nullptr;
-  int rc = build_pack(c, c->a_stream ? c->st_nodes : 0, false, &pk);
+  int rc = guarded(c, [&] { return build_pack(c, c->a_stream ? c->st_nodes : 0, false, &pk); });
   if (rc) return rc;
   rc = fw_arena_commit_pack(c, pk, scene_out);
   delete pk;  // pageable: its copies were staged before they returned

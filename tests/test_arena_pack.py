@@ -83,3 +83,41 @@ def test_options_read_back():
     with pytest.raises(_native.NativeError):
         st.get_option(_native.FW_OPT_WAIT_LIMIT)
     st.close()
+
+
+_NO_THREADS = """
+import resource
+import flatworld_b200 as fw
+from flatworld_b200 import _native
+from flatworld_b200.world import PackedWorld, SceneLayout, stage
+
+conn, coords = fw.structured_rectangle(80, 60, 0.8, 0.6, origin=(0.0, 0.0))
+fem = fw.FemDomain(fw.Mesh(2, conn, coords), fw.SolidProp(fw.Elastic(5e4, 0.3, 500.0)), [])
+packed = PackedWorld([SceneLayout([fw.GroundDomain(2, [0.0, 0.0], [0.0, 1.0]), fem])])
+size = []
+for limited in (False, True):
+    st = _native.NativeWorld.stage()
+    stage(st, packed)
+    if limited:  # room for the pack, but not for a thread's stack
+        pages = int(open("/proc/self/statm").read().split()[0])
+        resource.setrlimit(resource.RLIMIT_AS, (pages * resource.getpagesize() + (256 << 20),) * 2)
+    size.append(st.arena_pack(64).device_bytes)
+assert size[0] == size[1], size
+"""
+
+
+def test_pack_where_no_thread_can_be_made():
+    """Part of a pack is cut on a second thread; without one the pack is the same, and the process goes on."""
+    import os
+    import resource
+    import subprocess
+    import sys
+
+    def large_stacks():
+        resource.setrlimit(resource.RLIMIT_STACK, (1 << 30, resource.getrlimit(resource.RLIMIT_STACK)[1]))
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, OPENBLAS_NUM_THREADS="1", OMP_NUM_THREADS="1")
+    done = subprocess.run([sys.executable, "-c", _NO_THREADS], cwd=root, env=env, preexec_fn=large_stacks,
+                          capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, (done.returncode, done.stderr[-2000:])
