@@ -1360,6 +1360,8 @@ struct fw_ctx {
   bool a_stream = false;
   FreeList fl_patch, fl_halo, fl_ptri, fl_csrp, fl_cpatch, fl_cblob;
   int64_t st_ptri_cap = 0;  // patch triangles the arena holds
+  int64_t occ_cap = 0;      // voxel cells the arena holds
+  bool vox_asked = false;   // their table has been asked for
   CluPatch* d_cpatch = nullptr;
   unsigned char* d_cblob = nullptr;
   CluScene* d_cscene = nullptr;  // the scenes of a call, in launch order
@@ -1521,10 +1523,29 @@ template <typename T>
 int dalloc(fw_ctx* c, T** p, size_t count) {
   size_t bytes = sizeof(T) * (count ? count : 1);
   cudaError_t e = cudaMalloc((void**)p, bytes);
-  if (e != cudaSuccess)
+  if (e != cudaSuccess) {
+    cudaGetLastError();
     return fail(c, FW_ERR_OOM, "cudaMalloc(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
+  }
   c->allocs.push_back((void*)*p);
   return FW_OK;
+}
+
+// Device memory that a world gets faster with but does without: false (and a
+// null *p) where there is none.
+template <typename T>
+bool dalloc_spare(fw_ctx* c, T** p, size_t count) {
+  const std::string err = c->err;
+  if (dalloc(c, p, count) == FW_OK) return true;
+  c->err = err;
+  *p = nullptr;
+  return false;
+}
+
+// Gives back what was allocated after the first `mark` allocations.
+void dfree_from(fw_ctx* c, size_t mark) {
+  cudaStreamSynchronize(c->stream);  // copies into it may be on their way
+  for (; c->allocs.size() > mark; c->allocs.pop_back()) cudaFree(c->allocs.back());
 }
 
 int alloc_flags(fw_ctx* c) {
@@ -2534,6 +2555,25 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
   }
   c->clu_patches = (int)patches.size();
   return clu_side_streams(c);
+}
+
+// build_cluster where there is device memory for it; else the path's own
+// kernels step every scene.
+int try_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<int32_t>& slot,
+                const std::vector<float2>& x0, const std::vector<uint32_t>& word, bool single) {
+  const size_t mark = c->allocs.size();
+  const std::string err = c->err;
+  const int rc = build_cluster(c, off, slot, x0, word, single);
+  if (rc != FW_ERR_OOM) return rc;
+  dfree_from(c, mark);
+  c->err = err;
+  c->clu.clear();
+  c->clu_order.clear();
+  c->rest_scenes.clear();
+  c->d_rest_scenes = nullptr;
+  c->d_rest_rng = nullptr;
+  c->sd.list = nullptr;
+  return FW_OK;
 }
 
 // The resident patches, laid out when they are first needed (> 0: they do not fit).
@@ -4243,8 +4283,7 @@ static int finalize(fw_ctx* c) {
   c->launches += 2;
   bool table = false;  // of the nearest free voxel cells
   for (const Pair& p : pairs) table |= p.kind == fw::PAIR_VOXEL && !p.pad;
-  if (table) {
-    if ((rc = dalloc(c, &d.vox, c->h_occ.size()))) return rc;
+  if (table && dalloc_spare(c, &d.vox, c->h_occ.size())) {  // without it the grids are walked
     k_voxel_table<<<(unsigned)pairs.size(), 256, 0, c->stream>>>(d, 0);
     c->launches += 1;
   }
@@ -4354,11 +4393,11 @@ static int finalize(fw_ctx* c) {
   }
   if (c->path_req == FW_PATH_STREAM) {
     if ((rc = build_stream(c, off, slot, x0, has_j2))) return rc;
-    if ((rc = build_cluster(c, off, slot, x0, word, false))) return rc;
+    if ((rc = try_cluster(c, off, slot, x0, word, false))) return rc;
     c->path = FW_PATH_STREAM;
     FW_CUDA(c, cudaStreamSynchronize(c->stream));
   } else if (c->path_req != FW_PATH_GATHER) {
-    if (S == 1 && c->patches_req == 0 && (rc = build_cluster(c, off, slot, x0, word, true))) return rc;
+    if (S == 1 && c->patches_req == 0 && (rc = try_cluster(c, off, slot, x0, word, true))) return rc;
     if (!c->clu.empty()) {
       c->path = FW_PATH_RESIDENT;
     } else {
@@ -4631,7 +4670,6 @@ int fw_arena_init(fw_ctx* c, int64_t max_nodes, int64_t max_elems, int32_t max_b
       (rc = dalloc(c, &d.aabb_ring, 8 * (size_t)B)) || (rc = dalloc(c, &c->a_young, E)) ||
       (rc = dalloc(c, &c->a_poisson, E)) || (rc = dalloc(c, &c->a_rho, E)) || (rc = dalloc(c, &d.scene_bad, S)))
     return rc;
-  if (max_occ > 0 && (rc = dalloc(c, &d.vox, max_occ))) return rc;
   FW_CUDA(c, cudaMemsetAsync(d.scene_bad, 0, sizeof(int32_t) * S, c->stream));
   c->stage_cap = (size_t)64 << 20;  // packs up to 64 MB commit in one copy (larger ones part by part)
   if ((rc = dalloc(c, &c->d_stage, c->stage_cap))) return rc;
@@ -4659,6 +4697,7 @@ int fw_arena_init(fw_ctx* c, int64_t max_nodes, int64_t max_elems, int32_t max_b
   c->fl_pairs.init(max_pairs);
   c->fl_heights.init(max_heights);
   c->fl_occ.init(max_occ);
+  c->occ_cap = max_occ;
   c->ascenes.assign(S, fw_ctx::ArenaScene{});
   c->a_body_scene.assign(B, S - 1);
   c->free_scene_ids.clear();
@@ -4699,11 +4738,18 @@ int fw_arena_init(fw_ctx* c, int64_t max_nodes, int64_t max_elems, int32_t max_b
     c->fl_csrp.init(CPcap);
     if (c->clu_opt) {
       const int64_t Qcap = N / kCluServedNodes * 2 + 16 * (int64_t)S, Bcap = 24 * N + 32 * E + 256 * Qcap;
-      if ((rc = dalloc(c, &c->d_cpatch, Qcap)) || (rc = dalloc(c, &c->d_cblob, Bcap)) || (rc = dalloc(c, &c->d_cscene, S)) ||
-          (rc = dalloc(c, &c->d_runs, S)) || (rc = clu_prepare(c, &c->clu_cap, c->clu_size_ok)))
-        return rc;
-      c->fl_cpatch.init(Qcap);
-      c->fl_cblob.init(Bcap);
+      const size_t mark = c->allocs.size();
+      if (dalloc_spare(c, &c->d_cblob, Bcap) && dalloc_spare(c, &c->d_cscene, S) && dalloc_spare(c, &c->d_runs, S) &&
+          dalloc_spare(c, &c->d_cpatch, Qcap)) {
+        if ((rc = clu_prepare(c, &c->clu_cap, c->clu_size_ok))) return rc;
+        c->fl_cpatch.init(Qcap);
+        c->fl_cblob.init(Bcap);
+      } else {  // no room: the stream kernels step every scene
+        dfree_from(c, mark);
+        c->d_cblob = nullptr;
+        c->d_cscene = nullptr;
+        c->d_runs = nullptr;
+      }
     }
     stream_smem(1, 1, 1, &c->st_smem, &c->st_smem_bulk);
     if ((rc = stream_attrs(c, shared_optin(c)))) return rc;
@@ -4862,7 +4908,14 @@ int fw_arena_commit_pack(fw_ctx* c, const fw_pack* pk, int32_t* scene_out) {
   r.count = std::max<int64_t>({3 * a.ne, a.nn, a.nb, a.np, a.nhh, a.nt, a.npp});
   k_arena_reloc<<<(int)std::min<int64_t>((r.count + kBlock - 1) / kBlock, 8 * c->sms), kBlock, 0, c->stream>>>(d, r);
   const int e_lo = (int)e0, e_hi = (int)(e0 + a.ne), n_lo = (int)n0, n_hi = (int)(n0 + a.nn);
-  if (a.np > 0 && a.no > 0) k_voxel_table<<<(unsigned)a.np, 256, 0, c->stream>>>(d, (int)a.p0);
+  if (a.np > 0 && a.no > 0) {
+    // the arena's first voxel pairs: the cell table, eight times the cells'
+    // bytes, which arenas without such pairs do not need (no room for it: the
+    // grids are walked)
+    if (!c->vox_asked) dalloc_spare(c, &d.vox, (size_t)c->occ_cap);
+    c->vox_asked = true;
+    if (d.vox) k_voxel_table<<<(unsigned)a.np, 256, 0, c->stream>>>(d, (int)a.p0);
+  }
   k_prepare_elements<<<(int)((a.ne + kBlock - 1) / kBlock), kBlock, 0, c->stream>>>(d, c->a_young + e0, c->a_poisson + e0,
                                                                                   c->a_rho + e0, e_lo, e_hi);
   k_prepare_mass<<<(int)((a.nn + kBlock - 1) / kBlock), kBlock, 0, c->stream>>>(d, n_lo, n_hi);
@@ -5083,8 +5136,7 @@ int fw_adj_begin(fw_ctx* c, int32_t max_segment_steps) {
       CluAdjKernel k = clu_adj_kernel(threads);
       FW_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)optin - kCluStatic)));
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, need) == cudaSuccess &&
-          per_sm * sms >= q.r.ctas) {
-        if ((rc = dalloc(c, &q.words, 4 * (size_t)q.r.n_halo))) return rc;
+          per_sm * sms >= q.r.ctas && dalloc_spare(c, &q.words, 4 * (size_t)q.r.n_halo)) {
         FW_CUDA(c, cudaMemsetAsync(q.words, 0, sizeof(ulonglong2) * 4 * (size_t)q.r.n_halo, c->stream));
         c->clu_adj = q;
         c->clu_adj_threads = threads;

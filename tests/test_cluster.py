@@ -352,6 +352,32 @@ def test_voxel_contact_on_long_grids(nx, ny, at):
     assert np.array_equal(batch.coords(1).astype(np.float64), x)
 
 
+def test_voxel_cells_take_a_table_only_where_there_is_room():
+    """An arena without voxel grounds takes no memory for them beyond the cells, and one whose cell table the device
+    cannot hold (192 GiB here) walks the grids: the same bits as a scene of its own."""
+    import torch
+
+    from flatworld_b200.serve import Arena
+
+    torch.cuda.init()
+    before = torch.cuda.mem_get_info()[0]
+    ar = Arena(20_000, 40_000, 8, 8, 32, 1 << 10, 1 << 30)
+    assert before - torch.cuda.mem_get_info()[0] < 3 << 30
+    ar.close()
+    ar = Arena(20_000, 40_000, 8, 8, 32, 1 << 10, 24 << 30)
+    dt = np.float32(5e-5)
+    build = [lambda: _rectangle(12, 7, MATS["elastic"], _plane()), lambda: _terrain_scene(31, 64, "marked"),
+             lambda: _terrain_scene(130, 33, "solid")]
+    sc = [ar.insert(b()) for b in build]
+    for n in (1, 2, 18):
+        ar.native.step_served_n(np.where(np.isin(np.arange(ar.S), sc), dt, np.float32(0.0)), n)
+    for s, b in zip(sc, build):
+        lp = fw.ExplicitLoop(5e-5, b(), useAdapativeDT=False)
+        lp.advance_n(20)
+        assert np.array_equal(ar.coords(s), lp.femSpringManager.coords.numpy()[: lp._packed.N])
+    ar.close()
+
+
 @pytest.mark.parametrize("n,ground", [(3, "plane"), (16, "plane"), (41, "bump"), (70, "bump"), (150, "plane")])
 def test_reverse_pass_matches_the_gather_reverse(n, ground):
     """One patch, several, and meshes whose patches hold more than 512 triangles; contact on."""
