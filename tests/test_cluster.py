@@ -283,6 +283,30 @@ def test_wait_runs_out_and_the_context_recovers():
     b.synchronize()
 
 
+@pytest.mark.parametrize("name", ["two patches", "records in L2"])
+def test_a_wait_that_ran_out_is_reported_whatever_ran_after(name):
+    """A call whose waits gave up, then calls on the gather kernels, or the on-chip step given up for good (the large
+    mesh then has the gather kernels only): the next synchronisation still reports it, and once."""
+    for after in ("short call", "off"):
+        lp = fw.ExplicitLoop(0.0, SINGLE[name]())
+        lp.advance_n(5)
+        lp.advance_n(1)
+        lp.synchronize()
+        lp._native.set_option(_native.FW_OPT_WAIT_LIMIT, 4096)
+        lp._native.set_option(_native.FW_OPT_TEST_WITHHOLD, 1)
+        lp.advance_n(10)
+        lp._native.set_option(_native.FW_OPT_TEST_WITHHOLD, -1)
+        if after == "off":
+            lp._native.set_option(_native.FW_OPT_CLUSTER, 0)
+            assert lp._native.get_path()[0] == (2 if name == "two patches" else 1)
+        else:
+            lp.advance_n(1)
+        with pytest.raises(RuntimeError, match="gave up"):
+            lp.synchronize()
+        lp.advance_n(1)
+        lp.synchronize()
+
+
 def _terrain_scene(nx, ny, kind):
     """A block on (and partly inside) a voxel grid of nx x ny cells: solid, solid with cells of neither state, or
     random."""
