@@ -63,16 +63,14 @@ int clu_min_steps(int sms, int64_t triangles) {
   return triangles <= (int64_t)sms * 1500 ? 3 : triangles <= (int64_t)sms * 6500 ? 5 : 8;
 }
 
-// The same for a single scene, whose shorter calls run on the gather kernels:
-// one substep is two plain launches, 5 to 10 us less than a cooperative one and
-// the patches' loads; more of them, as a graph, only where a mesh is so large
-// that the loads take as long as the gather kernels' substeps.  A call and its
-// synchronisation, on chip / gather, us: up to 131072 triangles 1 substep 31 /
-// 25, 2: 31 / 33; 537600 2: 49 / 43, 3: 55 / 62; 655360 2: 54 / 51, 3: 64 / 65,
-// 4: 73 / 87; 798000 3: 79 / 75, 4: 88 / 92.
-int grid_min_steps(int sms, int64_t triangles) {
-  return triangles <= (int64_t)sms * 2500 ? 2 : triangles <= (int64_t)sms * 4000 ? 3 : 4;
-}
+// The same for a single scene, whose shorter calls run on the gather kernels,
+// two plain launches a substep instead of a cooperative one and the patches'
+// loads.  A call and its synchronisation, on chip / gather, us: 2 substeps of
+// 2048 triangles 30 / 23, of 131072 35 / 25, of 319200 42 / 31; 3 of 2048 29 / 31,
+// 32768 33 / 32, 131072 41 / 33, 409600 53 / 46; 4 of 131072 41 / 43, 409600
+// 53 / 58, 655360 72 / 78.  A call and a read of one node: 3 of 32768 37 / 40,
+// 131072 42 / 41, 409600 53 / 52.
+int grid_min_steps(int sms, int64_t triangles) { return triangles <= (int64_t)sms * 500 ? 3 : 4; }
 
 struct Dev {
   float2* x;

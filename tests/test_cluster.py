@@ -216,6 +216,16 @@ def test_short_calls_of_one_scene_equal_the_gather_kernels(n):
     _same(a, b)
 
 
+@pytest.mark.parametrize("n,least", [(20, 3), (150, 4), (420, 4)])
+def test_least_substeps_of_an_on_chip_call(n, least):
+    """Shorter calls are two plain launches a substep: 15,200, 114,000 and 319,200 triangles."""
+    lp = fw.ExplicitLoop(0.0, _rectangle(n, 380, MATS["neohookean"], _plane(-0.0005), cell=0.002))
+    for k in range(1, 6):
+        before = lp._native.launch_count()
+        lp.advance_n(k)
+        assert lp._native.launch_count() - before == (1 if k >= least else 2 * k)
+
+
 @pytest.mark.parametrize("bodies", [4, 34])
 def test_short_calls_equal_the_stream_kernels(bodies):
     """Calls on both sides of the length from which a batch is stepped on chip, below and above 1500 triangles per SM."""
