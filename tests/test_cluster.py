@@ -270,6 +270,25 @@ def test_nan_nodes_leave_the_contact_of_the_others(build, bad):
         _same(loops[0], lp)
 
 
+def test_tuning_a_single_scene_times_the_default_too(tmp_path, monkeypatch):
+    import json
+
+    from flatworld_b200 import autotune
+
+    monkeypatch.setenv("FLATWORLD_B200_CACHE", str(tmp_path))
+    kw = autotune.tune_resident(SINGLE["two patches"], fronts=(4, 6), patches=(0, 2), steps=50)
+    (entry,) = json.loads((tmp_path / "autotune.json").read_text()).values()
+    shapes = [(c["front_warps"], c["patches"]) for c in entry["candidates"]]
+    assert shapes == [(0, 0), (4, 0), (4, 2), (6, 0), (6, 2)]
+    best = min(entry["candidates"], key=lambda c: c["ms"])
+    assert kw == {"front_warps": best["front_warps"], "patches": best["patches"]}
+    a, b = fw.ExplicitLoop(0.0, SINGLE["two patches"](), **kw), fw.ExplicitLoop(0.0, SINGLE["two patches"]())
+    assert a._native.get_option(_native.FW_OPT_CLUSTER) == (1 if kw == {"front_warps": 0, "patches": 0} else 0)
+    for lp in (a, b):
+        lp.advance_n(50)
+    _same(a, b)
+
+
 def test_wait_runs_out_and_the_context_recovers():
     lp = fw.ExplicitLoop(0.0, SINGLE["two patches"]())
     lp.advance_n(20)
