@@ -53,13 +53,15 @@ def _gpu_name(device):
     return torch.cuda.get_device_name(device)
 
 
-def _time_steps(native, steps, dt, stream):
+def _time_steps(native, steps, dt, stream, per_call=0):
+    """Milliseconds per substep of ``steps`` substeps, in one call or ``per_call`` at a time."""
     import torch
 
     s = torch.cuda.Event(enable_timing=True)
     e = torch.cuda.Event(enable_timing=True)
     s.record(stream)
-    native.step(steps, dt)
+    for done in range(0, steps, per_call or steps):
+        native.step(min(per_call or steps, steps - done), dt)
     e.record(stream)
     e.synchronize()
     return s.elapsed_time(e) / steps
@@ -73,23 +75,23 @@ def tune_stream(loop, steps=16, use_cache=True):
     (bulk copy or per-thread loads) for ``loop`` (a BatchedLoop on the stream
     path), timed on the loop's own world from a snapshot, as tune_batched.
 
-    A loop whose scenes are all stepped on chip keeps that: setting a shape of
-    the stream kernels would give it up (2048 ragged bodies, 100 substeps in a
-    call: 290 us per substep on chip, 418 on the best stream shape)."""
+    Scenes that are stepped on chip stay there (2048 ragged bodies, 100 substeps
+    in a call: 290 us per substep on chip, 418 on the best stream shape); the
+    stream kernels run their shorter calls, so for a loop with such scenes
+    (``on_chip`` in the result) calls of two substeps are timed."""
     import torch
 
     from . import _native
 
-    if loop._native.get_option(_native.FW_OPT_CLUSTER) == 1:
-        return {"path": "stream", "patch": loop.stream_patch, "minb": loop.stream_minb, "bulk": bool(loop.stream_bulk),
-                "on_chip": True, "candidates": []}
+    on_chip = loop._native.get_option(_native.FW_OPT_CLUSTER) != 0
+    per_call = 2 if on_chip else steps
     key = (f"stream|{_gpu_name(loop._native.device)}|N={loop.n_nodes}|E={loop.n_elems}|S={loop.S}"
            f"|patch={loop.stream_patch}")
     if use_cache:
         hit = _load_cache().get(key)
         if hit:
             loop.set_stream_shape(hit["minb"], hit["bulk"])
-            return dict(hit, cached=True)
+            return dict(hit, cached=True, on_chip=on_chip)
     stream = torch.cuda.Stream(device=loop._native.device)
     loop.set_stream(stream.cuda_stream)
     dt = float(np.float32(loop.dt.min()))
@@ -105,14 +107,14 @@ def tune_stream(loop, steps=16, use_cache=True):
             nat.restore(_SNAP)
             nat.step(2, dt)
             nat.restore(_SNAP)
-            results.append((_time_steps(nat, steps, dt, stream), minb, bulk))
+            results.append((_time_steps(nat, steps, dt, stream, per_call), minb, bulk))
     nat.restore(_SNAP)
     nat.synchronize()
     ms, minb, bulk = min(results)
     loop.set_stream_shape(minb, bulk)
     loop.set_stream(None)
     out = {"path": "stream", "patch": loop.stream_patch, "minb": minb, "bulk": bool(bulk), "ms_per_step": ms,
-           "candidates": [{"minb": m, "bulk": bool(b), "ms": t} for t, m, b in results]}
+           "on_chip": on_chip, "candidates": [{"minb": m, "bulk": bool(b), "ms": t} for t, m, b in results]}
     _store_cache(key, out)
     return out
 

@@ -4518,9 +4518,7 @@ int fw_set_option(fw_ctx* c, int32_t option, int32_t value) {
                     c->st_nodes == 64 ? "16, 20, 24 or 32" : "8, 10, 12 or 16");
       c->st_minb = value;
       if (c->st_bulk && !stream_kernel(c->st_nodes, value, 1)) c->st_bulk = 0;  // loads-only budget
-      c->shape_asked = true;
-      if (!c->arena)
-        if (int rc = cluster_off(c)) return rc;
+      if (!c->finalized) c->shape_asked = true;
       drop_graphs(c);
       return FW_OK;
     }
@@ -4531,9 +4529,7 @@ int fw_set_option(fw_ctx* c, int32_t option, int32_t value) {
       if (value && !stream_kernel(c->st_nodes, c->st_minb, 1))
         return fail(c, FW_ERR_ARG, "FW_OPT_STREAM_BULK: no staged variant at %d CTAs per SM", c->st_minb);
       c->st_bulk = value;
-      c->shape_asked = true;
-      if (!c->arena)
-        if (int rc = cluster_off(c)) return rc;
+      if (!c->finalized) c->shape_asked = true;
       drop_graphs(c);
       return FW_OK;
     }

@@ -316,11 +316,13 @@ int fw_set_path(fw_ctx* ctx, int32_t path, int32_t patches);
  * to one patch per SM, and every scene of the stream path that fits the shared
  * memory of a thread-block cluster, each on its own.  0 leaves every scene to
  * the path's own kernels, also when set after fw_finalize.  Setting a launch
- * shape of the resident or stream step (FRONT_WARPS, RES_THREADS, RES_SYNC,
- * STREAM_PATCH / MINB / BULK, or a patch count in fw_set_path) has the same
- * effect, and so have more than 8 bodies or 32 contact pairs in a scene.  Calls
- * of one or a few substeps (by the world's size) run on the gather or stream
- * kernels in any case.  Same bits.  fw_get_option: 0 none, 1 every scene, 2 some
+ * shape of the resident or stream step before fw_finalize (FRONT_WARPS,
+ * RES_THREADS, RES_SYNC, STREAM_PATCH / MINB / BULK, or a patch count in
+ * fw_set_path) has the same effect -- except in an arena -- and so have more
+ * than 8 bodies or 32 contact pairs in a scene.  After fw_finalize STREAM_MINB
+ * and STREAM_BULK shape the stream kernels where those run and leave the other
+ * scenes on chip.  Calls of one or a few substeps (by the world's size) run on
+ * the gather or stream kernels in any case.  Same bits.  fw_get_option: 0 none, 1 every scene, 2 some
  * scenes of the world are stepped this way. */
 #define FW_OPT_CLUSTER 12
 int fw_set_option(fw_ctx* ctx, int32_t option, int32_t value);

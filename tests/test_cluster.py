@@ -270,6 +270,26 @@ def test_nan_nodes_leave_the_contact_of_the_others(build, bad):
         _same(loops[0], lp)
 
 
+@pytest.mark.parametrize("sizes,covered", [([(20, 9), (7, 30)], 1), ([(20, 9), (200, 160)], 2)])
+def test_tuning_shapes_the_stream_kernels_of_short_calls(sizes, covered, tmp_path, monkeypatch):
+    """The scenes on chip stay there, also beside one too large for it; the stream kernels get the shape."""
+    from flatworld_b200 import autotune
+
+    monkeypatch.setenv("FLATWORLD_B200_CACHE", str(tmp_path))
+    a, b = (BatchedLoop(_batch(sizes), dt=5e-5, useAdapativeDT=False) for _ in range(2))
+    best = autotune.tune_batched(a, steps=4)
+    assert a._native.get_option(_native.FW_OPT_CLUSTER) == covered and best["on_chip"]
+    assert (best["minb"], best["bulk"]) in [(c["minb"], c["bulk"]) for c in best["candidates"]]
+    a.set_stream_shape(16, True)
+    assert a._native.get_option(_native.FW_OPT_CLUSTER) == covered
+    assert a._native.get_option(_native.FW_OPT_STREAM_MINB) == 16
+    for lp in (a, b):
+        lp._packed = lp.packed
+        for n in (1, 2, 9, 1, 20):
+            lp.advance(n)
+    _same(a, b)
+
+
 def test_tuning_a_single_scene_times_the_default_too(tmp_path, monkeypatch):
     import json
 
