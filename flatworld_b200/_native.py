@@ -88,6 +88,7 @@ _SIGNATURES = {
     "fw_tan_begin": (C.c_int, [_vp, _vp, _vp, _vp, C.c_int32]),
     "fw_tan_step": (C.c_int, [_vp, C.c_int32, C.c_float]),
     "fw_tan_read": (C.c_int, [_vp, _vp, _vp, C.c_int32]),
+    "fw_log_f32": (C.c_int, [_vp, _vp, _vp, C.c_int64, _vp]),
     "fw_arena_init": (C.c_int, [_vp, C.c_int64, C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int64, C.c_int64]),
     "fw_arena_commit": (C.c_int, [_vp, _i32p]),
     "fw_arena_remove": (C.c_int, [_vp, C.c_int32]),

@@ -725,6 +725,13 @@ __global__ void k_rigid_init(Rigid* rig, int n) {
   if (rig[a].type != fw::RIGID_ANALYTICAL) fw::rigid_aabb(rig[a]);  // an analytical entry starts at getBBox()
 }
 
+__global__ void k_log(const float* __restrict__ x, float* __restrict__ y, float* __restrict__ quotient, int64_t n) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  y[i] = fw::fw_log(x[i]);
+  if (quotient) quotient[i] = fw::log_quotient(x[i]);
+}
+
 // Per cell of the voxel pairs [p0, p0 + gridDim.x) the nearest free cells that
 // fw::contact_force looks for (zero for a cell that is not occupied): a block
 // per pair, a thread per row (walked both ways) and per column.
@@ -5713,6 +5720,13 @@ int fw_read_counters(fw_ctx* c, int64_t* counters) {
 }
 
 int64_t fw_launch_count(const fw_ctx* c) { return c ? c->launches : 0; }
+
+int fw_log_f32(const float* x, float* log_x, float* quotient, int64_t n, void* stream) {
+  if (!x || !log_x || n < 0 || n > (1ll << 31)) return FW_ERR_ARG;
+  if (n == 0) return FW_OK;
+  k_log<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, (cudaStream_t)stream>>>(x, log_x, quotient, n);
+  return cudaGetLastError() == cudaSuccess ? FW_OK : FW_ERR_CUDA;
+}
 
 const char* fw_build_info(void) {
   return "libfwb200: sm_100a, -fmad=false, IEEE div/sqrt; gather step + shared-memory-resident step";

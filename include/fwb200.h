@@ -587,6 +587,13 @@ int fw_tan_begin(fw_ctx* ctx, const float* dx0, const float* dv0, const float* d
 int fw_tan_step(fw_ctx* ctx, int32_t n_steps, float dt);
 int fw_tan_read(fw_ctx* ctx, float* dx, float* dv, int32_t on_device);
 
+/* The logarithm of the NeoHookean law as the kernels evaluate it, on n floats of
+ * device memory: log_x[i] = log(x[i]) and, where quotient is not NULL,
+ * quotient[i] = (x[i] - 1) / (x[i] + 1) as the logarithm forms it (x[i] in
+ * (sqrt(1/2), sqrt(2)]).  For comparing it with another implementation; no
+ * reference counterpart (the reference calls the device's logf). */
+int fw_log_f32(const float* x, float* log_x, float* quotient, int64_t n, void* stream);
+
 /* Library build identification string (arch, flags). */
 const char* fw_build_info(void);
 

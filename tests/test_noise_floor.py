@@ -11,6 +11,7 @@ bit-identical operation for operation will show.
 """
 
 import numpy as np
+import pytest
 
 import flatworld_b200 as fw
 import oracle
@@ -53,3 +54,50 @@ def test_log_method_accuracy():
         worst = max(worst, abs(got - ref) / ulp)
     assert worst < 2.0, worst
     assert log32(1.0) == 0.0 and log32(0.0) == -np.inf and np.isnan(log32(-1.0)) and log32(np.inf) == np.inf
+
+
+def _device_log(x, quotient=False):
+    import torch
+
+    from flatworld_b200 import _native
+
+    t = torch.from_numpy(x).cuda()
+    out, q = torch.empty_like(t), torch.empty_like(t)
+    rc = _native.lib().fw_log_f32(t.data_ptr(), out.data_ptr(), q.data_ptr() if quotient else None, t.numel(),
+                                  torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    return (out.cpu().numpy(), q.cpu().numpy()) if quotient else out.cpu().numpy()
+
+
+def _same_bits(a, b):
+    same = (a.view(np.uint32) == b.view(np.uint32)) | (np.isnan(a) & np.isnan(b))
+    assert same.all(), (int((~same).sum()), int(np.flatnonzero(~same)[0]))
+
+
+@pytest.mark.gpu
+def test_device_quotient_is_the_division_on_every_mantissa():
+    """The kernels form the logarithm's quotient without a division: equal to it for all 2^23 arguments."""
+    m = np.arange(0x3F3504F4, 0x3FB504F4, dtype=np.uint32).view(np.float32)
+    assert len(m) == 1 << 23 and m[0] ** 2.0 > 0.5 and m[-1] ** 2.0 <= 2.0
+    one = np.float32(1.0)
+    _same_bits(_device_log(m, quotient=True)[1], (m - one) / (m + one))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sample", ["near one", "bit patterns", "edges"])
+def test_device_log_is_the_oracles(sample):
+    """The kernels' logarithm against the CPU oracle's: subnormals, zeros, negatives, infinities and NaN included."""
+    from oracle.scene import log32
+
+    if sample == "near one":  # every 64th float of [0.5, 2)
+        bits = np.arange(0x3F000000, 0x40000000, 64, dtype=np.uint32)
+    elif sample == "bit patterns":  # all signs and exponents
+        bits = np.random.default_rng(5).integers(0, 1 << 32, 300_000, dtype=np.uint32)
+    else:  # both sides of each power of two and of each change of the reduced mantissa
+        exps = np.arange(0, 256, dtype=np.uint32) << np.uint32(23)
+        near = np.arange(-3, 4).astype(np.int64)
+        bits = np.concatenate([(exps[:, None].astype(np.int64) + near[None] + off).ravel()
+                               for off in (0, 0x3504F4)]).astype(np.uint64) & np.uint64(0xFFFFFFFF)
+        bits = np.concatenate([bits.astype(np.uint32), bits.astype(np.uint32) | np.uint32(0x80000000)])
+    x = bits.view(np.float32)
+    _same_bits(_device_log(x), np.array([log32(v) for v in x], np.float32))
