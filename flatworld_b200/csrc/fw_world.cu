@@ -4136,10 +4136,15 @@ int build_flex(fw_ctx* c) {
   c->flex_pre_smem = sizeof(float4) * (size_t)max_dom_fem;
   int optin = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  if ((long)c->flex_pre_smem > optin)
+  // always the most that the kernel's static arrays leave: the attribute belongs
+  // to the function, so one context's figure must not fall below what another
+  // context launches with
+  cudaFuncAttributes fa{};
+  FW_CUDA(c, cudaFuncGetAttributes(&fa, k_flex_pre));
+  const size_t most = (size_t)optin - fa.sharedSizeBytes;
+  if (c->flex_pre_smem > most)
     return fail(c, FW_ERR_ARG, "FEM-FEM contact: a scene's domains need %zu B of shared memory", c->flex_pre_smem);
-  if (c->flex_pre_smem > 48 * 1024)
-    FW_CUDA(c, cudaFuncSetAttribute(k_flex_pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->flex_pre_smem));
+  FW_CUDA(c, cudaFuncSetAttribute(k_flex_pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   c->fx = f;
   c->d.flex_slot = dslot;
   c->d.flex_cnt = dcnt;

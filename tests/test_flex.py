@@ -241,3 +241,35 @@ def test_gpu_edge_search_equals_oracle(cells, radius, steps):
         assert np.array_equal(cache, o.flex_cache()), k
         touched |= bool((cache >= 0).any())
     assert touched
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bodies", [1475, 1520])
+def test_gpu_scenes_of_many_bodies_equal_oracle(bodies):
+    """Two disks in contact among bodies that meet nothing: 2951 and 3041 domain and body boxes, whose 16 bytes each
+    stay below 48 KB of shared memory by themselves, but not beside the kernel's own arrays."""
+    from flatworld_b200.definitions import COLLISION_CATEGORY_FEM, COLLISION_MASK_ALL
+
+    def build():
+        conn = np.array([[0, 1, 3], [0, 3, 2]], np.int32)
+        doms = [fw.GroundDomain(2, [0.0, 0.0], [0.0, 1.0])] + [
+            fw.FemDomain(scenes.ccw_disk(fw, 3, 0.025, (x, 0.025)), fw.SolidProp(fw.Elastic(E=1e5, nu=0.3, rho=1000.0)),
+                         [fw.Gravity([g, -9.8])]) for x, g in ((0.1, 9.8), (0.1 + 0.05 * (1.0 - 2e-4), -9.8))]
+        for k in range(bodies - 2):
+            at = np.array([1.0 + 0.1 * (k % 40), 0.1 + 0.1 * (k // 40)])
+            xy = (at + 0.05 * np.array([[0, 0], [1, 0], [0, 1], [1, 1]])).astype(np.float32)
+            fem = fw.FemDomain(fw.Mesh(2, conn, xy), fw.SolidProp(fw.Elastic(E=1e5, nu=0.3, rho=1000.0)), [])
+            fem.collide_bits = COLLISION_MASK_ALL & ~COLLISION_CATEGORY_FEM
+            doms.append(fem)
+        return doms
+
+    doms = build()
+    dt = 0.3 * SceneLayout(doms, useAdapativeDT=True).dt
+    lp = fw.ExplicitLoop(dt, doms, useAdapativeDT=False)
+    o = oracle.OracleLoop(doms, dt=dt, useAdapativeDT=False, threads=4)
+    lp.advance_n(120)
+    o.advance(120)
+    xo, vo, _ = o.state()
+    assert (o.flex_cache() >= 0).any()
+    assert np.array_equal(lp.femSpringManager.coords.numpy()[: o.N].astype(np.float64), xo)
+    assert np.array_equal(lp.femSpringManager.V.numpy()[: o.N].astype(np.float64), vo)
