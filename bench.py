@@ -185,12 +185,13 @@ def peaks():
     return 6650.0, "fallback"
 
 
-def ncu_traffic():
-    """Per-substep DRAM bytes of the step kernels from the committed ncu summary."""
+def ncu_traffic(kernel):
+    """Per-substep DRAM bytes of the step kernel ``kernel`` from the committed
+    ncu summary, or None where that kernel was not captured."""
     path = os.path.join(ROOT, "profiles", "traffic_plain_large.json")
     if os.path.exists(path):
         with open(path) as f:
-            return json.load(f).get("dram_bytes_per_substep")
+            return json.load(f).get(kernel, {}).get("dram_bytes_per_substep")
     return None
 
 
@@ -329,20 +330,29 @@ def run_batched(args, rank, world, local):
             torch.cuda.synchronize()
         launches = b.launch_count() - l0
         # ---- end to end: every body's positions and velocities in from pinned
-        # host memory, one step of 100 substeps, and back out
+        # host memory, one step of 100 substeps, and back out -- on the loop as
+        # it is by default (scenes that fit are stepped on chip), unless a patch
+        # size was asked for
         N = b.n_nodes
         xh = torch.empty((N, 2), dtype=torch.float32, pin_memory=True)
         vh = torch.empty((N, 2), dtype=torch.float32, pin_memory=True)
         b._native.read_nodes_ptr(0, 0, N, xh.data_ptr())
         b._native.read_nodes_ptr(1, 0, N, vh.data_ptr())
+        whole = b
+        if patch_tuning is not None:
+            whole = BatchedLoop(batch, dt=5e-5, useAdapativeDT=False, device=local, path=args.batch_path)
+            whole.set_stream(stream.cuda_stream)
+            for _ in range(args.warmup):
+                whole.advance(100)
+        on_chip = whole._native.get_option(_native.FW_OPT_CLUSTER)
         ev2 = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
         for s_, e_ in ev2:
             s_.record(stream)
-            b._native.write_nodes_ptr(0, 0, N, xh.data_ptr())
-            b._native.write_nodes_ptr(1, 0, N, vh.data_ptr())
-            b.advance(100)
-            b._native.read_nodes_ptr(0, 0, N, xh.data_ptr())
-            b._native.read_nodes_ptr(1, 0, N, vh.data_ptr())
+            whole._native.write_nodes_ptr(0, 0, N, xh.data_ptr())
+            whole._native.write_nodes_ptr(1, 0, N, vh.data_ptr())
+            whole.advance(100)
+            whole._native.read_nodes_ptr(0, 0, N, xh.data_ptr())
+            whole._native.read_nodes_ptr(1, 0, N, vh.data_ptr())
             e_.record(stream)
         torch.cuda.synchronize()
     barrier(dist)
@@ -403,7 +413,8 @@ def run_batched(args, rank, world, local):
                      "traffic_from": ("DRAM bytes per substep scaled from an ncu capture of a 256-body batch: "
                                       f"{ratio_src}")},
         "e2e": {"value": work_e2e / (ms_e2e / 1e3), "unit": "element-steps/s",
-                "h2d_bytes_per_step": 2 * N * 8, "d2h_bytes_per_step": 2 * N * 8},
+                "h2d_bytes_per_step": 2 * N * 8, "d2h_bytes_per_step": 2 * N * 8,
+                "step": f"100 substeps a call, {['no', 'all', 'some'][on_chip]} scenes on chip"},
         "gpu_launches": launches, "clocks": clk.summary(),
     }
     if rank == 0 and not args.no_cpu_baseline:
@@ -1156,7 +1167,9 @@ def main():
         per_sub_s = (ms / 1e3) / (substeps * args.steps)
         achieved = bstep / per_sub_s / 1e9
         peak, which = peaks()
-        traffic = ncu_traffic()
+        kernel = ("substep" if loop.path != 2 else
+                  "k_cluster" if loop._native.get_option(_native.FW_OPT_CLUSTER) else "k_resident")
+        traffic = ncu_traffic(kernel) if args.mesh == 256 else None
         line = {
             "metric": "FEM element-steps/s", "value": value, "unit": "element-steps/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps,
@@ -1171,16 +1184,16 @@ def main():
                        "front_warps": loop._native.get_option(_native.FW_OPT_FRONT_WARPS)
                        if loop.path == 2 and not loop._native.get_option(_native.FW_OPT_CLUSTER) else None},
             "roofline": {"bound": "hbm",
-                         "kernel": ("k_cluster, grid form (all substeps of a step)"
-                                    if loop._native.get_option(_native.FW_OPT_CLUSTER) else
-                                    "k_resident (all substeps of a step)") if loop.path == 2 else
-                                   "substep = k_elements + k_nodes",
+                         "kernel": {"k_cluster": "k_cluster, grid form (all substeps of a step)",
+                                    "k_resident": "k_resident (all substeps of a step)",
+                                    "substep": "substep = k_elements + k_nodes"}[kernel],
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_kind": which, "algorithmic_bytes_per_substep": bstep,
                          "us_per_substep": per_sub_s * 1e6,
                          "traffic": traffic,
-                         "traffic_from": "profiles/traffic_plain_large.json (ncu capture of this workload, "
-                                         "committed; not measured in this run)"},
+                         "traffic_from": None if traffic is None else
+                                         f"profiles/traffic_plain_large.json (ncu capture of {kernel} on this "
+                                         "workload, committed; not measured in this run)"},
             "e2e": {"value": e2e, "unit": "element-steps/s", "h2d_bytes_per_step": 2 * N * 8,
                     "d2h_bytes_per_step": 2 * N * 8},
             "gpu_launches": launches,

@@ -37,3 +37,18 @@ def test_stream_traffic_record_of_the_tuned_shape():
     with open(os.path.join(bench.ROOT, "profiles", "traffic_batched.json")) as f:
         shapes = json.load(f)["stream_shapes"]
     assert all(v >= 1.0 for v in shapes.values())
+
+
+def test_traffic_record_is_the_kernels_own():
+    """The plain line's DRAM bytes are a capture of the kernel that it names."""
+    import json
+    import os
+
+    with open(os.path.join(bench.ROOT, "profiles", "traffic_plain_large.json")) as f:
+        record = json.load(f)
+    assert "k_cluster" in record
+    for kernel, d in record.items():
+        assert d["kernel"].startswith(kernel + "<") and f"-k regex:{kernel} " in d["source"]
+        per = (d["dram_bytes_read_per_launch"] + d["dram_bytes_write_per_launch"]) / d["substeps_per_launch"]
+        assert bench.ncu_traffic(kernel) == d["dram_bytes_per_substep"] and abs(per - d["dram_bytes_per_substep"]) < 1
+    assert bench.ncu_traffic("substep") is None
