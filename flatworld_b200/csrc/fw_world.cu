@@ -1422,6 +1422,7 @@ struct fw_ctx {
   std::vector<CluScene> clu_scenes;
   int* d_flags = nullptr;  // the steps' error flags, one word each, read in one copy: enum Flag
   enum Flag { kFlagFlex, kFlagRigid, kFlagStream, kFlagCluster, kFlagResident, kFlags };
+  uint64_t short_key = 0;   // the last gather call of two or three substeps (launch_singly)
   bool flags_due = false;   // launches whose waits may give up, since the flags were last found clear
   bool flags_kept = false;  // ... and one of them went into a caller's graph, which may run at any time
   uint32_t clu_epoch = 0;  // grid form: tags used so far
@@ -1674,10 +1675,30 @@ uint32_t float_bits(float v) {
   return bits;
 }
 
+uint64_t graph_key(const fw_ctx* c, int n) {
+  return ((uint64_t)(c->d.uniform_dt ? 1 : 0) << 63) | ((uint64_t)n << 32) |
+         (c->d.uniform_dt ? float_bits(c->d.dt_uniform) : 0u);
+}
+
+// Two or three substeps at a step size that neither a graph nor the last such
+// call has: launched one by one, since making a graph costs more than it gives
+// once (a call of 2 with a new step size each time and its synchronisation, 2048
+// triangles: 90 us with a graph made for it, 33 without; a repeated one 23).
+bool launch_singly(fw_ctx* c, int n) {
+  if (n > 3) return false;
+  const uint64_t key = graph_key(c, n);
+  const bool again = key == c->short_key;
+  c->short_key = key;
+  if (again) return false;
+  if (c->graph_stream == c->stream)
+    for (const auto& g : c->graphs)
+      if (g.first == key) return false;
+  return true;
+}
+
 // Graph of n substeps (n <= kGraphSteps) of the gather step.
 int get_graph(fw_ctx* c, int n, cudaGraphExec_t* out) {
-  const uint64_t key = ((uint64_t)(c->d.uniform_dt ? 1 : 0) << 63) | ((uint64_t)n << 32) |
-                       (c->d.uniform_dt ? float_bits(c->d.dt_uniform) : 0u);
+  const uint64_t key = graph_key(c, n);
   const int64_t before = c->launches;
   const int rc = cached_graph(c, c->graphs, key, [&] {
     for (int k = 0; k < n; ++k) launch_step(c);  // every launch of a substep, FEM-FEM contact included
@@ -1719,7 +1740,7 @@ int run_steps(fw_ctx* c, int n) {
       n -= kGraphSteps;
     }
   }
-  if (n >= 2) {  // the remainder as one graph too
+  if (n >= 2 && !launch_singly(c, n)) {  // the remainder as one graph too
     cudaGraphExec_t g = nullptr;
     if ((rc = get_graph(c, n, &g))) return rc;
     FW_CUDA(c, cudaGraphLaunch(g, c->stream));

@@ -226,6 +226,19 @@ def test_least_substeps_of_an_on_chip_call(n, least):
         assert lp._native.launch_count() - before == (1 if k >= least else 2 * k)
 
 
+def test_short_calls_with_new_and_repeated_step_sizes():
+    """Launched one by one at first, as a graph when repeated: the same bits, and the launches of the substeps."""
+    a, b = (fw.ExplicitLoop(5e-5, _rectangle(20, 30, MATS["mises"], _plane()), useAdapativeDT=False, path=p)
+            for p in ("auto", "gather"))
+    for n, dt in ((2, 5e-5), (2, 5e-5), (2, 5e-5), (2, 4e-5), (2, 5e-5), (3, 3e-5), (2, 3e-5), (2, 4e-5), (2, 4e-5)):
+        before = a._native.launch_count()
+        a.advance_n(n, dt)
+        assert a._native.launch_count() - before == (4 if n == 2 else 1)
+        for _ in range(n):
+            b.advance_n(1, dt)
+    _same(a, b)
+
+
 @pytest.mark.parametrize("bodies", [4, 34])
 def test_short_calls_equal_the_stream_kernels(bodies):
     """Calls on both sides of the length from which a batch is stepped on chip, below and above 1500 triangles per SM."""
