@@ -1186,7 +1186,7 @@ __device__ void node_energy(const Dev& d, int i, double& ke, double& ext, double
 constexpr int kEnergyThreads = 256;
 // Nodes and triangles of a block.  The FP64 logarithm and divides of a NeoHookean
 // triangle set a block's time, so the blocks have to fill the SMs: chunks of
-// 8192 left 131072 triangles on 16 of them (92 us a report, 43 with 1024).
+// 8192 left 131072 triangles on 16 of them (92 us a report, 40 with 1024).
 constexpr int kEnergyChunk = 1024;
 
 // One block per chunk: fixed-order strided sums, then a fixed tree.
@@ -3431,8 +3431,8 @@ int build_pack(fw_ctx* c, int patch_nodes, bool pinned, fw_pack** out) {
       r.nb = Bs;
       r.np = (int)pairs.size();
       r.per_tri = per_tri;
-      r.one = 0;  // the larger of the two carve-ups
       clu_threads(r, true);
+      r.one = 0;  // the larger of the two carve-ups: a launch decides by its largest patch
       if (clu_smem(r) > kCluSharedBytes) continue;
       clu = r;
       return;
