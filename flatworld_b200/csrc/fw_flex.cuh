@@ -69,6 +69,7 @@ struct FlexDev {
   int max_pairs;
   float mpd;  // max(pow(100000.0f, 0.5f), 1.0f), evaluated on the host
   const FlexScene* sc;
+  const int4* scene_rng;   // per scene of the world: (first body, bodies, first pair, pairs)
   const double* clock_dt;  // per FEM-FEM scene: its substep dt as the host's float64 holds it
   int* err;                // bit 0: a node's contribution list overflowed
   const int32_t* item_node;
@@ -852,8 +853,11 @@ __device__ __forceinline__ void flex_item(const Dev& d, const FlexDev& f, const 
 }
 
 // Second launch of a substep: a warp per group of work items (grid stride).
-// control != 0: one block does the scenes' step control meanwhile, which only
-// the node step waits for.
+// The first `control` blocks of each row do the scenes' step control meanwhile,
+// which only the node step waits for: a block per scene.  (All scenes in one
+// block made it the longest part of a batch's substep: 2048 scenes of two disks
+// 160 us a substep, 70 now, 100 where it had 256 threads beside the element step; one
+// scene of 1400 bodies 44.7, 34.2 and 38.8.)
 // Bound by the latency of an item's chain of loads (node, cached edge, window,
 // candidates), times the groups a warp takes.  36 disks in contact: a substep
 // went from 49.2 to 22.3 us; four disks of 160 edges from 108 to 22, of 400
@@ -861,8 +865,9 @@ __device__ __forceinline__ void flex_item(const Dev& d, const FlexDev& f, const 
 // at 32 (a block's registers are free again when its slower warp ends); groups
 // of 8 items run the disks of 400 edges in 23.3 us instead of 20.0.
 __global__ void __launch_bounds__(kFlexContactThreads) k_flex_contact(Dev d, FlexDev f0, int control) {
-  if (control && blockIdx.x == 0) {
-    if (blockIdx.y == 0) step_control(d);
+  if ((int)blockIdx.x < control) {
+    const int s = blockIdx.x * f0.n_fs + blockIdx.y;
+    if (s < d.S) scene_control(d, s, f0.scene_rng[s]);
     return;
   }
   const FlexDev f = flex_view(f0, blockIdx.y);  // blockIdx.y: the scene

@@ -165,6 +165,22 @@ namespace {
 
 // ------------------------------------------------------------------ kernels
 
+// The gate of pair pr of a body whose box of the previous substep is r, in
+// substep k of its scene.
+__device__ __forceinline__ int gate_of(const Dev& d, const Pair& pr, const int* r, int k) {
+  if (pr.kind == fw::PAIR_RIGID) {  // the rigid's current box; plain overlap when the loop skips the BVH
+    const Rigid& g = d.rig[pr.table];
+    return fw::box_gate(fw::ord2f(r[0]), fw::ord2f(r[1]), fw::ord2f(r[2]), fw::ord2f(r[3]), g.lb[0], g.lb[1], g.ub[0],
+                        g.ub[1], pr.n1 ? 1 : k) ? 1 : 0;
+  }
+  if (pr.gate > 0) {  // a ground of a loop with a moving plane: its entry's current box
+    const Rigid& g = d.rig[pr.gate - 1];
+    return fw::box_gate(fw::ord2f(r[0]), fw::ord2f(r[1]), fw::ord2f(r[2]), fw::ord2f(r[3]), g.lb[0], g.lb[1], g.ub[0],
+                        g.ub[1], k) ? 1 : 0;
+  }
+  return fw::pair_gate(pr, fw::ord2f(r[0]), fw::ord2f(r[1]), fw::ord2f(r[2]), fw::ord2f(r[3]), k) ? 1 : 0;
+}
+
 __device__ void step_control(const Dev& d) {
   const int t = threadIdx.x;
   for (int s = t; s < d.S; s += blockDim.x) {
@@ -179,21 +195,7 @@ __device__ void step_control(const Dev& d) {
     const int s = d.body_scene[pr.body];
     if (d.scene_mode[s] != fw::MODE_STEP) continue;
     const int k = d.scene_counter[s];
-    const int* r = d.aabb_ring + ((size_t)(k & 1) * d.B + pr.body) * 4;
-    if (pr.kind == fw::PAIR_RIGID) {  // the rigid's current box; plain overlap when the loop skips the BVH
-      const Rigid& g = d.rig[pr.table];
-      d.pair_active[p] = fw::box_gate(fw::ord2f(r[0]), fw::ord2f(r[1]), fw::ord2f(r[2]), fw::ord2f(r[3]),
-                                      g.lb[0], g.lb[1], g.ub[0], g.ub[1], pr.n1 ? 1 : k) ? 1 : 0;
-      continue;
-    }
-    if (pr.gate > 0) {  // a ground of a loop with a moving plane: its entry's current box
-      const Rigid& g = d.rig[pr.gate - 1];
-      d.pair_active[p] = fw::box_gate(fw::ord2f(r[0]), fw::ord2f(r[1]), fw::ord2f(r[2]), fw::ord2f(r[3]),
-                                      g.lb[0], g.lb[1], g.ub[0], g.ub[1], k) ? 1 : 0;
-      continue;
-    }
-    d.pair_active[p] = fw::pair_gate(pr, fw::ord2f(r[0]), fw::ord2f(r[1]), fw::ord2f(r[2]),
-                                     fw::ord2f(r[3]), k) ? 1 : 0;
+    d.pair_active[p] = gate_of(d, pr, d.aabb_ring + ((size_t)(k & 1) * d.B + pr.body) * 4, k);
   }
   __syncthreads();
   for (int s = t; s < d.S; s += blockDim.x)
@@ -208,6 +210,42 @@ __device__ void step_control(const Dev& d) {
     r[2] = fw::f2ord(-1e30f);
     r[3] = fw::f2ord(-1e30f);
   }
+}
+
+// step_control for one scene whose bodies and pairs are the ranges rng (first
+// body, bodies, first pair, pairs), by one block: nothing is looked up per body,
+// and a few pairs' loads are in flight together.
+__device__ void scene_control(const Dev& d, int s, int4 rng) {
+  const int t = threadIdx.x, T = blockDim.x;
+  const int act = d.scene_active[s], req = d.scene_mode_req[s], k = d.scene_counter[s];
+  const int mode = act ? (req ? fw::MODE_INIT : fw::MODE_STEP) : fw::MODE_FROZEN;
+  const bool step = mode == fw::MODE_STEP;
+  __syncthreads();  // every thread has read them
+  if (t == 0) {
+    d.scene_mode[s] = mode;
+    if (act && req) d.scene_mode_req[s] = 0;
+    if (step) d.scene_counter[s] = k + 1;
+  }
+  if (mode == fw::MODE_FROZEN) return;
+  if (step) {
+    constexpr int U = 4;
+    for (int p0 = rng.z + t; p0 < rng.z + rng.w; p0 += U * T) {
+      Pair pr[U];
+      int4 box[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) pr[u] = d.pairs[min(p0 + u * T, rng.z + rng.w - 1)];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        box[u] = *reinterpret_cast<const int4*>(d.aabb_ring + ((size_t)(k & 1) * d.B + pr[u].body) * 4);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (p0 + u * T < rng.z + rng.w) d.pair_active[p0 + u * T] = gate_of(d, pr[u], &box[u].x, k);
+    }
+  }
+  const int k2 = step ? k + 1 : k;
+  const int big = fw::f2ord(1e30f), low = fw::f2ord(-1e30f);
+  for (int b = rng.x + t; b < rng.x + rng.y; b += T)
+    *reinterpret_cast<int4*>(d.aabb_ring + ((size_t)(k2 & 1) * d.B + b) * 4) = make_int4(big, big, low, low);
 }
 
 // step_control for a list of scenes (stream arenas: the active scenes of the
@@ -1593,6 +1631,7 @@ void set_grids(fw_ctx* c) {
 void flex_launch(fw_ctx* c, int force) {
   const FlexDev& f = c->fx;
   const int with_step = force || c->has_rigid ? 0 : 1;
+  const int cb = with_step ? (c->S + f.n_fs - 1) / f.n_fs : 0;  // blocks of step control per row
   const int eb = with_step ? std::max(1, std::min((c->E + 127) / 128, std::max(c->sms - f.n_fs, (c->E + 2047) / 2048))) : 0;
   k_flex_pre<<<f.n_fs + eb, kFlexScanThreads, c->flex_pre_smem, c->stream>>>(c->d, f, force);
   c->launches += 1;
@@ -1600,7 +1639,7 @@ void flex_launch(fw_ctx* c, int force) {
     const int64_t threads = (int64_t)f.n_items * kFlexLanes;
     const int64_t want = (threads + kFlexContactThreads - 1) / kFlexContactThreads;
     const int bx = (int)std::max<int64_t>(1, std::min<int64_t>(want, 8 * c->sms) / f.n_fs);
-    k_flex_contact<<<dim3(bx + with_step, f.n_fs), kFlexContactThreads, 0, c->stream>>>(c->d, f, with_step);
+    k_flex_contact<<<dim3(bx + cb, f.n_fs), kFlexContactThreads, 0, c->stream>>>(c->d, f, cb);
     c->launches += 1;
   }
 }
@@ -4153,6 +4192,23 @@ int build_flex(fw_ctx* c) {
   f.srec = srec; f.scell = scell;
   f.seg = dseg; f.unit = dunit; f.bcell = bcell;
   f.sc = dsc; f.clock_dt = c->d_flex_clock; f.err = c->d_flags + fw_ctx::kFlagFlex;
+  {  // the scenes' bodies and pairs as ranges (the pairs go to the device in body order)
+    std::vector<int4> rng(c->S, make_int4(0, 0, 0, 0));
+    std::vector<int> cnt(B, 0);
+    for (const Pair& p : c->h_pairs) cnt[p.body]++;
+    int at = 0;
+    for (int b = 0; b < B; ++b) {
+      int4& r = rng[c->h_scene[b]];
+      if (r.y == 0) r = make_int4(b, 0, at, 0);
+      r.y += 1;
+      r.w += cnt[b];
+      at += cnt[b];
+    }
+    int4* drng = nullptr;
+    if ((rc = upload(c, &drng, rng))) return rc;
+    FW_CUDA(c, cudaStreamSynchronize(c->stream));
+    f.scene_rng = drng;
+  }
   f.pair_tied = ptied; f.tie_elem = telem; f.tie_w0 = tw0; f.tie_w1 = tw1; f.tie_gap = tgap;
   c->flex_pre_smem = sizeof(float4) * (size_t)max_dom_fem;
   int optin = 0;

@@ -273,3 +273,43 @@ def test_gpu_scenes_of_many_bodies_equal_oracle(bodies):
     assert (o.flex_cache() >= 0).any()
     assert np.array_equal(lp.femSpringManager.coords.numpy()[: o.N].astype(np.float64), xo)
     assert np.array_equal(lp.femSpringManager.V.numpy()[: o.N].astype(np.float64), vo)
+
+
+def _disks(n, gap, y=0.0255):
+    return [fw.GroundDomain(2, [0.0, 0.0], [0.0, 1.0])] + [
+        fw.FemDomain(scenes.ccw_disk(fw, 4, 0.025, (0.1 + (0.05 + gap) * k, y)),
+                     fw.SolidProp((fw.Elastic, fw.HyperElastic)[k % 2](E=1e5, nu=0.3, rho=1000.0)),
+                     [fw.Gravity([9.8 * (1 - 2 * k) if gap < 0 else 0.0, -9.8])], friction=0.2) for k in range(n)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("others", [0, 1, 5, 70])
+def test_gpu_step_control_of_batches(others):
+    """A scene in FEM-FEM contact beside scenes without: a block of the contact launch controls each scene, whether or
+    not they are more than the FEM-FEM scenes; scenes sit out now and then; one has no contact at all."""
+    from flatworld_b200.batch import BatchedLoop
+
+    def build(k):
+        if k == 0:
+            return _disks(2, -1e-5)
+        return _disks(1, 0.0)[1:] if k == 1 else _disks(1, 0.0, 0.0245 + 0.001 * (k % 7))
+
+    dt = 0.3 * SceneLayout(build(0), useAdapativeDT=True).dt
+    b = BatchedLoop([build(k) for k in range(1 + others)], dt=dt, useAdapativeDT=False, damping=0.02)
+    alone = [fw.ExplicitLoop(dt, build(k), useAdapativeDT=False, damping=0.02, path="gather") for k in range(1 + others)]
+    before = b.launch_count()
+    for n, out in ((1, 0), (40, 2), (70, 3), (3, 2)):
+        active = [1 if not out or k % out else 0 for k in range(1 + others)]
+        active[0] = 1 if n != 3 else 0
+        b._set_active(active)
+        b.advance(n)
+        for lp, on in zip(alone, active):
+            if on:
+                lp.advance_n(n)
+    assert b.launch_count() - before == 3 * 114
+    assert (alone[0]._native.read_flex_state(32)[0] >= 0).any()
+    for k, lp in enumerate(alone):
+        n = lp._packed.N
+        assert np.array_equal(b.coords(k), lp._native.read_nodes(0, 0, n)), k
+        assert np.array_equal(b.velocities(k), lp._native.read_nodes(1, 0, n)), k
+        assert b._native.read_counters(1 + others)[k] == lp._native.read_counters(1)[0]
