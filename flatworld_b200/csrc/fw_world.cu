@@ -58,10 +58,14 @@ constexpr size_t kCluSharedBytes = 232448 - 64;  // of a CTA on sm_100
 // substeps gain, and gain less the more patches share an SM.  One call of ragged
 // bodies, on chip / stream kernels, us: 109,000 triangles 3 substeps 43 / 53;
 // 517,000 4: 99 / 94, 5: 110 / 113; 959,000 5: 175 / 177; 1,732,000 6: 340 / 332,
-// 8: 399 / 437; 3,674,000 6: 678 / 622, 8: 801 / 824.
-int clu_min_steps(int sms, int64_t triangles) {
-  return triangles <= (int64_t)sms * 1500 ? 3 : triangles <= (int64_t)sms * 6500 ? 5 : 8;
+// 8: 399 / 437; 3,674,000 6: 678 / 622, 8: 801 / 824.  A substep more where the
+// scenes' wide clusters (8 CTAs and more: an SM for each) do not run all at once
+// and each load is waited for twice: 3 substeps of 16 scenes of 3200 triangles 60
+// / 47, 4: 59 / 55; of 8 scenes of 7200 triangles 3: 46 / 44, 4: 47 / 55.
+int clu_min_steps(int sms, int64_t triangles, int64_t wide_ctas) {
+  return triangles <= (int64_t)sms * 1500 ? (wide_ctas > sms ? 4 : 3) : triangles <= (int64_t)sms * 6500 ? 5 : 8;
 }
+constexpr int kCluWide = 8;
 
 // The same for a single scene, whose shorter calls run on the gather kernels,
 // two plain launches a substep instead of a cooperative one and the patches'
@@ -1471,6 +1475,7 @@ struct fw_ctx {
   CluRun* d_runs = nullptr;  // fw_step_runs: every scene's runs, in the groups' order
   std::vector<int> clu_order;  // the scenes in the groups' order
   int clu_patches = 0;
+  int64_t clu_wide = 0;  // CTAs of the scenes' wide clusters (clu_min_steps)
   uint64_t clu_last_key = 0;
   HostLists lists;
   std::vector<cudaStream_t> side_streams;  // the groups after the first run beside it
@@ -1813,7 +1818,7 @@ StreamKernel stream_kernel(int nodes, int minb, int bulk) {
 // (starting buffer, dt mode, dt, count).
 int stream_steps(fw_ctx* c, int n) {
   c->host_counter += n;
-  const bool clu = !c->clu.empty() && n >= clu_min_steps(c->sms, c->E);
+  const bool clu = !c->clu.empty() && n >= clu_min_steps(c->sms, c->E, c->clu_wide);
   StreamDev sd = c->sd;
   if (!clu) sd.list = nullptr;
   if (clu) {
@@ -2516,6 +2521,7 @@ int build_cluster(fw_ctx* c, const std::vector<int32_t>& off, const std::vector<
     }
     blob.insert(blob.end(), k.blob.begin(), k.blob.end());
     made.push_back(Made{s, k.ctas, k.smem, k.kind, single ? 1 : 0});
+    if (!single && k.ctas >= kCluWide) c->clu_wide += k.ctas;
   }
   if (made.empty()) return FW_OK;
   if (single && made.size() != (size_t)S) return FW_OK;
@@ -3270,10 +3276,13 @@ int arena_cluster_steps(fw_ctx* c, int n) {
 // n substeps of a stream arena: k_control + k_stream over the active scenes'
 // patches each, then (n odd) the carry back into the first buffers.
 int arena_stream_steps(fw_ctx* c, int n) {
-  int64_t tris = 0;
+  int64_t tris = 0, wide = 0;
   for (size_t s = 0; n < 8 && s < c->ascenes.size(); ++s)
-    if (c->ascenes[s].live && c->cur_active[s]) tris += c->ascenes[s].ne;
-  const bool clu = c->clu_opt && c->d_cpatch && n >= clu_min_steps(c->sms, tris);
+    if (c->ascenes[s].live && c->cur_active[s]) {
+      tris += c->ascenes[s].ne;
+      wide += c->ascenes[s].clu.ctas >= kCluWide ? c->ascenes[s].clu.ctas : 0;
+    }
+  const bool clu = c->clu_opt && c->d_cpatch && n >= clu_min_steps(c->sms, tris, wide);
   if (clu != c->arena_clu) {  // the lists hold what is not stepped on chip
     c->arena_clu = clu;
     c->chunks_dirty = true;

@@ -253,6 +253,18 @@ def test_short_calls_equal_the_stream_kernels(bodies):
     _same(a, b)
 
 
+@pytest.mark.parametrize("sizes,least", [([(8, 8)] * 20, 3), ([(60, 60)] * 8, 3), ([(40, 40)] * 16, 4),
+                                         ([(60, 60)] * 40, 5)])
+def test_least_substeps_of_an_on_chip_batch(sizes, least):
+    """Shorter calls are two launches a substep; one more substep where the wide clusters take turns on the SMs."""
+    lp = BatchedLoop([_rectangle(nx, ny, MATS["elastic"], _plane(), cell=0.01) for nx, ny in sizes], dt=5e-5,
+                     useAdapativeDT=False)
+    for k in range(1, 7):
+        before = lp.launch_count()
+        lp.advance(k)
+        assert lp.launch_count() - before == (1 if k >= least else 2 * k)
+
+
 @pytest.mark.parametrize("patch,on_chip", [(0, 1), (64, 0)])
 def test_tuning_keeps_the_on_chip_step(patch, on_chip, tmp_path, monkeypatch):
     from flatworld_b200 import autotune
