@@ -775,29 +775,71 @@ __global__ void k_log(const float* __restrict__ x, float* __restrict__ y, float*
 }
 
 // Per cell of the voxel pairs [p0, p0 + gridDim.x) the nearest free cells that
-// fw::contact_force looks for (zero for a cell that is not occupied): a block
-// per pair, a thread per row (walked both ways) and per column.
-__global__ void k_voxel_table(Dev d, int p0) {
+// fw::contact_force looks for (zero for a cell that is not occupied): left + 1,
+// right, below + 1, above (0, nx, 0, ny: the grid's edge).  A pair's warps, one
+// to a block, take 32 columns each (a lane walks one, 32 loads in flight), one way
+// or the other, and then the rows (32 cells at a time, by ballots).  A new scene waits
+// for this before its first substep: 128 x 128 cells 9 us, 66 by one block with a
+// thread per row and per column, bound by a walk's loads one after the other.
+constexpr int kVoxelBlocks = 128;
+__global__ void __launch_bounds__(32) k_voxel_table(Dev d, int p0) {
   const Pair pr = d.pairs[p0 + blockIdx.x];
   if (pr.kind != fw::PAIR_VOXEL || pr.pad) return;
-  const int nx = pr.n0, ny = pr.n1;
+  const int nx = pr.n0, ny = pr.n1, lane = threadIdx.x, cols = (ny + 31) / 32;
   const int8_t* g = d.occ + pr.table;
   ushort4* w = d.vox + pr.table;
-  for (int line = threadIdx.x; line < nx + ny; line += blockDim.x) {
-    const bool col = line < ny;  // a line along i at j = line, or along j at i = line - ny
-    const int n = col ? nx : ny;
-    const size_t at = col ? (size_t)line : (size_t)(line - ny) * ny, step = col ? (size_t)ny : 1;
-    int free1 = 0;  // nearest free cell passed, + 1
-    for (int k = 0; k < n; ++k) {
-      const int8_t o = g[at + k * step];
-      (col ? w[at + k * step].x : w[at + k * step].z) = o == 1 ? (unsigned short)free1 : 0;
-      if (o == 0) free1 = k + 1;
+  for (int unit = blockIdx.y; unit < 2 * cols + nx; unit += gridDim.y) {
+    constexpr int U = 32;
+    if (unit < cols) {
+      const int j = 32 * unit + lane;
+      if (j >= ny) continue;
+      int near = 0;
+      for (int i0 = 0; i0 < nx; i0 += U) {
+        int8_t o[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) o[u] = __ldg(g + (size_t)min(i0 + u, nx - 1) * ny + j);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i0 + u < nx) {
+            w[(size_t)(i0 + u) * ny + j].x = o[u] == 1 ? (unsigned short)near : 0;
+            if (o[u] == 0) near = i0 + u + 1;
+          }
+      }
+      continue;
     }
-    int ahead = n;
-    for (int k = n - 1; k >= 0; --k) {
-      const int8_t o = g[at + k * step];
-      (col ? w[at + k * step].y : w[at + k * step].w) = o == 1 ? (unsigned short)ahead : 0;
-      if (o == 0) ahead = k;
+    if (unit < 2 * cols) {
+      const int j = 32 * (unit - cols) + lane;
+      if (j >= ny) continue;
+      int near = nx;
+      for (int i0 = nx - 1; i0 >= 0; i0 -= U) {
+        int8_t o[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) o[u] = __ldg(g + (size_t)max(i0 - u, 0) * ny + j);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i0 - u >= 0) {
+            w[(size_t)(i0 - u) * ny + j].y = o[u] == 1 ? (unsigned short)near : 0;
+            if (o[u] == 0) near = i0 - u;
+          }
+      }
+      continue;
+    }
+    const size_t row = (size_t)(unit - 2 * cols) * ny;
+    int near = 0;
+    for (int j0 = 0; j0 < ny; j0 += 32) {
+      const int j = j0 + lane;
+      const int8_t o = j < ny ? __ldg(g + row + j) : (int8_t)1;
+      const unsigned free = __ballot_sync(0xFFFFFFFFu, o == 0), before = free & ((1u << lane) - 1u);
+      if (j < ny) w[row + j].z = o == 1 ? (unsigned short)(before ? j0 + 32 - __clz(before) : near) : 0;
+      if (free) near = j0 + 32 - __clz(free);
+    }
+    near = ny;
+    for (int j0 = (cols - 1) * 32; j0 >= 0; j0 -= 32) {
+      const int j = j0 + lane;
+      const int8_t o = j < ny ? __ldg(g + row + j) : (int8_t)1;
+      const unsigned free = __ballot_sync(0xFFFFFFFFu, o == 0), after = free & ~((2u << lane) - 1u);
+      if (j < ny) w[row + j].w = o == 1 ? (unsigned short)(after ? j0 + __ffs(after) - 1 : near) : 0;
+      if (free) near = j0 + __ffs(free) - 1;
     }
   }
 }
@@ -4397,7 +4439,7 @@ static int finalize(fw_ctx* c) {
   bool table = false;  // of the nearest free voxel cells
   for (const Pair& p : pairs) table |= p.kind == fw::PAIR_VOXEL && !p.pad;
   if (table && dalloc_spare(c, &d.vox, c->h_occ.size())) {  // without it the grids are walked
-    k_voxel_table<<<(unsigned)pairs.size(), 256, 0, c->stream>>>(d, 0);
+    k_voxel_table<<<dim3((unsigned)pairs.size(), kVoxelBlocks), 32, 0, c->stream>>>(d, 0);
     c->launches += 1;
   }
   if ((rc = check_kernel(c, "prepare"))) return rc;
@@ -5023,7 +5065,7 @@ int fw_arena_commit_pack(fw_ctx* c, const fw_pack* pk, int32_t* scene_out) {
     // grids are walked)
     if (!c->vox_asked) dalloc_spare(c, &d.vox, (size_t)c->occ_cap);
     c->vox_asked = true;
-    if (d.vox) k_voxel_table<<<(unsigned)a.np, 256, 0, c->stream>>>(d, (int)a.p0);
+    if (d.vox) k_voxel_table<<<dim3((unsigned)a.np, kVoxelBlocks), 32, 0, c->stream>>>(d, (int)a.p0);
   }
   k_prepare_elements<<<(int)((a.ne + kBlock - 1) / kBlock), kBlock, 0, c->stream>>>(d, c->a_young + e0, c->a_poisson + e0,
                                                                                   c->a_rho + e0, e_lo, e_hi);
