@@ -67,6 +67,18 @@ int clu_min_steps(int sms, int64_t triangles, int64_t wide_ctas) {
 }
 constexpr int kCluWide = 8;
 
+// ... and of an arena, whose patches are smaller (kCluServedNodes: latency before
+// throughput), so that its scenes take more CTAs, and whose launches are put
+// together on the host for each call.  One call, on chip / stream kernels, us:
+// wide clusters of 1.7 CTAs an SM, 3 substeps 75 / 74, 6: 91 / 104; of 2.6, 6: 117 /
+// 111, 8: 133 / 141; of 5.1, 8: 223 / 207, 12: 286 / 298; of 6.9 (scenes of 16,200
+// triangles), 12: 423 / 387, 16: 532 / 511, 24: 730 / 756; of 27, 16: 1623 /
+// 1622; of 32, 16: 2140 / 1910, 50: 5550 / 5870; 512 scenes of 200 triangles, 4: 87 / 62, 6: 90 / 85, 8: 99 / 106.
+int arena_min_steps(int sms, int64_t triangles, int64_t wide_ctas, int64_t scenes) {
+  const int wide = wide_ctas > 16 * (int64_t)sms ? 32 : wide_ctas > 4 * (int64_t)sms ? 16 : wide_ctas > 2 * (int64_t)sms ? 7 : 3;
+  return std::max({clu_min_steps(sms, triangles, wide_ctas), wide, scenes > 2 * (int64_t)sms ? 6 : 3});
+}
+
 // The same for a single scene, whose shorter calls run on the gather kernels,
 // two plain launches a substep instead of a cooperative one and the patches'
 // loads.  A call and its synchronisation, on chip / gather, us: 2 substeps of
@@ -3243,6 +3255,7 @@ int stream_attrs(fw_ctx* c, int optin) {
 // cluster size.
 int arena_cluster_steps(fw_ctx* c, int n) {
   struct Item {
+    uint64_t key;  // cluster size, triangles of the largest patch
     int s;
     CluRun run;
   };
@@ -3259,21 +3272,27 @@ int arena_cluster_steps(fw_ctx* c, int n) {
       run.dt[1] = c->h_dt2[s];
     }
     if (run.n[0] + run.n[1] == 0) continue;
-    items.push_back(Item{(int)s, run});
+    items.push_back(Item{(uint64_t)a.clu.ctas << 32 | (uint32_t)a.clu.ne, (int)s, run});
     tris += a.ne;
   }
   c->clu.clear();
   if (items.empty()) return FW_OK;
   // the largest scenes first, so that the small ones fill in behind them
-  std::stable_sort(items.begin(), items.end(), [&](const Item& p, const Item& q) {
-    const CluLaunch &a = c->ascenes[p.s].clu, &b = c->ascenes[q.s].clu;
-    return a.ctas != b.ctas ? a.ctas > b.ctas : a.ne > b.ne;
-  });
+  std::sort(items.begin(), items.end(),
+            [](const Item& p, const Item& q) { return p.key != q.key ? p.key > q.key : p.s < q.s; });
   const bool shared = tris > (int64_t)c->sms * 900;
   std::vector<CluScene> scenes;
   std::vector<CluRun> runs;
+  scenes.reserve(items.size());
+  runs.reserve(items.size());
   for (const Item& it : items) {
     const fw_ctx::ArenaScene& a = c->ascenes[it.s];
+    // most scenes are no larger than those before them in any respect: nothing to lay out anew
+    auto within = [&](const CluLaunch& r) {
+      const CluLaunch& b = a.clu;
+      return b.no <= r.no && b.nh <= r.nh && b.ne <= r.ne && b.deg <= r.deg && b.npush <= r.npush && b.nbnd <= r.nbnd &&
+             b.nb <= r.nb && b.np <= r.np && b.has_j2 <= r.has_j2 && b.per_tri <= r.per_tri;
+    };
     auto widened = [&](CluLaunch r) {
       const CluLaunch& b = a.clu;
       r.no = std::max(r.no, b.no); r.nh = std::max(r.nh, b.nh); r.ne = std::max(r.ne, b.ne); r.deg = std::max(r.deg, b.deg);
@@ -3284,14 +3303,15 @@ int arena_cluster_steps(fw_ctx* c, int n) {
       return r;
     };
     bool join = !c->clu.empty() && c->clu.back().r.ctas == a.clu.ctas && 4 * a.clu.ne > c->clu.back().r.ne;
-    if (join && clu_smem(widened(c->clu.back().r)) > c->clu_cap) join = false;
+    const bool inside = join && within(c->clu.back().r);
+    if (join && !inside && clu_smem(widened(c->clu.back().r)) > c->clu_cap) join = false;
     if (!join) {
       fw_ctx::CluGroup g;
       g.r.ctas = a.clu.ctas;
       c->clu.push_back(g);
     }
     fw_ctx::CluGroup& g = c->clu.back();
-    g.r = widened(g.r);
+    if (!inside) g.r = widened(g.r);
     g.scenes += 1;
     scenes.push_back(CluScene{a.cb0, it.s, (int)a.cq0, (int)a.n0, (int)a.e0, (int)a.b0, (int)a.nb, (int)a.p0, (int)a.np});
     runs.push_back(it.run);
@@ -3318,13 +3338,14 @@ int arena_cluster_steps(fw_ctx* c, int n) {
 // n substeps of a stream arena: k_control + k_stream over the active scenes'
 // patches each, then (n odd) the carry back into the first buffers.
 int arena_stream_steps(fw_ctx* c, int n) {
-  int64_t tris = 0, wide = 0;
-  for (size_t s = 0; n < 8 && s < c->ascenes.size(); ++s)
+  int64_t tris = 0, wide = 0, scenes = 0;
+  for (size_t s = 0; n < 32 && s < c->ascenes.size(); ++s)
     if (c->ascenes[s].live && c->cur_active[s]) {
+      scenes += 1;
       tris += c->ascenes[s].ne;
       wide += c->ascenes[s].clu.ctas >= kCluWide ? c->ascenes[s].clu.ctas : 0;
     }
-  const bool clu = c->clu_opt && c->d_cpatch && n >= clu_min_steps(c->sms, tris, wide);
+  const bool clu = c->clu_opt && c->d_cpatch && n >= arena_min_steps(c->sms, tris, wide, scenes);
   if (clu != c->arena_clu) {  // the lists hold what is not stepped on chip
     c->arena_clu = clu;
     c->chunks_dirty = true;

@@ -265,6 +265,33 @@ def test_least_substeps_of_an_on_chip_batch(sizes, least):
         assert lp.launch_count() - before == (1 if k >= least else 2 * k)
 
 
+@pytest.mark.parametrize("size,scenes,least", [((8, 8), 20, 3), ((8, 8), 320, 6), ((50, 50), 20, 7), ((50, 50), 40, 16)])
+def test_least_substeps_of_an_on_chip_arena(size, scenes, least):
+    """Shorter calls are two launches a substep (and one that carries an odd call's state back), by the scenes and by
+    the SMs that their wide clusters take; the same bits on both sides."""
+    from flatworld_b200.serve import Arena
+    from flatworld_b200.world import PackedWorld, SceneLayout
+
+    lay = SceneLayout(_rectangle(*size, MATS["mises"], _plane(), cell=0.01))
+    ar = Arena(400_000, 800_000, 512, 512, 512, 1, 1)
+    pk = ar.pack(lay, PackedWorld([lay]))
+    sc = [ar.insert_pack(lay, pk) for _ in range(scenes)]
+    dts = np.zeros(ar.S, np.float32)
+    dts[sc] = 2e-5
+    ran = 0
+    for n in (1, 2, 3, 4, 5, 6, 7, 15, 16, 17, 3):
+        before = ar.native.launch_count()
+        ar.native.step_served_n(dts, n)
+        ran += n
+        assert ar.native.launch_count() - before == (1 if n >= least else 2 * n + n % 2)
+    lp = fw.ExplicitLoop(2e-5, _rectangle(*size, MATS["mises"], _plane(), cell=0.01), useAdapativeDT=False, path="gather")
+    lp.advance_n(ran - 1)
+    for s in (sc[0], sc[-1]):
+        assert np.array_equal(ar.coords(s), lp.femSpringManager.coords.numpy()[: lp._packed.N])
+    pk.close()
+    ar.close()
+
+
 @pytest.mark.parametrize("patch,on_chip", [(0, 1), (64, 0)])
 def test_tuning_keeps_the_on_chip_step(patch, on_chip, tmp_path, monkeypatch):
     from flatworld_b200 import autotune
