@@ -322,8 +322,9 @@ int fw_set_path(fw_ctx* ctx, int32_t path, int32_t patches);
  * than 8 bodies or 32 contact pairs in a scene.  After fw_finalize STREAM_MINB
  * and STREAM_BULK shape the stream kernels where those run and leave the other
  * scenes on chip.  Calls of one or a few substeps (by the world's size) run on
- * the gather or stream kernels in any case.  Same bits.  fw_get_option: 0 none, 1 every scene, 2 some
- * scenes of the world are stepped this way. */
+ * the gather or stream kernels in any case.  Same bits.  fw_get_option: 0 none,
+ * 1 every scene, 2 some scenes of the world are stepped this way (0 for an
+ * arena, whose scenes come and go). */
 #define FW_OPT_CLUSTER 12
 int fw_set_option(fw_ctx* ctx, int32_t option, int32_t value);
 /* The value an option has now.  Readable: FRONT_WARPS, RES_THREADS,
